@@ -2,11 +2,14 @@
 //
 // C_b = alpha * op(A_b) * op(B_b) + beta * C_b, column-major, op in {N, T, C, R}.
 // GB300 executes FP64 at a small fraction of its FP32 rate, so this kernel is
-// compute-bound for every shape that matters; a 64x64 tile with 4x4 outputs per
-// thread keeps the FP64 pipes busy.  Loads are mapped so that consecutive threads
-// touch consecutive addresses for either operand orientation.
+// compute-bound for every shape that matters: 64x64 tiles with 4x4 outputs per thread for
+// outputs that fill whole waves of SMs, 16x16 tiles with a cluster split of K for all
+// others, and a row-per-thread form for products with a sparse operator tensor.  Loads
+// are mapped so that consecutive threads touch consecutive addresses for either operand
+// orientation.
 #include "nsg_internal.h"
-#include "tuning_table.h"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <map>
@@ -28,10 +31,32 @@ __device__ __forceinline__ void zero(double& v) { v = 0.0; }
 __device__ __forceinline__ bool nonzero(double v) { return v != 0.0; }
 __device__ __forceinline__ bool nonzero(double2 v) { return v.x != 0.0 || v.y != 0.0; }
 __device__ __forceinline__ void zero(double2& v) { v = make_double2(0.0, 0.0); }
+__device__ __forceinline__ double plus(double a, double b) { return a + b; }
+__device__ __forceinline__ double2 plus(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ void mac(double& acc, double a, double b) { acc = fma(a, b, acc); }
 __device__ __forceinline__ void mac(double2& acc, double2 a, double2 b) {
   acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
   acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
+
+// shift of a coefficient +-2^s with |s| < 512 as 2 s + (negative), `none` for any other
+// value; and a times that coefficient: by adding s to a's exponent field and flipping its
+// sign bit when the result is a normal number, else by the multiplication (same value)
+__device__ __forceinline__ int pow2_shift(double v, int none) {
+  const long long b = __double_as_longlong(v);
+  const int s = int((b >> 52) & 0x7ff) - 1023;
+  if ((b & 0xfffffffffffffll) != 0 || s <= -512 || s >= 512) return none;
+  return 2 * s + (b < 0 ? 1 : 0);
+}
+__device__ __forceinline__ int pow2_shift(double2 v, int none) { return v.y == 0.0 ? pow2_shift(v.x, none) : none; }
+__device__ __forceinline__ double mul_pow2(double a, int code, double v) {
+  const long long b = __double_as_longlong(a);
+  const int e = int((b >> 52) & 0x7ff), s = code >> 1;
+  if (e == 0x7ff || e == 0 || e + s <= 0 || e + s >= 0x7ff) return a * v;
+  return __longlong_as_double((b + ((long long)s << 52)) ^ ((long long)(code & 1) << 63));
+}
+__device__ __forceinline__ double2 mul_pow2(double2 a, int code, double2 v) {
+  return make_double2(mul_pow2(a.x, code, v.x), mul_pow2(a.y, code, v.x));
 }
 
 template <typename T>
@@ -174,129 +199,266 @@ __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int64_t batch, int sp
   }
 }
 
-// Tall-skinny products with N, K <= 32: the site-operator steps of H_eff and of the
-// environment updates (K, N = w d, batched over the other bond).  op(B) is an MPO
-// tensor and mostly zeros, so each CTA lists its non-zeros per column (warp ballots)
-// and stages a 256-row tile of op(A) in shared memory ([k][row], conflict-free); thread
-// r then forms row r of C from exactly nnz(B) multiply-adds.  The FP64 work drops by
-// the operator's sparsity and the kernel runs at the HBM rate of reading A and writing C.
-constexpr int kSkinnyRows = 256;
-template <typename T>
-__global__ void __launch_bounds__(kSkinnyRows)
-    gemm_skinny_kernel(int64_t M, int N, int K, const T* __restrict__ A, int64_t lda, int64_t sA, bool conjA,
-                       const T* __restrict__ B, int64_t ldb, int64_t sB, int opB, T* __restrict__ C,
-                       int64_t ldc, int64_t sC, int64_t batch, Scal<T> sc) {
-  extern __shared__ __align__(16) unsigned char sk_smem[];
-  T* As = (T*)sk_smem;                        // [K][kSkinnyRows]
-  __shared__ T nzv[32 * 32];                  // non-zeros of op(B), column-major order
-  __shared__ unsigned char nzk[32 * 32];      // their row index k
-  __shared__ int colptr[33];
+// Small-tile form: one 16 x 16 output tile per CTA of 256 threads (one output each), K cut
+// into `splits` slices held by the CTAs of one thread-block cluster.  An SM retires two
+// FP64 multiply-adds per clock and a warp's one holds its sub-partition's pipe for 64
+// clocks, so neither register blocking nor operand traffic matters (a tile's operands are
+// re-read from L2 at 1 byte per multiply-add): small tiles waste the least work on padding
+// and fill the SMs evenly.  Measured against 32 x 32 tiles (2 x 2 to 2 x 4 outputs per
+// thread) and 16 x 16 tiles of 128 threads or with K dealt to the warps: fastest or within
+// 2 % at every size from 36^2 to 2072 x 924.  The slices' partial tiles are added through
+// distributed shared memory in rank order: no workspace, no second launch.  The next K slab
+// is loaded into registers while the current one is multiplied.  With launch, 64^3: 8 us
+// (64 x 64 tiles with split K: 29), 128^3: 12 (31), 256^3: 41 (49), 2072 x 924 x 259: 0.85 ms
+// (1.10); complex 64^3: 12 (77), 512^3: 0.95 ms (1.06).
+constexpr int TB = 16, kTileThreads = TB * TB;
+template <typename T, int BK>
+__global__ void __launch_bounds__(kTileThreads)
+    gemm_tile_kernel(int64_t M, int64_t N, int64_t Kfull, const T* __restrict__ A, int64_t lda, int64_t sA, int opA,
+                     const T* __restrict__ B, int64_t ldb, int64_t sB, int opB, T* __restrict__ C, int64_t ldc,
+                     int64_t sC, int64_t batch, Scal<T> sc, int splits, int64_t kslice) {
+  constexpr int NL = BK / TB;
+  __shared__ T As[2][BK][TB + 1], Bs[2][BK][TB + 1];
+  __shared__ T Cs[kTileThreads];
+  const int tid = threadIdx.x, ti = tid % TB, tj = tid / TB;
+  const int64_t m0 = int64_t(blockIdx.x) * TB, n0 = int64_t(blockIdx.y) * TB;
+  const bool transA = (opA == OP_T || opA == OP_C), conjA = (opA == OP_C || opA == OP_R);
   const bool transB = (opB == OP_T || opB == OP_C), conjB = (opB == OP_C || opB == OP_R);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t tiles = (M + kSkinnyRows - 1) / kSkinnyRows;
-  for (int64_t job = blockIdx.x; job < tiles * batch; job += gridDim.x) {
-    const int64_t bz = job / tiles, i0 = (job % tiles) * kSkinnyRows;
-    const T* Bb = B + bz * sB;
+  const int64_t zstep = int64_t(gridDim.z) / splits;  // splits > 1: grid z is exactly batch x splits
+  const int sp = int(blockIdx.z % unsigned(splits));
+  const int64_t kb = sp * kslice, K = max(int64_t(0), min(kslice, Kfull - kb));
+  for (int64_t bz = blockIdx.z / unsigned(splits); bz < batch; bz += zstep) {
     const T* Ab = A + bz * sA;
-    __syncthreads();  // the previous job's readers are done
-    if (warp == 0) {
-      int base = 0;
-      for (int j = 0; j < N; ++j) {
-        T v;
-        zero(v);
-        if (lane < K) v = ld(transB ? Bb + j + (int64_t)lane * ldb : Bb + lane + (int64_t)j * ldb, conjB);
-        const unsigned m = __ballot_sync(0xffffffffu, nonzero(v));
-        if (lane == 0) colptr[j] = base;
-        if (nonzero(v)) {
-          const int pos = base + __popc(m & ((1u << lane) - 1u));
-          nzv[pos] = v;
-          nzk[pos] = (unsigned char)lane;
-        }
-        base += __popc(m);
+    const T* Bb = B + bz * sB;
+    T ra[NL], rb[NL];
+    // lanes run along the contiguous axis of each operand as stored
+    auto load = [&](int64_t k0) {
+#pragma unroll
+      for (int r = 0; r < NL; ++r) {
+        const int i = transA ? tj : ti, ka = (transA ? ti : tj) + TB * r;
+        const int j = transB ? ti : tj, kc = (transB ? tj : ti) + TB * r;
+        const int64_t gi = m0 + i, gka = kb + k0 + ka, gj = n0 + j, gkb = kb + k0 + kc;
+        zero(ra[r]);
+        zero(rb[r]);
+        if (gi < M && k0 + ka < K) ra[r] = ld(transA ? Ab + gka + gi * lda : Ab + gi + gka * lda, conjA);
+        if (gj < N && k0 + kc < K) rb[r] = ld(transB ? Bb + gj + gkb * ldb : Bb + gkb + gj * ldb, conjB);
       }
-      if (lane == 0) colptr[N] = base;
+    };
+    T acc;
+    zero(acc);
+    load(0);
+    int buf = 0;
+    for (int64_t k0 = 0; k0 < K; k0 += BK, buf ^= 1) {
+#pragma unroll
+      for (int r = 0; r < NL; ++r) {
+        As[buf][(transA ? ti : tj) + TB * r][transA ? tj : ti] = ra[r];
+        Bs[buf][(transB ? tj : ti) + TB * r][transB ? ti : tj] = rb[r];
+      }
+      __syncthreads();  // (the other buffer's readers passed the previous slab's barrier)
+      if (k0 + BK < K) load(k0 + BK);
+      const int kn = int(min(int64_t(BK), K - k0));
+      if (kn == BK) {
+#pragma unroll
+        for (int k = 0; k < BK; ++k) mac(acc, As[buf][k][ti], Bs[buf][k][tj]);
+      } else {  // the ragged last slab: no multiply-adds on its padding
+        for (int k = 0; k < kn; ++k) mac(acc, As[buf][k][ti], Bs[buf][k][tj]);
+      }
     }
-    const int64_t i = i0 + tid;
-    for (int k = 0; k < K; ++k) {
-      T a;
-      zero(a);
-      if (i < M) a = ld(Ab + i + (int64_t)k * lda, conjA);
-      As[k * kSkinnyRows + tid] = a;
+    T* Cb = C + bz * sC;
+    if (splits == 1) {
+      const int64_t gi = m0 + ti, gj = n0 + tj;
+      if (gi < M && gj < N) {
+        T* cp = Cb + gi + gj * ldc;
+        *cp = sc.epi(acc, cp);
+      }
+      __syncthreads();  // this batch entry's slabs are read before the next one's are stored
+    } else {
+      namespace cg = cooperative_groups;
+      cg::cluster_group cluster = cg::this_cluster();
+      Cs[tid] = acc;
+      cluster.sync();
+      const int per = kTileThreads / splits, e = sp * per + tid;
+      const int64_t gi = m0 + e % TB, gj = n0 + e / TB;
+      if (tid < per && gi < M && gj < N) {
+        T sum = *cluster.map_shared_rank(Cs + e, 0);
+        for (int r = 1; r < splits; ++r) sum = plus(sum, *cluster.map_shared_rank(Cs + e, r));
+        T* cp = Cb + gi + gj * ldc;
+        *cp = sc.epi(sum, cp);
+      }
+      cluster.sync();  // no CTA leaves while another may still read its tile
+    }
+  }
+}
+
+// Tall-skinny products with N, K <= 32: the site-operator steps of H_eff and of the
+// environment updates (K, N = w d, batched over the other bond).  op(B) is an MPO tensor
+// and mostly zeros: each CTA stages it in shared memory and lists the non-zeros of every
+// column (one warp per column, ballots), and thread r forms row r of C from exactly
+// nnz(B) multiply-adds on a [k][row] tile of op(A).  The rows of all batch entries that
+// share B (strideB = 0) form one row space, so short batch entries fill whole CTAs.  The
+// FP64 pipe (two multiply-adds per clock and SM) bounds the kernel beside the HBM traffic
+// of A and C, so a column's first term is an exponent addition where its coefficient is a
+// power of two (half of an MPO's entries) and alpha = 1, beta = 0 cost nothing.  A step of
+// 216 rows took 20 us when one warp read B's columns one after the other; it takes 5.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    gemm_skinny_kernel(int64_t M, int64_t rows, int N, int K, const T* __restrict__ A, int64_t lda, int64_t sA,
+                       bool conjA, const T* __restrict__ B, int64_t ldb, int64_t sB, int opB, T* __restrict__ C,
+                       int64_t ldc, int64_t sC, int64_t groups, Scal<T> sc, bool plain) {
+  extern __shared__ __align__(16) unsigned char sk_smem[];
+  const int nt = blockDim.x;
+  T* As = (T*)sk_smem;                       // [K][nt]
+  __shared__ T Bs[32][33];                   // op(B)
+  __shared__ T nzv[32][32];                  // non-zeros of each column of op(B)
+  __shared__ unsigned char nzk[32][32];      // their row index k
+  __shared__ int cnt[32], lead[32];          // their number; exponent of a real power-of-two first one
+  constexpr int kNoLead = 1 << 20;
+  const bool transB = (opB == OP_T || opB == OP_C), conjB = (opB == OP_C || opB == OP_R);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+  const int64_t tiles = (rows + nt - 1) / nt;
+  int64_t listed = -1;
+  for (int64_t job = blockIdx.x; job < tiles * groups; job += gridDim.x) {
+    const int64_t g = job / tiles, r = (job % tiles) * nt + tid;
+    const int64_t bz = g + r / M, i = r % M;  // (groups > 1: rows = M, so r / M = 0)
+    __syncthreads();  // the previous job's readers are done
+    if (g != listed) {
+      const T* Bb = B + g * sB;
+      for (int e = tid; e < N * K; e += nt) {
+        const int j = transB ? e % N : e / K, k = transB ? e / N : e % K;
+        Bs[j][k] = ld(transB ? Bb + j + (int64_t)k * ldb : Bb + k + (int64_t)j * ldb, conjB);
+      }
+    }
+    T* Ar = As + tid;
+    if (r < rows) {
+      const T* Ab = A + bz * sA + i;
+#pragma unroll 8
+      for (int k = 0; k < K; ++k) Ar[k * nt] = ld(Ab + (int64_t)k * lda, conjA);
     }
     __syncthreads();
-    if (i < M) {
+    if (g != listed) {
+      for (int j = warp; j < N; j += nw) {
+        T v;
+        zero(v);
+        if (lane < K) v = Bs[j][lane];
+        const unsigned m = __ballot_sync(0xffffffffu, nonzero(v));
+        if (nonzero(v)) {
+          const int pos = __popc(m & ((1u << lane) - 1u));
+          nzv[j][pos] = v;
+          nzk[j][pos] = (unsigned char)lane;
+          if (pos == 0) lead[j] = pow2_shift(v, kNoLead);
+        }
+        if (lane == 0) cnt[j] = __popc(m);
+      }
+      listed = g;
+      __syncthreads();
+    }
+    if (r < rows) {
       T* Cb = C + bz * sC + i;
       for (int j = 0; j < N; ++j) {
+        const int c = cnt[j];
         T acc;
         zero(acc);
-        for (int t = colptr[j]; t < colptr[j + 1]; ++t) mac(acc, As[nzk[t] * kSkinnyRows + tid], nzv[t]);
+        int t = 0;
+        if (c > 0) {
+          const T a = Ar[nzk[j][0] * nt];
+          if (lead[j] != kNoLead)
+            acc = mul_pow2(a, lead[j], nzv[j][0]);
+          else
+            mac(acc, a, nzv[j][0]);
+          t = 1;
+        }
+        for (; t < c; ++t) mac(acc, Ar[nzk[j][t] * nt], nzv[j][t]);
         T* cp = Cb + (int64_t)j * ldc;
-        *cp = sc.epi(acc, cp);
+        *cp = plain ? acc : sc.epi(acc, cp);
       }
     }
   }
 }
 
-void raise_smem_limit_gemm(const void* fn, int bytes) { ensure_smem_limit(fn, bytes); }
+template <typename T, int BK>
+void launch_tile(nsg_ctx* c, const GemmArgs& g, Scal<T> sc, int splits, int64_t kslice) {
+  cudaLaunchConfig_t cfg = {};
+  const int64_t z = std::min<int64_t>(g.batch * splits, 65535);
+  cfg.gridDim = dim3(unsigned((g.M + TB - 1) / TB), unsigned((g.N + TB - 1) / TB), unsigned(z));
+  cfg.blockDim = dim3(kTileThreads);
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = unsigned(splits);
+  cfg.attrs = attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+  NSG_CUDA(cudaLaunchKernelEx(&cfg, gemm_tile_kernel<T, BK>, g.M, g.N, g.K, (const T*)g.A, g.lda, g.strideA, g.opA,
+                              (const T*)g.B, g.ldb, g.strideB, g.opB, (T*)g.C, g.ldc, g.strideC, g.batch, sc, splits,
+                              kslice));
+}
+
+// The 16 x 16 tiles unless the 64 x 64 tiles fill whole waves of SMs: both run the FP64
+// pipe at its rate (96 % and 98 % of two multiply-adds per clock and SM measured on large
+// products), so the line is where the last wave's idle SMs and the padding cost less than
+// that difference.  K is split only while the tiles leave half of the SMs idle, into slices
+// of at least 16 (more CTAs than SMs lose to the slices' fixed cost: 256^3 takes 42 us
+// whole, 51 us in two slices).
+bool gemm_small_tiles(nsg_ctx* c, const GemmArgs& g, int64_t sms, double flops) {
+  auto tiles = [&](int64_t t) { return ((g.M + t - 1) / t) * ((g.N + t - 1) / t) * g.batch; };
+  if (g.K < 1 || (g.N + TB - 1) / TB > 65535 || (g.M + TB - 1) / TB >= (1ll << 31)) return false;
+  if (double((tiles(BM) + sms - 1) / sms * sms) * BM * BN < double(tiles(TB)) * TB * TB * 1.02) return false;
+  int splits = 1;
+  while (splits < 8 && tiles(TB) * splits * 2 <= sms && g.K >= 32 * splits) splits *= 2;
+  const int64_t kslice = splits == 1 ? g.K : ((g.K + splits - 1) / splits + 3) / 4 * 4;
+  ProfScope ps(c, NSG_PROF_SIMT_GEMM, flops);
+  if (g.dtype == NSG_C128)
+    launch_tile<double2, 16>(
+        c, g, Scal<double2>{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)}, splits, kslice);
+  else
+    launch_tile<double, 32>(c, g, Scal<double>{g.alpha_re, g.beta_re}, splits, kslice);
+  count_launch(c);
+  check_launch("gemm_tile");
+  return true;
+}
 
 }  // namespace
 
 void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
   if (g.M == 0 || g.N == 0 || g.batch == 0) return;
+  const int64_t sms = c->num_sms > 0 ? c->num_sms : 152;
+  const bool cplx = g.dtype == NSG_C128;
+  const double flops = double(g.M) * double(g.N) * double(g.K) * double(g.batch) * (cplx ? 8.0 : 2.0);
   if (g.N <= 32 && g.K <= 32 && g.K >= 1 && (g.opA == OP_N || g.opA == OP_R)) {
-    const int64_t sms = c->num_sms > 0 ? c->num_sms : 152;
-    const int64_t jobs = ((g.M + kSkinnyRows - 1) / kSkinnyRows) * g.batch;
-    const int grid = int(std::min<int64_t>(jobs, sms * 16));
-    ProfScope ps(c, NSG_PROF_SIMT_GEMM,
-                 double(g.M) * double(g.N) * double(g.K) * double(g.batch) * (g.dtype == NSG_C128 ? 8.0 : 2.0));
-    if (g.dtype == NSG_C128) {
-      const int shm = int(g.K) * kSkinnyRows * 16;
-      Scal<double2> sc{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)};
-      raise_smem_limit_gemm((const void*)gemm_skinny_kernel<double2>, 32 * kSkinnyRows * 16);
-      gemm_skinny_kernel<double2><<<grid, kSkinnyRows, shm, c->stream>>>(
-          g.M, int(g.N), int(g.K), (const double2*)g.A, g.lda, g.strideA, g.opA == OP_R, (const double2*)g.B,
-          g.ldb, g.strideB, g.opB, (double2*)g.C, g.ldc, g.strideC, g.batch, sc);
-    } else {
-      const int shm = int(g.K) * kSkinnyRows * 8;
-      Scal<double> sc{g.alpha_re, g.beta_re};
-      raise_smem_limit_gemm((const void*)gemm_skinny_kernel<double>, 32 * kSkinnyRows * 8);
-      gemm_skinny_kernel<double><<<grid, kSkinnyRows, shm, c->stream>>>(
-          g.M, int(g.N), int(g.K), (const double*)g.A, g.lda, g.strideA, false, (const double*)g.B, g.ldb,
-          g.strideB, g.opB, (double*)g.C, g.ldc, g.strideC, g.batch, sc);
-    }
+    // batch entries that share B are one row space; rows per CTA: the smallest of 64, 128,
+    // 256 with which the rows still take every SM (the list of B's non-zeros is built per CTA)
+    const bool shared_b = g.strideB == 0 || g.batch == 1;
+    const int64_t groups = shared_b ? 1 : g.batch, rows = shared_b ? g.M * g.batch : g.M;
+    int nt = 64;
+    while (nt < 256 && (rows + nt - 1) / nt * groups > 2 * sms) nt *= 2;
+    const int grid = int(std::min<int64_t>((rows + nt - 1) / nt * groups, sms * 16));
+    const bool plain = g.alpha_re == 1.0 && g.alpha_im == 0.0 && g.beta_re == 0.0 && g.beta_im == 0.0;
+    ProfScope ps(c, NSG_PROF_SIMT_GEMM, flops);
+    auto launch = [&](auto zero_value, auto sc) {
+      using T = decltype(zero_value);
+      ensure_smem_limit((const void*)gemm_skinny_kernel<T>, 32 * 256 * int(sizeof(T)));
+      gemm_skinny_kernel<T><<<grid, nt, size_t(g.K) * nt * sizeof(T), c->stream>>>(
+          g.M, rows, int(g.N), int(g.K), (const T*)g.A, g.lda, g.strideA, g.opA == OP_R, (const T*)g.B, g.ldb,
+          g.strideB, g.opB, (T*)g.C, g.ldc, g.strideC, groups, sc, plain);
+    };
+    if (cplx)
+      launch(double2{}, Scal<double2>{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)});
+    else
+      launch(double{}, Scal<double>{g.alpha_re, g.beta_re});
     count_launch(c);
     check_launch("gemm_skinny");
     return;
   }
+  if (c->tune_splitk == 0 && gemm_small_tiles(c, g, sms, flops)) return;
   int64_t gx = (g.M + BM - 1) / BM, gy = (g.N + BN - 1) / BN;
   NSG_CHECK(gx < (1ll << 31) && gy < 65536, NSG_ERR_UNSUPPORTED, "gemm: grid too large");
-  // split K when the tile grid cannot fill the GPU
+  // K is split here only by the context's override: without one, products of few tiles
+  // are the small tiles' (above), which split K themselves
   int splits = 1;
   int64_t ksplit = g.K;
-  const int64_t tiles = gx * gy * g.batch;
-  const int64_t sms = c->num_sms > 0 ? c->num_sms : 152;
-  if (tiles < sms && g.K >= 64) {
-    // small outputs (the eigensolver's GEMMs at bond dimension <= 128 have a handful of
-    // tiles): spread K over more SMs, down to 32-deep slices; the FP64 pipe of one SM is
-    // the bound otherwise
-    int64_t want = (2 * sms + tiles - 1) / tiles;
-    int64_t maxs = g.K >= 512 ? g.K / 256 : g.K / 32;
-    splits = int(std::min<int64_t>({want, maxs, 64}));
-    if (splits < 2) splits = 1;
-    ksplit = (g.K + splits - 1) / splits;
-    ksplit = ((ksplit + 15) / 16) * 16;
-    splits = int((g.K + ksplit - 1) / ksplit);
-  }
-  // the tuning table (or the context's override) replaces the rule for its buckets
-  int tuned = c->tune_splitk;
-  if (tuned == 0)
-    for (const auto& t : tuning::kSplit)
-      if (t.splits > 0 && tiles <= t.max_tiles && g.K <= t.max_k) {
-        tuned = t.splits;
-        break;
-      }
-  if (tuned > 0) {
-    splits = int(std::min<int64_t>(tuned, std::max<int64_t>(1, g.K / 16)));
+  if (c->tune_splitk > 0) {
+    splits = int(std::min<int64_t>(c->tune_splitk, std::max<int64_t>(1, g.K / 16)));
     ksplit = (g.K + splits - 1) / splits;
     ksplit = ((ksplit + 15) / 16) * 16;
     splits = int((g.K + ksplit - 1) / ksplit);
@@ -304,9 +466,8 @@ void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
   int64_t zt = g.batch * splits;
   int64_t gz = zt < 65535 ? zt : 65535;
   dim3 grid{unsigned(gx), unsigned(gy), unsigned(gz)};
-  const size_t eb = g.dtype == NSG_C128 ? 16 : 8;
-  ProfScope ps(c, NSG_PROF_SIMT_GEMM,
-               double(g.M) * double(g.N) * double(g.K) * double(g.batch) * (g.dtype == NSG_C128 ? 8.0 : 2.0));
+  const size_t eb = cplx ? 16 : 8;
+  ProfScope ps(c, NSG_PROF_SIMT_GEMM, flops);
   void* W = nullptr;
   size_t wbytes = 0;
   void* Cout = g.C;
@@ -315,7 +476,7 @@ void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
     W = dalloc(c, wbytes);
     Cout = W;
   }
-  if (g.dtype == NSG_C128) {
+  if (cplx) {
     Scal<double2> sc{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)};
     gemm_kernel<double2, 8><<<grid, NT, 0, c->stream>>>(g.M, g.N, g.K, (const double2*)g.A, g.lda, g.strideA, g.opA,
                                                         (const double2*)g.B, g.ldb, g.strideB, g.opB,

@@ -58,7 +58,7 @@ struct nsg_ctx {
   // steps without host synchronisation before it checks convergence
   int krylov_hint = 0;
   // launch-choice overrides set by nsg_ctx_set_tuning (0: the compiled-in tuning table)
-  int tune_splitk = 0;  // FP64 GEMM K slices (> 0 forces that count)
+  int tune_splitk = 0;  // FP64 GEMM K slices of the 64 x 64 tiles (> 0 forces both)
   int tune_tri = 0;     // tridiagonalisation: -1 grid kernel, 2..16 cluster size
   int tune_dc_leaf = 0; // divide and conquer leaf order (4..32; 0 the default)
   // pinned host staging for scalar readback
