@@ -131,6 +131,11 @@ double* dev_scratch(nsg_ctx* c, size_t n) {
   return c->dev_scratch;
 }
 
+cudaEvent_t read_event(nsg_ctx* c) {
+  if (!c->read_done) NSG_CUDA(cudaEventCreateWithFlags(&c->read_done, cudaEventDisableTiming));
+  return c->read_done;
+}
+
 // Waits for a device flag with the bounded pattern of the library's kernels (poll,
 // back off, give up after `polls` polls) and, when the wait runs out, raises the
 // context's error flag and returns: the context stays usable.
@@ -231,6 +236,7 @@ int nsg_ctx_destroy(nsg_ctx* c) {
   clear_phases(c);
   for (auto& e : c->events)
     if (e) cudaEventDestroy(e);
+  if (c->read_done) cudaEventDestroy(c->read_done);
   if (c->host_scalars) cudaFreeHost(c->host_scalars);
   if (c->dev_scratch) cudaFree(c->dev_scratch);
   if (c->dev_flag) cudaFree(c->dev_flag);

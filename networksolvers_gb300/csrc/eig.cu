@@ -21,7 +21,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <numeric>
 
 namespace nsg {
 
@@ -210,14 +209,12 @@ static bool factorize_right(nsg_ctx* c, nsg_tensor* M, int64_t m, int64_t ncol, 
     kr = 0;
     while (kr < k && P[kr] > 1e-11 * P[0]) ++kr;
     ok = P[0] > 0.0 && P[k - 1] > 0.0 && (k - kr) + n <= m;
-    if (!ok) return std::vector<int>();
+    if (!ok) return EigCols{};
     vbytes = eb * size_t(n) * size_t(k);
     V = dalloc(c, vbytes);
     *Z = V;
     *ldz = n;
-    std::vector<int> cols(k);
-    for (int64_t i = 0; i < k; ++i) cols[i] = int(n - 1 - i);
-    return cols;
+    return EigCols{n - 1, -1, k};  // descending
   };
   try {
     syevd_dc(c, dt, int(n), G, w, pick);
@@ -299,9 +296,7 @@ static bool factorize_right(nsg_ctx* c, nsg_tensor* M, int64_t m, int64_t ncol, 
     PickFn all = [&](const std::vector<double>&, void** Z, int64_t* ldz) {
       *Z = E;
       *ldz = kt;
-      std::vector<int> cols(kt);
-      std::iota(cols.begin(), cols.end(), 0);
-      return cols;
+      return EigCols{0, 1, kt};
     };
     try {
       syevd_dc(c, dt, int(kt), Gt, wt, all);
@@ -455,9 +450,7 @@ static int factorize_impl(nsg_ctx* c, const nsg_tensor* T, const int* left_axes,
     }
     *Z = Zall ? Zall : Ut->data;
     *ldz = m;
-    std::vector<int> cols(ncols);
-    for (int64_t i = 0; i < ncols; ++i) cols[i] = int(m - 1 - i);
-    return cols;
+    return EigCols{m - 1, -1, ncols};
   };
   try {
     syevd_dc(c, dt, int(m), G, w, pick);
@@ -561,9 +554,7 @@ int nsg_eigh(nsg_ctx* c, const nsg_tensor* rho, const int* row_axes, int n_row, 
     Ut = new_tensor(c, dt, int(udims.size()), udims.data(), false);
     *Z = Ut->data;
     *ldz = m;
-    std::vector<int> cols(k);
-    for (int64_t i = 0; i < k; ++i) cols[i] = int(m - 1 - i);
-    return cols;
+    return EigCols{m - 1, -1, k};
   };
   try {
     syevd_dc(c, dt, int(m), A, w, pick);

@@ -70,6 +70,7 @@ struct nsg_ctx {
   int* dev_flag = nullptr;     // raised by tensor-core kernels whose bounded waits expired
   bool flag_pending = false;   // a launch since the last check may have raised it
   int num_sms = 0;
+  cudaEvent_t read_done = nullptr;  // recorded after a device-to-host copy the host will wait for
   cudaEvent_t events[16] = {};
   bool profiling = false;
   struct ProfRec {
@@ -110,6 +111,7 @@ nsg_tensor* new_tensor(nsg_ctx* c, int dtype, int rank, const int64_t* dims, boo
 void free_tensor(nsg_ctx* c, nsg_tensor* t);
 double* host_scalars(nsg_ctx* c, size_t n);
 double* dev_scratch(nsg_ctx* c, size_t n);
+cudaEvent_t read_event(nsg_ctx* c);
 // The context's device error flag (zeroed on creation).  Kernels that may time out
 // write 1 into it instead of forcing a synchronisation per launch; every public entry
 // point checks it once at its end (check_device_flag) and reports NSG_ERR_TIMEOUT.
@@ -215,10 +217,20 @@ void copy_rows(nsg_ctx* c, int dtype, int64_t nrows_out, int64_t ncols, const vo
 void row_norms2(nsg_ctx* c, int dtype, int64_t rows, int64_t cols, const void* A, int64_t lda,
                 double* out_dev);
 
+// Eigen-decomposition of the real symmetric tridiagonal (d, e) on the device (dc.cu):
+// eigenvalues ascending into w, eigenvectors into the returned one of the n x n buffers Q0
+// and Q1 (column-major; both are scratch).  A leaf that does not converge sets *err (which
+// the caller zeroes before and reads after).
+double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* Q0, double* Q1, double* w, int* err);
+
 // Hermitian eigensolver (tridiagonalisation + divide and conquer + back-transformation).
 // A (n x n) is consumed.  `pick` receives the eigenvalues in ascending order and returns
-// the indices whose eigenvectors are wanted, after pointing *Z / *ldz at the output.
-using PickFn = std::function<std::vector<int>(const std::vector<double>&, void** Z, int64_t* ldz)>;
+// which eigenvectors are wanted (count of them, from index first in steps of step), after
+// pointing *Z / *ldz at the output.
+struct EigCols {
+  int64_t first = 0, step = 1, count = 0;
+};
+using PickFn = std::function<EigCols(const std::vector<double>&, void** Z, int64_t* ldz)>;
 void syevd_dc(nsg_ctx* c, int dtype, int n, void* A, std::vector<double>& w_host, const PickFn& pick);
 
 // host helpers

@@ -3,11 +3,7 @@
 //      cluster holding the matrix in distributed shared memory (orders up to the tuning
 //      table's limit), else one cooperative kernel over all SMs with one grid barrier
 //      per column (the matrix stays L2-resident),
-//   2. Cuppen divide and conquer on T: implicit-QL leaves (8 rows by default), rank-one
-//      merges with deflation (small z / close poles), every merge of a tree level in one
-//      launch per step, secular roots by the two-pole rational model inside a bracket
-//      with the origin at the nearer pole (one warp per root), Gu-Eisenstat recomputed z
-//      for orthogonal vectors, merged by one batched product per level,
+//   2. Cuppen divide and conquer on T (dc.cu),
 //   3. back-transformation of the kept eigenvectors with the Householder reflectors
 //      in blocks of 64 (compact WY, three GEMMs per block; every block's T factor is
 //      formed up front in one launch).
@@ -24,11 +20,7 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstdlib>
-#include <functional>
-#include <map>
-#include <mutex>
-#include <numeric>
+#include <cstring>
 
 namespace nsg {
 
@@ -37,7 +29,6 @@ static void raise_smem_limit(const void* fn, int bytes) { ensure_smem_limit(fn, 
 
 namespace {
 
-constexpr int kLeaf = 32;
 constexpr int kTriUnits = 1024;  // pass work units per CTA and step (columns x row blocks)
 
 __device__ __forceinline__ double cre(double v) { return v; }
@@ -173,10 +164,19 @@ __device__ __forceinline__ void hh_scalars_warp(T alpha, double xnorm2, int lane
   }
 }
 
+// The last subdiagonal entry has no reflector to make it real: for complex data its
+// modulus is T's entry and its phase goes to *phase (the back-transformation multiplies
+// the last row by it).
+__device__ __forceinline__ double last_offdiagonal(double a, double2*) { return a; }
+__device__ __forceinline__ double last_offdiagonal(double2 a, double2* phase) {
+  const double r = hypot(a.x, a.y);
+  *phase = r > 0 ? make_double2(a.x / r, a.y / r) : make_double2(1.0, 0.0);
+  return r;
+}
+
 // Householder tridiagonalisation of the Hermitian n x n matrix A (column-major, both
 // triangles stored).  On exit d[k] = T_kk, e[k] = T_k,k+1 (real), tau[k], the reflector
-// vectors v_k (v_k[k+1] = 1 implicit) below the subdiagonal of column k, and
-// A[n-1, n-2] updated (its phase is handled by the caller for complex A).
+// vectors v_k (v_k[k+1] = 1 implicit) below the subdiagonal of column k.
 // Step k: reflector from column k; x = tau A22 v; w = x - tau/2 (x^H v) v;
 // A22 -= v w^H + w v^H.  The rank-2 update of step k-1 is applied lazily: every CTA
 // rebuilds the updated pivot column itself, and one pass over the trailing block both
@@ -188,7 +188,8 @@ __device__ __forceinline__ void hh_scalars_warp(T alpha, double xnorm2, int lane
 template <typename T, int NT>
 __global__ void __launch_bounds__(NT)
     tridiag_kernel(T* __restrict__ A, int n, double* __restrict__ d, double* __restrict__ e, T* __restrict__ tau,
-                   T* __restrict__ xbuf, T* __restrict__ partial, Barrier* bar, int per_thread) {
+                   T* __restrict__ xbuf, T* __restrict__ partial, Barrier* bar, int per_thread,
+                   double2* __restrict__ phase) {
   extern __shared__ unsigned char smem_raw[];
   T* vprev = (T*)smem_raw;  // pending update (relative to rows >= k)
   T* wprev = vprev + n;
@@ -508,9 +509,8 @@ __global__ void __launch_bounds__(NT)
     if (n >= 2) {
       T a11 = upd(n - 2, n - 2), a21 = upd(n - 1, n - 2), a22 = upd(n - 1, n - 1);
       d[n - 2] = cre(a11);
-      e[n - 2] = cre(a21);
+      e[n - 2] = last_offdiagonal(a21, phase);
       d[n - 1] = cre(a22);
-      A[(n - 1) + (size_t)(n - 2) * n] = a21;
     } else {
       d[0] = cre(A[0]);
     }
@@ -532,7 +532,7 @@ constexpr int kClusterTriThreads = 256;
 template <typename T>
 __global__ void __launch_bounds__(kClusterTriThreads)
     tridiag_cluster_kernel(T* __restrict__ A, int n, double* __restrict__ d, double* __restrict__ e,
-                           T* __restrict__ tau) {
+                           T* __restrict__ tau, double2* __restrict__ phase) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int C = int(cluster.num_blocks());
@@ -696,8 +696,7 @@ __global__ void __launch_bounds__(kClusterTriThreads)
       const T* c2 = cols + (size_t)((n - 2) / C) * n;
       const T a11 = c2[n - 2], a21 = c2[n - 1];
       d[n - 2] = cre(a11);
-      e[n - 2] = cre(a21);
-      A[(n - 1) + (size_t)(n - 2) * n] = a21;
+      e[n - 2] = last_offdiagonal(a21, phase);
     }
     if (rank == o1 && tid == 0) d[n - 1] = cre(cols[(size_t)((n - 1) / C) * n + (n - 1)]);
   } else if (rank == 0 && tid == 0) {
@@ -706,756 +705,22 @@ __global__ void __launch_bounds__(kClusterTriThreads)
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
-// For complex A the last subdiagonal element may be complex: handled on the host by a
-// unitary diagonal scaling (phase folded into the back-transformation).
-
-// ---------------------------------------------------------------------------
-// divide and conquer
-// ---------------------------------------------------------------------------
-
-struct MergeDesc {
-  int lo, mid, hi;
-  double beta;
-};
-
-
-// Scatter leaf eigenpairs into Q (n x n, column-major) and w, sorted ascending.
-// Leaves of the divide and conquer: the symmetric tridiagonal blocks (order <= 32) are
-// diagonalised by the implicit QL method with Wilkinson shifts (Givens chase from the
-// bottom of the unreduced block to its top), one warp per leaf.  Lane 0 runs each
-// chase's scalar recurrence and records its rotations; then every lane applies them, in
-// order, to its own row of the eigenvector matrix Z (columns = eigenvectors).  The
-// eigenpairs are sorted ascending and written into the leaf's diagonal block of Q and w.
-// A block that fails to converge in 60 chases per eigenvalue raises *err.
-constexpr int kLeafWarps = 4;
-__global__ void __launch_bounds__(32 * kLeafWarps)
-    leaf_ql_kernel(const double* __restrict__ dsrc, const double* __restrict__ esrc, const int* leaf_lo,
-                   const int* leaf_hi, int nleaf, double* Q, int n, double* w, int* err) {
-  __shared__ double Zs[kLeafWarps][kLeaf][kLeaf + 1];
-  __shared__ double ds_[kLeafWarps][kLeaf], es_[kLeafWarps][kLeaf], cs_[kLeafWarps][kLeaf],
-      sn_[kLeafWarps][kLeaf];
-  __shared__ int ord_[kLeafWarps][kLeaf];
-  const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int L = blockIdx.x * kLeafWarps + wl;
-  if (L >= nleaf) return;  // whole warps only
-  const int lo = leaf_lo[L], s = leaf_hi[L] - lo;
-  double(*Z)[kLeaf + 1] = Zs[wl];
-  double* d = ds_[wl];
-  double* e = es_[wl];
-  for (int c = 0; c < kLeaf; ++c) Z[lane][c] = (lane == c) ? 1.0 : 0.0;
-  if (lane < s) {
-    d[lane] = dsrc[lo + lane];
-    e[lane] = (lane + 1 < s) ? esrc[lo + lane] : 0.0;
-  }
-  __syncwarp();
-  const double eps = 2.220446049250313e-16;
-  bool failed = false;
-  for (int l = 0; l < s && !failed; ++l) {
-    for (int iter = 0;; ++iter) {
-      int m = l;
-      while (m < s - 1) {
-        const double dd = fabs(d[m]) + fabs(d[m + 1]);
-        if (fabs(e[m]) <= eps * dd) break;
-        ++m;
-      }
-      if (m == l) break;
-      if (iter == 60) {
-        failed = true;
-        break;
-      }
-      int lowest = l;  // rotations recorded for i = m-1 .. lowest
-      if (lane == 0) {
-        double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-        double r = sqrt(g * g + 1.0);
-        g = d[m] - d[l] + e[l] / (g + (g >= 0.0 ? r : -r));
-        double sv = 1.0, cv = 1.0, p = 0.0;
-        int i = m - 1;
-        for (; i >= l; --i) {
-          const double f = sv * e[i], b = cv * e[i];
-          r = sqrt(f * f + g * g);
-          e[i + 1] = r;
-          if (r == 0.0) {  // the block splits: undo the pending shift and restart
-            d[i + 1] -= p;
-            e[m] = 0.0;
-            break;
-          }
-          const double ir = 1.0 / r;
-          sv = f * ir;
-          cv = g * ir;
-          g = d[i + 1] - p;
-          r = (d[i] - g) * sv + 2.0 * cv * b;
-          p = sv * r;
-          d[i + 1] = g + p;
-          g = cv * r - b;
-          cs_[wl][i] = cv;
-          sn_[wl][i] = sv;
-        }
-        if (i < l) {
-          d[l] -= p;
-          e[l] = g;
-          e[m] = 0.0;
-        } else {
-          lowest = i + 1;
-        }
-        ord_[wl][0] = lowest;
-      }
-      __syncwarp();
-      lowest = ord_[wl][0];
-      // each lane rotates its row of Z through the chase's rotations, in order
-      for (int i = m - 1; i >= lowest; --i) {
-        const double cv = cs_[wl][i], sv = sn_[wl][i];
-        const double f = Z[lane][i + 1], zi = Z[lane][i];
-        Z[lane][i + 1] = sv * zi + cv * f;
-        Z[lane][i] = cv * zi - sv * f;
-      }
-      __syncwarp();
-    }
-  }
-  if (failed && lane == 0) atomicExch(err, 1);
-  // ascending order (insertion sort by lane 0), then the leaf's block of Q and w
-  if (lane == 0) {
-    int* o = ord_[wl];
-    for (int a = 0; a < s; ++a) o[a] = a;
-    for (int a = 1; a < s; ++a) {
-      const int x = o[a];
-      int b2 = a - 1;
-      while (b2 >= 0 && d[o[b2]] > d[x]) {
-        o[b2 + 1] = o[b2];
-        --b2;
-      }
-      o[b2 + 1] = x;
-    }
-  }
-  __syncwarp();
-  if (lane < s) {
-    for (int j = 0; j < s; ++j) Q[(size_t)(lo + j) * n + (lo + lane)] = Z[lane][ord_[wl][j]];
-    w[lo + lane] = d[ord_[wl][lane]];
+// Eigenvectors first, first + step, ... of T (columns of Q) as the columns of Z, the last
+// row times the phase of T's last subdiagonal entry.
+__global__ void gather_vectors_kernel(const double* __restrict__ Q, int64_t n, int64_t first, int64_t step,
+                                      int64_t count, double* __restrict__ Z, int64_t ldz, const double2*) {
+  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n * count; e += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = e % n, j = e / n;
+    Z[i + j * ldz] = Q[i + (first + j * step) * n];
   }
 }
-
-
-// Merges of the divide and conquer, one tree level at a time: every kernel below
-// handles all merges of a level in one launch (blockIdx.y or the warp index selects the
-// merge), so a level costs a fixed handful of launches and one host read of the
-// deflation counts, whatever the number of merges.
-//
-// Workspace (device arrays of length n; a merge uses the slice [lo, hi) of each):
-//   Ds, zs     sorted (sign-flipped) poles and normalised z, 0 for deflated slots
-//   perm       block-local column of sorted slot t
-//   kind       1 = non-deflated, 0 = deflated
-//   kinv       sorted slot of the q-th non-deflated pole
-//   Dk, zk     the non-deflated poles and weights, compacted
-//   lam, zh    secular roots and Gu-Eisenstat weights (first k entries)
-//   srck, srci, wn   final ordering: source kind / index and eigenvalue of output column
-//   rot_pq, rot_cs   deflation rotations (2 entries each per rotation, at 2 lo)
-//   gscr       scratch of the serial steps for blocks above the shared-memory limit
-// Per merge: rho, counts (k, nrot, flip).
-struct DcWork {
-  double *Ds, *zs, *Dk, *zk, *lam, *zh, *wn, *rot_cs, *gscr;
-  int *perm, *kind, *kinv, *srck, *srci, *rot_pq;
-  double* rho;
-  int* counts;
-};
-
-constexpr int kSmemMerge = 4096;  // rows of a block whose serial steps run in shared memory
-
-// Order-preserving integer key of a double (x < y exactly when key(x) < key(y); -0 and +0
-// equal), so the merges compare with integer instructions rather than the FP64 pipe,
-// and the exact negation -x by its sign bit.
-__device__ __forceinline__ long long order_key(double x) {
-  const long long b = __double_as_longlong(x);
-  if ((b & 0x7fffffffffffffffLL) == 0) return 0;
-  return b < 0 ? (b ^ 0x7fffffffffffffffLL) : b;
-}
-__device__ __forceinline__ double neg_exact(double x) {
-  return __longlong_as_double(__double_as_longlong(x) ^ (long long)(1ULL << 63));
-}
-
-// Exclusive prefix sum of v over the block's threads in thread order (sh: 32 ints);
-// the block total goes to *tot.  Every thread of the block must call it.
-__device__ int block_scan_excl(int v, int* sh, int* tot) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  int x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) sh[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    int t = lane < nw ? sh[lane] : 0;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
-    }
-    if (lane < nw) sh[lane] = t;
-  }
-  __syncthreads();
-  const int before = warp > 0 ? sh[warp - 1] : 0;
-  *tot = sh[nw - 1];
-  __syncthreads();
-  return before + x - v;
-}
-
-// Number of indices i in [0, len) with key(i) < k (strict) or key(i) <= k, for keys
-// ascending in i.
-template <bool kStrict, typename F>
-__device__ __forceinline__ int rank_in(F key, int len, long long k) {
-  int lo = 0, hi = len;
-  while (lo < hi) {
-    const int md = (lo + hi) >> 1;
-    const long long v = key(md);
-    if (kStrict ? (v < k) : (v <= k))
-      lo = md + 1;
-    else
-      hi = md;
-  }
-  return lo;
-}
-
-// Per merge (one CTA): gather the two halves' eigenvalues and the z vector (last row of
-// block 1, first row of block 2), flip for rho < 0, merge the ascending halves, normalise
-// z, deflate (small z_t; poles closer than tol rotated together), apply the deflation
-// rotations to the block's columns of Q, and compact the non-deflated poles.
-__global__ void dc_prep_kernel(const double* __restrict__ w, double* __restrict__ Q, int n,
-                               const MergeDesc* __restrict__ md, DcWork W) {
-  extern __shared__ double dp_smem[];
-  const int mi = blockIdx.x;
-  const MergeDesc M = md[mi];
-  const int lo = M.lo, mid = M.mid, hi = M.hi, nb = hi - lo, n1 = mid - lo;
-  const bool sm = nb <= kSmemMerge;
-  double* ws = sm ? dp_smem : W.gscr + 2 * (size_t)lo;  // block eigenvalues by local index
-  double* zr = ws + nb;                                  // z candidates by local index
-  double* Dsm = sm ? zr + nb : W.Ds + lo;
-  double* zsm = sm ? Dsm + nb : W.zs + lo;
-  int* pm = sm ? (int*)(zsm + nb) : W.perm + lo;
-  int* kd = sm ? pm + nb : W.kind + lo;
-  __shared__ double red[32], redm[32];
-  __shared__ int scan_sh[32], s_flag, s_nrot;
-  for (int li = threadIdx.x; li < nb; li += blockDim.x) {
-    ws[li] = w[lo + li];
-    zr[li] = (li < n1) ? Q[(size_t)(lo + li) * n + (mid - 1)] : Q[(size_t)(lo + li) * n + mid];
-  }
-  if (threadIdx.x == 0) {
-    s_flag = 0;
-    s_nrot = 0;
-  }
-  __syncthreads();
-  double rho = M.beta;
-  const int flip = rho < 0;
-  if (flip) rho = -rho;
-  // merge of the two ascending halves (both traversed from their top when flipped, values
-  // negated) into ascending poles; ties take the first half first.  An entry's slot is
-  // its rank in its own half plus its rank in the other, by binary search on integer keys.
-  const int n2 = nb - n1;
-  auto srcA = [&](int a) { return flip ? (n1 - 1 - a) : a; };
-  auto srcB = [&](int b2) { return flip ? (nb - 1 - b2) : (n1 + b2); };
-  auto valA = [&](int a) { return flip ? neg_exact(ws[srcA(a)]) : ws[srcA(a)]; };
-  auto valB = [&](int b2) { return flip ? neg_exact(ws[srcB(b2)]) : ws[srcB(b2)]; };
-  auto keyA = [&](int a) { return order_key(valA(a)); };
-  auto keyB = [&](int b2) { return order_key(valB(b2)); };
-  for (int t = threadIdx.x; t < nb; t += blockDim.x)  // halves out of order: the serial merge
-    if ((t > 0 && t < n1 && keyA(t) < keyA(t - 1)) || (t > n1 && keyB(t - n1) < keyB(t - n1 - 1))) s_flag = 1;
-  __syncthreads();
-  if (!s_flag) {
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      int pos, li;
-      if (t < n1) {
-        pos = t + rank_in<true>(keyB, n2, keyA(t));
-        li = srcA(t);
-      } else {
-        pos = (t - n1) + rank_in<false>(keyA, n1, keyB(t - n1));
-        li = srcB(t - n1);
-      }
-      pm[pos] = li;
-      Dsm[pos] = flip ? neg_exact(ws[li]) : ws[li];
-      zsm[pos] = zr[li];
-    }
-  } else if (threadIdx.x == 0) {
-    int a = 0, b2 = 0;
-    for (int t = 0; t < nb; ++t) {
-      bool takeA;
-      if (a >= n1)
-        takeA = false;
-      else if (b2 >= n2)
-        takeA = true;
-      else
-        takeA = keyA(a) <= keyB(b2);
-      const int li = takeA ? srcA(a) : srcB(b2);
-      if (takeA)
-        ++a;
-      else
-        ++b2;
-      pm[t] = li;
-      Dsm[t] = flip ? neg_exact(ws[li]) : ws[li];
-      zsm[t] = zr[li];
-    }
-  }
-  __syncthreads();
-  // |z| and max |D| (fixed-order block reductions)
-  double s2 = 0.0, dm = 0.0;
-  for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-    s2 += zsm[t] * zsm[t];
-    dm = fmax(dm, fabs(Dsm[t]));
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    dm = fmax(dm, __shfl_xor_sync(0xffffffffu, dm, o));
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  if (lane == 0) {
-    red[warp] = s2;
-    redm[warp] = dm;
-  }
-  __syncthreads();
-  double nz = 0.0, dmax = 0.0;
-  for (int q = 0; q < nw; ++q) {
-    nz += red[q];
-    dmax = fmax(dmax, redm[q]);
-  }
-  nz = sqrt(nz);
-  rho = rho * nz * nz;
-  const double tol = 8.0 * 2.220446049250313e-16 * fmax(dmax, rho);
-  // deflation of small weights (independent per pole), then of poles closer than tol:
-  // the sorted poles' closest kept pair is consecutive among the kept ones, so a pass
-  // that finds none proves that the serial rotation sweep would rotate nothing
-  for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-    const double z = zsm[t] / nz;
-    const bool small = rho * fabs(z) <= tol;
-    kd[t] = small ? 0 : 1;
-    zsm[t] = small ? 0.0 : z;
-  }
-  if (threadIdx.x == 0) s_flag = 0;
-  __syncthreads();
-  for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-    if (!kd[t]) continue;
-    for (int u = t + 1; u < nb; ++u)
-      if (kd[u]) {
-        if (fabs(Dsm[u] - Dsm[t]) <= tol) s_flag = 1;
-        break;
-      }
-  }
-  __syncthreads();
-  int* rpq = W.rot_pq + 2 * lo;
-  double* rcs = W.rot_cs + 2 * lo;
-  if (s_flag && threadIdx.x == 0) {
-    int nrot = 0, prev = -1;
-    for (int t = 0; t < nb; ++t) {
-      if (!kd[t]) continue;
-      if (prev >= 0 && fabs(Dsm[t] - Dsm[prev]) <= tol) {
-        const double r = hypot(zsm[t], zsm[prev]);
-        const double c = zsm[t] / r, sn = zsm[prev] / r;
-        const double dp = Dsm[prev], dt = Dsm[t];
-        Dsm[prev] = c * c * dp + sn * sn * dt;
-        Dsm[t] = sn * sn * dp + c * c * dt;
-        zsm[prev] = 0.0;
-        zsm[t] = r;
-        kd[prev] = 0;
-        rpq[2 * nrot] = pm[prev];
-        rpq[2 * nrot + 1] = pm[t];
-        rcs[2 * nrot] = c;
-        rcs[2 * nrot + 1] = sn;
-        ++nrot;
-      }
-      prev = t;
-    }
-    s_nrot = nrot;
-  }
-  __syncthreads();
-  // compaction of the non-deflated slots (block scan over contiguous chunks)
-  {
-    const int per = (nb + blockDim.x - 1) / blockDim.x;
-    const int c0 = min(nb, (int)threadIdx.x * per), c1 = min(nb, c0 + per);
-    int cnt = 0;
-    for (int t = c0; t < c1; ++t) cnt += kd[t];
-    int k = 0;
-    int off = block_scan_excl(cnt, scan_sh, &k);
-    int* kinv = W.kinv + lo;
-    double* Dk = W.Dk + lo;
-    double* zk = W.zk + lo;
-    for (int t = c0; t < c1; ++t)
-      if (kd[t]) {
-        kinv[off] = t;
-        Dk[off] = Dsm[t];
-        zk[off] = zsm[t];
-        ++off;
-      }
-    if (threadIdx.x == 0) {
-      W.rho[mi] = rho;
-      W.counts[3 * mi] = k;
-      W.counts[3 * mi + 1] = s_nrot;
-      W.counts[3 * mi + 2] = flip;
-    }
-  }
-  if (sm) {
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      W.Ds[lo + t] = Dsm[t];
-      W.zs[lo + t] = zsm[t];
-      W.perm[lo + t] = pm[t];
-      W.kind[lo + t] = kd[t];
-    }
-  }
-}
-
-// The deflation rotations of every merge of a level, in order, on the block's columns of
-// Q: one thread per row (blockIdx.y = merge), so a merge's rows are spread over many SMs
-// and each thread's chain of dependent rotations is one row long.
-__global__ void dc_rotate_kernel(double* __restrict__ Q, int n, const MergeDesc* __restrict__ md, DcWork W) {
-  const int mi = blockIdx.y;
-  const int nrot = W.counts[3 * mi + 1];
-  if (nrot == 0) return;
-  const int lo = md[mi].lo, nb = md[mi].hi - lo;
-  const int* rpq = W.rot_pq + 2 * lo;
-  const double* rcs = W.rot_cs + 2 * lo;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nb; r += gridDim.x * blockDim.x) {
-    double* row = Q + (lo + r);
-    for (int q = 0; q < nrot; ++q) {
-      const size_t cp = (size_t)(lo + rpq[2 * q]) * n, ci = (size_t)(lo + rpq[2 * q + 1]) * n;
-      const double c = rcs[2 * q], sn = rcs[2 * q + 1];
-      const double xp = row[cp], xi = row[ci];
-      row[cp] = c * xp - sn * xi;
-      row[ci] = sn * xp + c * xi;
-    }
-  }
-}
-
-// Secular roots: one warp per (merge, root).  Root i of 1 + rho sum_j z_j^2 / (D_j - lambda)
-// lies in (D_i, D_{i+1}) (the last one in (D_{k-1}, D_{k-1} + rho)); it is represented as
-// origin + tau with the origin at the nearer pole, so D_j - lambda = (D_j - origin) - tau
-// is exact enough for the Gu-Eisenstat vectors.  Iteration: the two-pole rational model
-// of Bunch, Nielsen and Sorensen (psi for poles j <= i, phi for j > i, each matched in
-// value and slope at tau), solved as a quadratic inside the bracket; bisection when the
-// model step leaves the bracket.  Delta_m[i * k + j] = D_j - lambda_i (block of kmax^2).
-__global__ void dc_secular_kernel(const MergeDesc* __restrict__ md, int nm, int kmax, DcWork W,
-                                  double* __restrict__ Delta_all) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (gw >= (int64_t)nm * kmax) return;
-  const int mi = int(gw / kmax), i = int(gw % kmax);
-  const int k = W.counts[3 * mi];
-  if (i >= k) return;
-  const int lo = md[mi].lo;
-  const double* Dk = W.Dk + lo;
-  const double* zk = W.zk + lo;
-  const double rho = W.rho[mi];
-  double* Delta = Delta_all + (size_t)mi * kmax * kmax;
-  const double eps = 2.220446049250313e-16;
-  int org;
-  double blo, bhi;
-  if (i < k - 1) {
-    const double gap = Dk[i + 1] - Dk[i];
-    const double mid = 0.5 * gap;  // relative to D_i
-    double f = 0.0;
-    for (int j = lane; j < k; j += 32) f += rho * zk[j] * zk[j] / ((Dk[j] - Dk[i]) - mid);
-    for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
-    f += 1.0;
-    if (f >= 0) {
-      org = i;
-      blo = 0.0;
-      bhi = mid;
-    } else {
-      org = i + 1;
-      blo = -mid;
-      bhi = 0.0;
-    }
-  } else {
-    org = k - 1;
-    blo = 0.0;
-    bhi = rho;
-  }
-  const double dorg = Dk[org];
-  const double ddi = Dk[i] - dorg;
-  const double ddi1 = (i < k - 1) ? Dk[i + 1] - dorg : 0.0;
-  double tau = 0.5 * (blo + bhi);
-  for (int it = 0; it < 100; ++it) {
-    double psi = 0.0, dpsi = 0.0, phi = 0.0, dphi = 0.0, fa = 0.0;
-    for (int j = lane; j < k; j += 32) {
-      const double del = (Dk[j] - dorg) - tau;
-      const double q = zk[j] / del;
-      const double term = rho * zk[j] * q;
-      const double dterm = rho * q * q;
-      if (j <= i) {
-        psi += term;
-        dpsi += dterm;
-      } else {
-        phi += term;
-        dphi += dterm;
-      }
-      fa += fabs(term);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      psi += __shfl_xor_sync(0xffffffffu, psi, o);
-      dpsi += __shfl_xor_sync(0xffffffffu, dpsi, o);
-      phi += __shfl_xor_sync(0xffffffffu, phi, o);
-      dphi += __shfl_xor_sync(0xffffffffu, dphi, o);
-      fa += __shfl_xor_sync(0xffffffffu, fa, o);
-    }
-    const double f = 1.0 + psi + phi;
-    if (f > 0)
-      bhi = tau;
-    else
-      blo = tau;
-    if (fabs(f) <= 4.0 * eps * (k + 1.0) * (1.0 + fa)) break;
-    if (bhi - blo <= 2.0 * eps * fmax(fabs(blo), fabs(bhi)) || bhi - blo < 1e-300) break;
-    double tn;
-    const double di = ddi - tau;
-    const double b1 = dpsi * di * di, a1 = psi - b1 / di;
-    if (i < k - 1) {
-      const double di1 = ddi1 - tau;
-      const double b2 = dphi * di1 * di1, a2 = phi - b2 / di1;
-      const double C = 1.0 + a1 + a2;
-      // C (ddi - x)(ddi1 - x) + b1 (ddi1 - x) + b2 (ddi - x) = 0
-      const double qa = C, qb = -(C * (ddi + ddi1) + b1 + b2), qc = C * ddi * ddi1 + b1 * ddi1 + b2 * ddi;
-      tn = NAN;
-      if (qa != 0.0) {
-        const double disc = qb * qb - 4.0 * qa * qc;
-        if (disc >= 0.0) {
-          const double sq = sqrt(disc);
-          const double qq = -0.5 * (qb + copysign(sq, qb));
-          const double r1 = qq / qa, r2 = (qq != 0.0) ? qc / qq : NAN;
-          if (r1 > blo && r1 < bhi)
-            tn = r1;
-          else if (r2 > blo && r2 < bhi)
-            tn = r2;
-        }
-      } else if (qb != 0.0) {
-        tn = -qc / qb;
-      }
-    } else {
-      // 1 + phi_const + a1 + b1/(ddi - x) = 0 with phi == 0
-      const double C = 1.0 + a1 + phi;
-      tn = (C != 0.0) ? ddi + b1 / C : NAN;
-    }
-    if (!(tn > blo && tn < bhi)) tn = 0.5 * (blo + bhi);
-    if (tn == tau) break;
-    tau = tn;
-  }
-  if (lane == 0) W.lam[lo + i] = dorg + tau;
-  for (int j = lane; j < k; j += 32) Delta[(size_t)i * k + j] = (Dk[j] - dorg) - tau;
-}
-
-// Gu-Eisenstat: zhat_j^2 = (lam_j - D_j)/rho * prod_{i != j} (lam_i - D_j)/(D_i - D_j);
-// one warp per (merge, j).
-__global__ void dc_gu_eisenstat_kernel(const MergeDesc* __restrict__ md, int nm, int kmax, DcWork W,
-                                       const double* __restrict__ Delta_all) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (gw >= (int64_t)nm * kmax) return;
-  const int mi = int(gw / kmax), j = int(gw % kmax);
-  const int k = W.counts[3 * mi];
-  if (j >= k) return;
-  const int lo = md[mi].lo;
-  const double* Dk = W.Dk + lo;
-  const double* Delta = Delta_all + (size_t)mi * kmax * kmax;
-  double p = 1.0;
-  for (int i = lane; i < k; i += 32)
-    if (i != j) p *= (-Delta[(size_t)i * k + j]) / (Dk[i] - Dk[j]);
-  for (int o = 16; o > 0; o >>= 1) p *= __shfl_xor_sync(0xffffffffu, p, o);
-  p *= -Delta[(size_t)j * k + j] / W.rho[mi];
-  if (lane == 0) W.zh[lo + j] = copysign(sqrt(fmax(p, 0.0)), W.zk[lo + j]);
-}
-
-// S^T of each merge (kmax x kmax, column-major, zero outside its k x k block: column i =
-// normalised eigenvector of root i); one warp per (merge, column).
-__global__ void dc_vectors_kernel(const MergeDesc* __restrict__ md, int nm, int kmax, DcWork W,
-                                  const double* __restrict__ Delta_all, double* __restrict__ St_all) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (gw >= (int64_t)nm * kmax) return;
-  const int mi = int(gw / kmax), i = int(gw % kmax);
-  const int k = W.counts[3 * mi];
-  double* St = St_all + (size_t)mi * kmax * kmax + (size_t)i * kmax;
-  if (i >= k) {
-    for (int j = lane; j < kmax; j += 32) St[j] = 0.0;
-    return;
-  }
-  const double* zh = W.zh + md[mi].lo;
-  const double* Delta = Delta_all + (size_t)mi * kmax * kmax + (size_t)i * k;
-  double nrm = 0.0;
-  for (int j = lane; j < k; j += 32) {
-    const double s = zh[j] / Delta[j];
-    nrm += s * s;
-  }
-  for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-  nrm = 1.0 / sqrt(nrm);
-  for (int j = lane; j < kmax; j += 32) St[j] = (j < k) ? zh[j] / Delta[j] * nrm : 0.0;
-}
-
-// The non-deflated (rotated) columns of each block, compacted into an nbmax x kmax
-// matrix per merge (zero padded); blockIdx.y = merge.
-__global__ void dc_gather_kernel(const double* __restrict__ Q, int n, const MergeDesc* __restrict__ md, int nbmax,
-                                 int kmax, DcWork W, double* __restrict__ Qk_all) {
-  const int mi = blockIdx.y;
-  const int lo = md[mi].lo, nb = md[mi].hi - lo, k = W.counts[3 * mi];
-  double* Qk = Qk_all + (size_t)mi * nbmax * kmax;
-  const size_t tot = (size_t)nbmax * kmax;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    const int r = int(e % nbmax), q = int(e / nbmax);
-    double v = 0.0;
-    if (r < nb && q < k) v = Q[(size_t)(lo + W.perm[lo + W.kinv[lo + q]]) * n + (lo + r)];
-    Qk[e] = v;
-  }
-}
-
-// Final ordering of each block (one CTA per merge): eigenvalues = roots (non-deflated)
-// and deflated poles, signs undone, ascending; the source of each output column.
-__global__ void dc_order_kernel(const MergeDesc* __restrict__ md, DcWork W) {
-  extern __shared__ double mo_smem[];
-  const int mi = blockIdx.x;
-  const int lo = md[mi].lo, nb = md[mi].hi - lo;
-  const int nr = W.counts[3 * mi], flip = W.counts[3 * mi + 2], nd = nb - nr;
-  const bool sm = nb <= kSmemMerge;
-  double* Dsm = sm ? mo_smem : W.Ds + lo;
-  double* lm = sm ? Dsm + nb : W.lam + lo;
-  double* wo = sm ? lm + nb : W.wn + lo;
-  int* kd = sm ? (int*)(wo + nb) : W.kind + lo;
-  int* sk = sm ? kd + nb : W.srck + lo;
-  int* si = sm ? sk + nb : W.srci + lo;
-  if (sm) {
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      Dsm[t] = W.Ds[lo + t];
-      kd[t] = W.kind[lo + t];
-    }
-    for (int t = threadIdx.x; t < nr; t += blockDim.x) lm[t] = W.lam[lo + t];
-  }
-  __syncthreads();
-  // the deflated slots in order (block scan), then a stable merge of the ascending roots
-  // with the deflated poles (ties: the root first) by ranks on integer keys; poles moved
-  // by a deflation rotation can be out of order by up to the deflation tolerance, and
-  // then the merge is the serial one
-  __shared__ int scan_sh[32], s_unsorted;
-  int* dl = si;  // deflated slots, in the output index array until the outputs are formed
-  {
-    const int per = (nb + blockDim.x - 1) / blockDim.x;
-    const int c0 = min(nb, (int)threadIdx.x * per), c1 = min(nb, c0 + per);
-    int cnt = 0;
-    for (int t = c0; t < c1; ++t) cnt += 1 - kd[t];
-    int tot = 0;
-    int off = block_scan_excl(cnt, scan_sh, &tot);
-    for (int t = c0; t < c1; ++t)
-      if (!kd[t]) dl[off++] = t;
-  }
-  // (each thread keeps its ranks in registers: at most 16 entries of each kind)
-  if (threadIdx.x == 0) s_unsorted = nb > 16 * (int)blockDim.x;
-  __syncthreads();
-  auto keyR = [&](int i) { return order_key(lm[i]); };
-  auto keyD = [&](int j) { return order_key(Dsm[dl[j]]); };
-  for (int i = threadIdx.x + 1; i < nr; i += blockDim.x)
-    if (keyR(i) < keyR(i - 1)) s_unsorted = 1;
-  for (int j = threadIdx.x + 1; j < nd; j += blockDim.x)
-    if (keyD(j) < keyD(j - 1)) s_unsorted = 1;
-  __syncthreads();
-  if (!s_unsorted) {
-    // ranks first (every thread reads dl), then the outputs (which overwrite si = dl)
-    int posr[16], posd[16];
-    int nrl = 0, ndl = 0;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) posr[nrl++] = i + rank_in<true>(keyD, nd, keyR(i));
-    for (int j = threadIdx.x; j < nd; j += blockDim.x) posd[ndl++] = j + rank_in<false>(keyR, nr, keyD(j));
-    int slots[16];
-    ndl = 0;
-    for (int j = threadIdx.x; j < nd; j += blockDim.x) slots[ndl++] = dl[j];
-    __syncthreads();
-    nrl = 0;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-      const int pos = posr[nrl++], out = flip ? (nb - 1 - pos) : pos;
-      sk[out] = 1;
-      si[out] = i;
-      wo[out] = flip ? neg_exact(lm[i]) : lm[i];
-    }
-    ndl = 0;
-    for (int j = threadIdx.x; j < nd; j += blockDim.x) {
-      const int pos = posd[ndl], slot = slots[ndl++], out = flip ? (nb - 1 - pos) : pos;
-      sk[out] = 0;
-      si[out] = slot;
-      wo[out] = flip ? neg_exact(Dsm[slot]) : Dsm[slot];
-    }
-  } else if (threadIdx.x == 0) {
-    int ia = 0, ib = 0, pos = 0, dslot = 0;
-    while (dslot < nb && kd[dslot]) ++dslot;
-    while (ia < nr || ib < nd) {
-      bool takeRoot;
-      if (ia >= nr)
-        takeRoot = false;
-      else if (ib >= nd)
-        takeRoot = true;
-      else
-        takeRoot = lm[ia] <= Dsm[dslot];
-      const int out = flip ? (nb - 1 - pos) : pos;
-      if (takeRoot) {
-        sk[out] = 1;
-        si[out] = ia;
-        wo[out] = flip ? -lm[ia] : lm[ia];
-        ++ia;
-      } else {
-        sk[out] = 0;
-        si[out] = dslot;
-        wo[out] = flip ? -Dsm[dslot] : Dsm[dslot];
-        ++ib;
-        ++dslot;
-        while (dslot < nb && kd[dslot]) ++dslot;
-      }
-      ++pos;
-    }
-  }
-  __syncthreads();
-  if (sm) {
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-      W.srck[lo + t] = sk[t];
-      W.srci[lo + t] = si[t];
-      W.wn[lo + t] = wo[t];
-    }
-  }
-}
-
-// The merged block of every merge into T (same position as in Q): output column `out`
-// is merged column srci (src kind 1) or the deflated column of Q it came from; the new
-// eigenvalues into w.  blockIdx.y = merge.
-__global__ void dc_scatter_kernel(const double* __restrict__ Q, int n, const MergeDesc* __restrict__ md, int nbmax,
-                                  int kmax, DcWork W, const double* __restrict__ Qm_all, double* __restrict__ T,
-                                  double* __restrict__ w) {
-  const int mi = blockIdx.y;
-  const int lo = md[mi].lo, nb = md[mi].hi - lo;
-  const double* Qm = Qm_all + (size_t)mi * nbmax * kmax;
-  const size_t tot = (size_t)nb * nb;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    const int r = int(e % nb), out = int(e / nb);
-    const int src = W.srci[lo + out];
-    const double v = W.srck[lo + out] ? Qm[r + (size_t)src * nbmax]
-                                      : Q[(size_t)(lo + W.perm[lo + src]) * n + (lo + r)];
-    T[(size_t)(lo + out) * n + (lo + r)] = v;
-  }
-  if (blockIdx.x == 0)
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) w[lo + t] = W.wn[lo + t];
-}
-
-// T's merged blocks back into Q; blockIdx.y = merge.
-__global__ void dc_copy_kernel(const double* __restrict__ T, int n, const MergeDesc* __restrict__ md,
-                               double* __restrict__ Q) {
-  const int mi = blockIdx.y;
-  const int lo = md[mi].lo, nb = md[mi].hi - lo;
-  const size_t tot = (size_t)nb * nb;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    const size_t idx = (size_t)(lo + e / nb) * n + (lo + e % nb);
-    Q[idx] = T[idx];
-  }
-}
-
-// complex phases: T's subdiagonal is real by construction except possibly the last one
-__global__ void real_to_complex_kernel(const double* Zr, int64_t rows, int64_t cols, int64_t ldr, double2* Zc,
-                                       int64_t ldc) {
-  size_t tot = (size_t)rows * cols;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    int64_t i = e % rows, j = e / rows;
-    Zc[i + j * ldc] = make_double2(Zr[i + j * ldr], 0.0);
-  }
-}
-
-__global__ void scale_rows_phase_kernel(double2* Z, int64_t rows, int64_t cols, int64_t ld, const double2* ph) {
-  size_t tot = (size_t)rows * cols;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot; e += (size_t)gridDim.x * blockDim.x) {
-    int64_t i = e % rows, j = e / rows;
-    double2 z = Z[i + j * ld], p = ph[i];
-    Z[i + j * ld] = make_double2(p.x * z.x - p.y * z.y, p.x * z.y + p.y * z.x);
+__global__ void gather_vectors_kernel(const double* __restrict__ Q, int64_t n, int64_t first, int64_t step,
+                                      int64_t count, double2* __restrict__ Z, int64_t ldz, const double2* phase) {
+  const double2 ph = *phase;
+  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n * count; e += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = e % n, j = e / n;
+    const double v = Q[i + (first + j * step) * n];
+    Z[i + j * ldz] = i == n - 1 ? make_double2(ph.x * v, ph.y * v) : make_double2(v, 0.0);
   }
 }
 
@@ -1525,206 +790,34 @@ struct DevBuf {
   }
 };
 
-static void build_tree(int lo, int hi, std::vector<std::vector<MergeDesc>>& levels, std::vector<int>& leaf_lo,
-                       std::vector<int>& leaf_hi, int depth, int leaf) {
-  if (hi - lo <= leaf) {
-    leaf_lo.push_back(lo);
-    leaf_hi.push_back(hi);
-    return;
-  }
-  int mid = lo + (hi - lo) / 2;
-  build_tree(lo, mid, levels, leaf_lo, leaf_hi, depth + 1, leaf);
-  build_tree(mid, hi, levels, leaf_lo, leaf_hi, depth + 1, leaf);
-  if ((int)levels.size() <= depth) levels.resize(depth + 1);
-  levels[depth].push_back(MergeDesc{lo, mid, hi, 0.0});
-}
-
-// Leaf order of the divide and conquer: the implicit-QL leaves are one warp each and
-// latency bound (a chain of FP64 square roots and divides per rotation), so small leaves
-// and more (batched) merge levels are cheaper for one solve.  The context's override
-// (4..32) trades that latency for fewer levels: fewer launches and host reads.
-static int dc_leaf_size(const nsg_ctx* c) { return c->tune_dc_leaf > 0 ? c->tune_dc_leaf : 8; }
-
-// Eigen-decomposition of the real symmetric tridiagonal (d, e); Q: n x n (device,
-// column-major), w: eigenvalues ascending (device).  Cuppen's divide and conquer with
-// every merge of a tree level batched into one launch per step.
-static void tridiag_dc(nsg_ctx* c, int n, const std::vector<double>& d_in, const std::vector<double>& e_in, double* Q,
-                       double* w) {
-  std::vector<std::vector<MergeDesc>> levels;
-  std::vector<int> llo, lhi;
-  build_tree(0, n, levels, llo, lhi, 0, dc_leaf_size(c));
-  // modified diagonal: for each split subtract beta at the two touching diagonals
-  std::vector<double> d = d_in;
-  for (auto& lv : levels)
-    for (auto& m : lv) {
-      m.beta = e_in[m.mid - 1];
-      d[m.mid - 1] -= m.beta;
-      d[m.mid] -= m.beta;
-    }
-  DevBuf dd(c, sizeof(double) * n), de(c, sizeof(double) * std::max(n, 1));
-  NSG_CUDA(cudaMemcpyAsync(dd.p, d.data(), sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-  NSG_CUDA(cudaMemcpyAsync(de.p, e_in.data(), sizeof(double) * std::max<size_t>(e_in.size(), 1),
-                           cudaMemcpyHostToDevice, c->stream));
-  NSG_CUDA(cudaMemsetAsync(Q, 0, sizeof(double) * n * n, c->stream));
-  // leaves
-  int nleaf = int(llo.size());
-  DevBuf dlo(c, sizeof(int) * nleaf), dhi(c, sizeof(int) * nleaf);
-  NSG_CUDA(cudaMemcpyAsync(dlo.p, llo.data(), sizeof(int) * nleaf, cudaMemcpyHostToDevice, c->stream));
-  NSG_CUDA(cudaMemcpyAsync(dhi.p, lhi.data(), sizeof(int) * nleaf, cudaMemcpyHostToDevice, c->stream));
-  DevBuf lerr(c, sizeof(int));
-  NSG_CUDA(cudaMemsetAsync(lerr.p, 0, sizeof(int), c->stream));
-  {
-    ProfScope ps(c, NSG_PROF_DC, 0.0);
-    leaf_ql_kernel<<<(nleaf + kLeafWarps - 1) / kLeafWarps, 32 * kLeafWarps, 0, c->stream>>>(
-        dd.as<double>(), de.as<double>(), dlo.as<int>(), dhi.as<int>(), nleaf, Q, n, w, lerr.as<int>());
-  }
-  count_launch(c);
-  check_launch("dc leaves");
-  if (levels.empty()) {
-    int leaf_failed = 0;
-    NSG_CUDA(cudaMemcpyAsync(&leaf_failed, lerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaStreamSynchronize(c->stream));
-    NSG_CHECK(leaf_failed == 0, NSG_ERR_NONFINITE, "eigensolver: a tridiagonal leaf did not converge");
-    return;
-  }
-  // all levels' merge descriptors in one upload
-  std::vector<MergeDesc> all;
-  std::vector<size_t> off(levels.size());
-  for (int L = int(levels.size()) - 1; L >= 0; --L) {
-    off[L] = all.size();
-    all.insert(all.end(), levels[L].begin(), levels[L].end());
-  }
-  DevBuf bmd(c, sizeof(MergeDesc) * all.size());
-  NSG_CUDA(cudaMemcpyAsync(bmd.p, all.data(), sizeof(MergeDesc) * all.size(), cudaMemcpyHostToDevice, c->stream));
-  size_t maxm = 0;
-  for (auto& lv : levels) maxm = std::max(maxm, lv.size());
-  DevBuf bDs(c, sizeof(double) * n), bzs(c, sizeof(double) * n), bDk(c, sizeof(double) * n),
-      bzk(c, sizeof(double) * n), blam(c, sizeof(double) * n), bzh(c, sizeof(double) * n), bwn(c, sizeof(double) * n),
-      brcs(c, sizeof(double) * 2 * n), bscr(c, sizeof(double) * 2 * n), bperm(c, sizeof(int) * n),
-      bkind(c, sizeof(int) * n), bkinv(c, sizeof(int) * n), bsrck(c, sizeof(int) * n), bsrci(c, sizeof(int) * n),
-      brpq(c, sizeof(int) * 2 * n), brho(c, sizeof(double) * maxm), bcnt(c, sizeof(int) * 3 * maxm),
-      Tbuf(c, sizeof(double) * (size_t)n * n);
-  DcWork W;
-  W.Ds = bDs.as<double>();
-  W.zs = bzs.as<double>();
-  W.Dk = bDk.as<double>();
-  W.zk = bzk.as<double>();
-  W.lam = blam.as<double>();
-  W.zh = bzh.as<double>();
-  W.wn = bwn.as<double>();
-  W.rot_cs = brcs.as<double>();
-  W.gscr = bscr.as<double>();
-  W.perm = bperm.as<int>();
-  W.kind = bkind.as<int>();
-  W.kinv = bkinv.as<int>();
-  W.srck = bsrck.as<int>();
-  W.srci = bsrci.as<int>();
-  W.rot_pq = brpq.as<int>();
-  W.rho = brho.as<double>();
-  W.counts = bcnt.as<int>();
-  std::vector<int> cnt(3 * maxm);
-  bool leaves_checked = false;
-  for (int L = int(levels.size()) - 1; L >= 0; --L) {
-    const auto& lv = levels[L];
-    const int nm = int(lv.size());
-    const MergeDesc* md = bmd.as<MergeDesc>() + off[L];
-    int nbmax = 0;
-    for (auto& m : lv) nbmax = std::max(nbmax, m.hi - m.lo);
-    {
-      const int shm = nbmax <= kSmemMerge ? nbmax * 40 : 0;
-      if (shm) raise_smem_limit((const void*)dc_prep_kernel, shm);
-      ProfScope ps(c, NSG_PROF_DC, 0.0);
-      dc_prep_kernel<<<nm, 256, shm, c->stream>>>(w, Q, n, md, W);
-    }
-    count_launch(c);
-    check_launch("dc prep");
-    NSG_CUDA(cudaMemcpyAsync(cnt.data(), W.counts, sizeof(int) * 3 * nm, cudaMemcpyDeviceToHost, c->stream));
-    int leaf_failed = 0;
-    if (!leaves_checked)
-      NSG_CUDA(cudaMemcpyAsync(&leaf_failed, lerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaStreamSynchronize(c->stream));
-    if (!leaves_checked) {
-      NSG_CHECK(leaf_failed == 0, NSG_ERR_NONFINITE, "eigensolver: a tridiagonal leaf did not converge");
-      leaves_checked = true;
-    }
-    int kmax = 0, rotations = 0;
-    for (int mi = 0; mi < nm; ++mi) {
-      kmax = std::max(kmax, cnt[3 * mi]);
-      rotations += cnt[3 * mi + 1];
-    }
-    // the deflation rotations, launched only for a level that has some (the counts are
-    // on the host already for the batched product's extent)
-    if (rotations > 0) {
-      {
-        ProfScope ps(c, NSG_PROF_DC, 0.0);
-        dc_rotate_kernel<<<dim3((nbmax + 127) / 128, nm), 128, 0, c->stream>>>(Q, n, md, W);
-      }
-      count_launch(c);
-      check_launch("dc rotate");
-    }
-    const int gxe = int(std::max<int64_t>(1, std::min<int64_t>(((int64_t)nbmax * nbmax + 255) / 256,
-                                                                 std::max<int64_t>(1, (int64_t)c->num_sms * 8 / nm))));
-    DevBuf Qm(c, sizeof(double) * (size_t)nm * nbmax * std::max(kmax, 1));
-    if (kmax > 0) {
-      DevBuf Delta(c, sizeof(double) * (size_t)nm * kmax * kmax), St(c, sizeof(double) * (size_t)nm * kmax * kmax),
-          Qk(c, sizeof(double) * (size_t)nm * nbmax * kmax);
-      const int64_t warps = (int64_t)nm * kmax;
-      const int tb = 256, gb = int((warps * 32 + tb - 1) / tb);
-      {
-        ProfScope ps(c, NSG_PROF_DC, 0.0);
-        dc_secular_kernel<<<gb, tb, 0, c->stream>>>(md, nm, kmax, W, Delta.as<double>());
-        dc_gu_eisenstat_kernel<<<gb, tb, 0, c->stream>>>(md, nm, kmax, W, Delta.as<double>());
-        dc_vectors_kernel<<<gb, tb, 0, c->stream>>>(md, nm, kmax, W, Delta.as<double>(), St.as<double>());
-        const int gxk = int(std::max<int64_t>(
-            1, std::min<int64_t>(((int64_t)nbmax * kmax + 255) / 256, std::max<int64_t>(1, (int64_t)c->num_sms * 8 / nm))));
-        dc_gather_kernel<<<dim3(gxk, nm), 256, 0, c->stream>>>(Q, n, md, nbmax, kmax, W, Qk.as<double>());
-      }
-      count_launch(c, 4);
-      check_launch("dc secular");
-      GemmArgs g;
-      g.dtype = NSG_F64;
-      g.M = nbmax;
-      g.N = kmax;
-      g.K = kmax;
-      g.A = Qk.p;
-      g.lda = nbmax;
-      g.opA = OP_N;
-      g.strideA = (int64_t)nbmax * kmax;
-      g.B = St.p;
-      g.ldb = kmax;
-      g.opB = OP_N;
-      g.strideB = (int64_t)kmax * kmax;
-      g.C = Qm.p;
-      g.ldc = nbmax;
-      g.strideC = (int64_t)nbmax * kmax;
-      g.batch = nm;
-      gemm_accurate(c, g);
-    }
-    {
-      const int shm = nbmax <= kSmemMerge ? nbmax * 36 : 0;
-      if (shm) raise_smem_limit((const void*)dc_order_kernel, shm);
-      ProfScope ps(c, NSG_PROF_DC, 0.0);
-      dc_order_kernel<<<nm, 256, shm, c->stream>>>(md, W);
-      dc_scatter_kernel<<<dim3(gxe, nm), 256, 0, c->stream>>>(Q, n, md, nbmax, std::max(kmax, 1), W, Qm.as<double>(),
-                                                             Tbuf.as<double>(), w);
-      dc_copy_kernel<<<dim3(gxe, nm), 256, 0, c->stream>>>(Tbuf.as<double>(), n, md, Q);
-    }
-    count_launch(c, 3);
-    check_launch("dc merge");
-  }
-}
+// Back-transformation Z <- H_0 H_1 ... H_{n-3} Z in blocks of kWY reflectors, last block
+// first.  Every block's V, S = V^H V and T factor are formed up front (one launch each,
+// before the eigenvalues are known on the host); the sequential part is then three GEMMs
+// per block.
+template <typename T>
+struct BackTransform {
+  nsg_ctx* c;
+  const int dtype, n, nref, NB, nblk, ncols;
+  DevBuf V, S, Tm, taup;
+  BackTransform(nsg_ctx* cc, int dt, int order, const T* A, const T* tau_dev);
+  void apply(T* Z, int64_t ldz, int64_t k);
+};
 
 template <typename T>
-static void back_transform(nsg_ctx* c, int dtype, int n, const T* A, const T* tau_dev, T* Z, int64_t ldz, int64_t k) {
-  // Z <- H_0 H_1 ... H_{n-3} Z in blocks of kWY reflectors, last block first.  Every
-  // block's V, S = V^H V and T factor are formed up front (one launch each); the
-  // sequential part is then three GEMMs per block.
-  const int nref = n - 2;
-  if (nref <= 0 || k == 0) return;
-  const int NB = kWY, nblk = (nref + NB - 1) / NB, ncols = nblk * NB;
+BackTransform<T>::BackTransform(nsg_ctx* cc, int dt, int order, const T* A, const T* tau_dev)
+    : c(cc),
+      dtype(dt),
+      n(order),
+      nref(std::max(order - 2, 0)),
+      NB(kWY),
+      nblk((nref + kWY - 1) / kWY),
+      ncols(nblk * kWY),
+      V(cc, sizeof(T) * (size_t)order * ncols),
+      S(cc, sizeof(T) * (size_t)kWY * kWY * nblk),
+      Tm(cc, sizeof(T) * (size_t)kWY * kWY * nblk),
+      taup(cc, sizeof(T) * ncols) {
+  if (nref == 0) return;
   const size_t eb = sizeof(T);
-  DevBuf V(c, eb * (size_t)n * ncols), S(c, eb * (size_t)NB * NB * nblk), Tm(c, eb * (size_t)NB * NB * nblk),
-      taup(c, eb * ncols), Wt(c, eb * (size_t)NB * k), W2(c, eb * (size_t)NB * k);
   {
     int gblocks = int(std::min<size_t>(((size_t)n * ncols + 255) / 256, (size_t)c->num_sms * 8));
     wy_extract_all_kernel<T><<<gblocks, 256, 0, c->stream>>>(A, n, nref, ncols, V.as<T>());
@@ -1757,6 +850,13 @@ static void back_transform(nsg_ctx* c, int dtype, int n, const T* A, const T* ta
     wy_tfactor_kernel<T><<<nblk, NB, shm, c->stream>>>(S.as<T>(), taup.as<T>(), Tm.as<T>());
   }
   count_launch(c);
+  check_launch("back_transform factors");
+}
+
+template <typename T>
+void BackTransform<T>::apply(T* Z, int64_t ldz, int64_t k) {
+  if (nref == 0 || k == 0) return;
+  DevBuf Wt(c, sizeof(T) * (size_t)NB * k), W2(c, sizeof(T) * (size_t)NB * k);
   for (int b = nblk - 1; b >= 0; --b) {
     const int k0 = b * NB, nbk = std::min(NB, nref - k0), rows = n - (k0 + 1);
     const T* Vb = V.as<T>() + (k0 + 1) + (size_t)k0 * n;
@@ -1818,7 +918,7 @@ static void back_transform(nsg_ctx* c, int dtype, int n, const T* A, const T* ta
 // context's override; it is raised until the columns fit.  Returns false (nothing
 // launched) for the grid kernel or when no cluster shape fits.
 template <typename T>
-static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* tau) {
+static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* tau, double2* phase) {
   if (n < 3 || c->tune_tri == -1) return false;
   const size_t eb = sizeof(T);
   int C = c->tune_tri;
@@ -1855,7 +955,7 @@ static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* ta
       continue;
     }
     ProfScope ps(c, NSG_PROF_TRIDIAG, (sizeof(T) == 16 ? 16.0 : 4.0) / 3.0 * double(n) * n * n);
-    NSG_CUDA(cudaLaunchKernelEx(&cfg, kfn, A, n, d, e, tau));
+    NSG_CUDA(cudaLaunchKernelEx(&cfg, kfn, A, n, d, e, tau, phase));
     count_launch(c);
     check_launch("tridiag (cluster)");
     return true;
@@ -1870,19 +970,30 @@ static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* ta
 template <typename T>
 static void syevd_dc_impl(nsg_ctx* c, int dtype, int n, T* A, std::vector<double>& w_host, const PickFn& pick) {
   const size_t eb = sizeof(T);
-  DevBuf dd(c, sizeof(double) * n), de(c, sizeof(double) * std::max(n, 1)), dtau(c, eb * std::max(n, 1));
-  NSG_CUDA(cudaMemsetAsync(dtau.p, 0, eb * std::max(n, 1), c->stream));
-  std::vector<double> d(n), e(std::max(n - 1, 0));
+  // what the host reads back, in one copy: the eigenvalues, then the leaves' error flag and
+  // the grid barrier
+  struct Status {
+    int leaf_err, pad;
+    Barrier bar;
+  };
+  const size_t out_bytes = sizeof(double) * n + sizeof(Status);
+  DevBuf out(c, out_bytes), dd(c, sizeof(double) * n), de(c, sizeof(double) * n), dtau(c, eb * n), ph(c, sizeof(double2)),
+      Q0(c, sizeof(double) * (size_t)n * n), Q1(c, sizeof(double) * (size_t)n * n);
+  double* w = out.as<double>();
+  Status* st = (Status*)(w + n);
+  NSG_CUDA(cudaMemsetAsync(st, 0, sizeof(Status), c->stream));
+  NSG_CUDA(cudaMemsetAsync(dtau.p, 0, eb * n, c->stream));
+  NSG_CUDA(cudaMemsetAsync(ph.p, 0, sizeof(double2), c->stream));
+  double* pd = dd.as<double>();
+  double* pe = de.as<double>();
+  T* pt = dtau.as<T>();
+  double2* pph = ph.as<double2>();
   if (n == 1) {
-    T a;
-    NSG_CUDA(cudaMemcpyAsync(&a, A, eb, cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaStreamSynchronize(c->stream));
-    d[0] = ((double*)&a)[0];
-  } else if (tridiag_cluster<T>(c, n, A, dd.as<double>(), de.as<double>(), dtau.as<T>())) {
-    NSG_CUDA(cudaMemcpyAsync(d.data(), dd.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaMemcpyAsync(e.data(), de.p, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaStreamSynchronize(c->stream));
-  } else {
+    NSG_CUDA(cudaMemcpyAsync(pd, A, sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    const double2 one = make_double2(1.0, 0.0);
+    NSG_CUDA(cudaMemcpyAsync(pph, &one, sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+    NSG_CUDA(cudaStreamSynchronize(c->stream));  // `one` leaves scope
+  } else if (!tridiag_cluster<T>(c, n, A, pd, pe, pt, pph)) {
     // cooperative tridiagonalisation
     int max_blocks = 0;
     size_t shm = eb * 3 * n;
@@ -1904,77 +1015,40 @@ static void syevd_dc_impl(nsg_ctx* c, int dtype, int n, T* A, std::vector<double
       const int64_t units = ((m + grid - 1) / grid) * ((m + rb - 1) / rb);
       NSG_CHECK(units <= kTriUnits, NSG_ERR_UNSUPPORTED, "tridiagonalisation: matrix order too large for the grid");
     }
-    DevBuf xbuf(c, eb * 2 * n), part(c, sizeof(double2) * 2 * grid), bar(c, sizeof(Barrier));
-    NSG_CUDA(cudaMemsetAsync(bar.p, 0, sizeof(Barrier), c->stream));
-    double* pd = dd.as<double>();
-    double* pe = de.as<double>();
-    T* pt = dtau.as<T>();
+    DevBuf xbuf(c, eb * 2 * n), part(c, sizeof(double2) * 2 * grid);
     T* px = xbuf.as<T>();
     T* pp = part.as<T>();
-    Barrier* pb = bar.as<Barrier>();
+    Barrier* pb = &st->bar;
     int pt_arg = 1024 / kTriThreads;  // trailing elements per thread before another CTA joins the pass
-    void* args[] = {&A, &n, &pd, &pe, &pt, &px, &pp, &pb, &pt_arg};
+    void* args[] = {&A, &n, &pd, &pe, &pt, &px, &pp, &pb, &pt_arg, &pph};
     ProfScope ps(c, NSG_PROF_TRIDIAG, (sizeof(T) == 16 ? 16.0 : 4.0) / 3.0 * double(n) * n * n);
     NSG_CUDA(cudaLaunchCooperativeKernel((void*)kfn, dim3(grid), dim3(kTriThreads), args, shm,
                                          c->stream));
     count_launch(c);
     check_launch("tridiag");
-    Barrier hb;
-    NSG_CUDA(cudaMemcpyAsync(&hb, bar.p, sizeof(Barrier), cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaMemcpyAsync(d.data(), dd.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaMemcpyAsync(e.data(), de.p, sizeof(double) * (n - 1), cudaMemcpyDeviceToHost, c->stream));
-    NSG_CUDA(cudaStreamSynchronize(c->stream));
-    NSG_CHECK(hb.err == 0, NSG_ERR_TIMEOUT, "tridiagonalisation: grid barrier timed out");
   }
-  std::vector<double2> phase(n, make_double2(1.0, 0.0));
-  if constexpr (sizeof(T) == 16) {
-    // the last subdiagonal entry A[n-1, n-2] may be complex: make it real with a phase on row n-1
-    if (n >= 2) {
-      double2 last;
-      NSG_CUDA(cudaMemcpyAsync(&last, (double2*)A + (n - 1) + (size_t)(n - 2) * n, sizeof(double2),
-                               cudaMemcpyDeviceToHost, c->stream));
-      NSG_CUDA(cudaStreamSynchronize(c->stream));
-      double r = std::hypot(last.x, last.y);
-      e[n - 2] = r;
-      if (r > 0) phase[n - 1] = make_double2(last.x / r, last.y / r);
-    }
-  }
-  for (double x : d) NSG_CHECK(std::isfinite(x), NSG_ERR_NONFINITE, "eigensolver: non-finite tridiagonal");
-  for (double x : e) NSG_CHECK(std::isfinite(x), NSG_ERR_NONFINITE, "eigensolver: non-finite tridiagonal");
-  DevBuf Q(c, sizeof(double) * (size_t)n * n), wdev(c, sizeof(double) * n);
-  if (n == 1) {
-    double one = 1.0;
-    NSG_CUDA(cudaMemcpyAsync(Q.p, &one, sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    NSG_CUDA(cudaMemcpyAsync(wdev.p, d.data(), sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  } else {
-    tridiag_dc(c, n, d, e, Q.as<double>(), wdev.as<double>());
-  }
-  w_host.resize(n);
-  NSG_CUDA(cudaMemcpyAsync(w_host.data(), wdev.p, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-  NSG_CUDA(cudaStreamSynchronize(c->stream));
+  const double* Q = tridiag_dc(c, n, pd, pe, Q0.as<double>(), Q1.as<double>(), w, &st->leaf_err);
+  double* host = host_scalars(c, out_bytes / sizeof(double) + 1);
+  NSG_CUDA(cudaMemcpyAsync(host, out.p, out_bytes, cudaMemcpyDeviceToHost, c->stream));
+  NSG_CUDA(cudaEventRecord(read_event(c), c->stream));
+  BackTransform<T> back(c, dtype, n, A, pt);  // (its factors are formed while the host reads)
+  NSG_CUDA(cudaEventSynchronize(read_event(c)));
+  Status hs;
+  std::memcpy(&hs, host + n, sizeof(Status));
+  NSG_CHECK(hs.bar.err == 0, NSG_ERR_TIMEOUT, "tridiagonalisation: grid barrier timed out");
+  NSG_CHECK(hs.leaf_err == 0, NSG_ERR_NONFINITE, "eigensolver: a tridiagonal leaf did not converge");
+  w_host.assign(host, host + n);
   for (double x : w_host) NSG_CHECK(std::isfinite(x), NSG_ERR_NONFINITE, "eigensolver: non-finite eigenvalue");
   void* Zv = nullptr;
   int64_t ldz = 0;
-  std::vector<int> cols = pick(w_host, &Zv, &ldz);
+  const EigCols cols = pick(w_host, &Zv, &ldz);
   T* Zout = (T*)Zv;
-  int64_t kc = int64_t(cols.size());
-  if (kc == 0) return;
-  // gather the chosen tridiagonal eigenvectors into Zout (real -> T)
-  DevBuf didx(c, sizeof(int) * kc);
-  NSG_CUDA(cudaMemcpyAsync(didx.p, cols.data(), sizeof(int) * kc, cudaMemcpyHostToDevice, c->stream));
-  if constexpr (sizeof(T) == 8) {
-    copy_columns(c, NSG_F64, n, kc, Q.p, n, didx.as<int>(), Zout, ldz);
-  } else {
-    DevBuf Zr(c, sizeof(double) * (size_t)n * kc);
-    copy_columns(c, NSG_F64, n, kc, Q.p, n, didx.as<int>(), Zr.p, n);
-    int gblocks = int(std::min<size_t>(((size_t)n * kc + 255) / 256, (size_t)c->num_sms * 8));
-    real_to_complex_kernel<<<gblocks, 256, 0, c->stream>>>(Zr.as<double>(), n, kc, n, (double2*)Zout, ldz);
-    DevBuf ph(c, sizeof(double2) * n);
-    NSG_CUDA(cudaMemcpyAsync(ph.p, phase.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, c->stream));
-    scale_rows_phase_kernel<<<gblocks, 256, 0, c->stream>>>((double2*)Zout, n, kc, ldz, ph.as<double2>());
-    count_launch(c, 2);
-  }
-  back_transform<T>(c, dtype, n, A, dtau.as<T>(), Zout, ldz, kc);
+  if (cols.count == 0) return;
+  const int gblocks = int(std::min<int64_t>(((int64_t)n * cols.count + 255) / 256, (int64_t)c->num_sms * 8));
+  gather_vectors_kernel<<<gblocks, 256, 0, c->stream>>>(Q, n, cols.first, cols.step, cols.count, Zout, ldz, pph);
+  count_launch(c);
+  check_launch("eigenvector gather");
+  back.apply(Zout, ldz, cols.count);
 }
 
 void syevd_dc(nsg_ctx* c, int dtype, int n, void* A, std::vector<double>& w_host, const PickFn& pick) {
