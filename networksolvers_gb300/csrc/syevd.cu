@@ -80,6 +80,12 @@ __device__ __forceinline__ double2 fcma(double2 acc, double2 a, double2 b) {
   return make_double2(fma(a.y, b.y, fma(a.x, b.x, acc.x)), fma(-a.y, b.x, fma(a.x, b.y, acc.y)));
 }
 
+// acc + a b
+__device__ __forceinline__ double cfma(double acc, double a, double b) { return fma(a, b, acc); }
+__device__ __forceinline__ double2 cfma(double2 acc, double2 a, double2 b) {
+  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, acc.x)), fma(a.y, b.x, fma(a.x, b.y, acc.y)));
+}
+
 // Grid barrier state of the tridiagonalisation (cooperative launch guarantees
 // co-residency): a monotonic arrival counter (every CTA knows how many arrivals close
 // each step, so nothing is reset between steps) and an error flag set by a wait that
@@ -725,33 +731,55 @@ __global__ void gather_vectors_kernel(const double* __restrict__ Q, int64_t n, i
 }
 
 // compact WY: T factors of all reflector blocks in one launch (block b = CTA b; kWY = 64
-// reflectors per block, zero-padded with tau = 0) from S_b = V_b^H V_b:
-// T_jj = tau_j, T[0:j, j] = -tau_j T[0:j, 0:j] S[0:j, j]; thread i owns row i; S_b and T_b
-// live in shared memory.
-constexpr int kWY = 64;
+// reflectors per block, zero-padded with tau = 0) from S_b = V_b^H V_b, by doubling: with the
+// factors T1, T2 of two neighbouring halves, T = [T1, -T1 S12 T2; 0, T2].  Each level is two
+// triangular products over all pairs at once, so the 64^3 / 6 multiply-adds spread over the
+// CTA's FP64 pipes (column by column, one thread per row, they were a chain of 119 us for
+// real and 483 us for complex data; this takes 34 and 94).
+constexpr int kWY = 64, kWYThreads = 512;
 template <typename T>
-__global__ void __launch_bounds__(kWY) wy_tfactor_kernel(const T* S, const T* tau, T* Tm) {
-  extern __shared__ unsigned char wy_smem[];  // 2 x kWY x (kWY + 1) elements
-  T(*Ss)[kWY + 1] = (T(*)[kWY + 1])wy_smem;
-  T(*Ts)[kWY + 1] = Ss + kWY;
-  const int i = threadIdx.x, b = blockIdx.x;
+__global__ void __launch_bounds__(kWYThreads) wy_tfactor_kernel(const T* S, const T* tau, T* Tm) {
+  extern __shared__ __align__(16) unsigned char wy_smem[];  // 2 x kWY x (kWY + 1) elements
+  T(*Ss)[kWY + 1] = (T(*)[kWY + 1])wy_smem;  // [column][row]; the pairs' S12 T2 replaces S12
+  T(*Ts)[kWY + 1] = Ss + kWY;                // [column][row]
+  const int tid = threadIdx.x, b = blockIdx.x;
   const T* Sb = S + (size_t)b * kWY * kWY;
-  const T* tb = tau + (size_t)b * kWY;
   T* Tb = Tm + (size_t)b * kWY * kWY;
-  for (int j = 0; j < kWY; ++j) {
-    Ss[i][j] = Sb[i + j * kWY];
-    Ts[i][j] = czero<T>();
+  for (int t = tid; t < kWY * kWY; t += kWYThreads) {
+    const int i = t % kWY, j = t / kWY;
+    Ss[j][i] = Sb[t];
+    Ts[j][i] = i == j ? tau[(size_t)b * kWY + i] : czero<T>();
   }
   __syncthreads();
-  for (int j = 0; j < kWY; ++j) {
-    T acc = czero<T>();
-    if (i < j)
-      for (int l = i; l < j; ++l) acc = cadd(acc, cmulv(Ts[i][l], Ss[l][j]));
-    if (i < j) Ts[i][j] = cscale(cmulv(tb[j], acc), -1.0);  // column j: read only columns < j above
-    if (i == j) Ts[j][j] = tb[j];
+  for (int h = 1; h < kWY; h *= 2) {
+    // output (i, j) of pair q: row i of its upper half, column j of its lower half
+    constexpr int NI = kWY * kWY / 4 / kWYThreads;  // outputs per thread, at the last level
+    T acc[NI];
+#pragma unroll
+    for (int x = 0; x < NI; ++x) {
+      const int t = tid + x * kWYThreads, i = t % h, j = t / h % h, q = t / (h * h);
+      acc[x] = czero<T>();
+      if (q < kWY / (2 * h)) {
+        const int r0 = 2 * h * q, c0 = r0 + h;
+        for (int l = 0; l <= j; ++l) acc[x] = cfma(acc[x], Ss[c0 + l][r0 + i], Ts[c0 + j][c0 + l]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < NI; ++x) {
+      const int t = tid + x * kWYThreads, i = t % h, j = t / h % h, q = t / (h * h);
+      if (q < kWY / (2 * h)) Ss[2 * h * q + h + j][2 * h * q + i] = acc[x];
+    }
+    __syncthreads();
+    for (int t = tid; t < kWY / 2 * h; t += kWYThreads) {
+      const int i = t % h, j = t / h % h, r0 = 2 * h * (t / (h * h)), c0 = r0 + h;
+      T sum = czero<T>();
+      for (int l = i; l < h; ++l) sum = cfma(sum, Ts[r0 + l][r0 + i], Ss[c0 + j][r0 + l]);
+      Ts[c0 + j][r0 + i] = cscale(sum, -1.0);
+    }
     __syncthreads();
   }
-  for (int j = 0; j < kWY; ++j) Tb[i + j * kWY] = Ts[i][j];
+  for (int t = tid; t < kWY * kWY; t += kWYThreads) Tb[t] = Ts[t / kWY][t % kWY];
 }
 
 // all reflectors as the columns of an n x ncols matrix (v_kk[kk+1] = 1, zeros above,
@@ -847,7 +875,7 @@ BackTransform<T>::BackTransform(nsg_ctx* cc, int dt, int order, const T* A, cons
   {
     const int shm = int(2 * NB * (NB + 1) * eb);
     raise_smem_limit((const void*)wy_tfactor_kernel<T>, shm);
-    wy_tfactor_kernel<T><<<nblk, NB, shm, c->stream>>>(S.as<T>(), taup.as<T>(), Tm.as<T>());
+    wy_tfactor_kernel<T><<<nblk, kWYThreads, shm, c->stream>>>(S.as<T>(), taup.as<T>(), Tm.as<T>());
   }
   count_launch(c);
   check_launch("back_transform factors");
