@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace nsg {
 
@@ -293,46 +294,51 @@ __global__ void __launch_bounds__(kTileThreads)
 // Tall-skinny products with N, K <= 32: the site-operator steps of H_eff and of the
 // environment updates (K, N = w d, batched over the other bond).  op(B) is an MPO tensor
 // and mostly zeros: each CTA stages it in shared memory and lists the non-zeros of every
-// column (one warp per column, ballots), and thread r forms row r of C from exactly
-// nnz(B) multiply-adds on a [k][row] tile of op(A).  The rows of all batch entries that
-// share B (strideB = 0) form one row space, so short batch entries fill whole CTAs.  The
-// FP64 pipe (two multiply-adds per clock and SM) bounds the kernel beside the HBM traffic
-// of A and C, so a column's first term is an exponent addition where its coefficient is a
-// power of two (half of an MPO's entries) and alpha = 1, beta = 0 cost nothing.  A step of
-// 216 rows took 20 us when one warp read B's columns one after the other; it takes 5.
-template <typename T>
-__global__ void __launch_bounds__(256)
+// column (one warp per column, ballots), and a warp forms 32 rows of its columns of C from
+// exactly their non-zeros, on a [k][row] tile of op(A).  A column's multiply-adds are a
+// chain of 64 clocks each, so with few rows the columns are dealt to up to CW = 8 warps
+// and with many to one.  The rows of all batch entries that share B (strideB = 0) form one
+// row space, so short batch entries fill whole CTAs.  The FP64 pipe (two multiply-adds per
+// clock and SM) bounds the kernel beside the HBM traffic of A and C, so a column's first
+// term is an exponent addition where its coefficient is a power of two (half of an MPO's
+// entries) and alpha = 1, beta = 0 cost nothing.  216 rows, N = K = 18 complex: 20 us with
+// one warp listing B and a row per thread, 15 with the parallel list, 6 with the columns
+// dealt out.
+constexpr int kSkinnyThreads = 256;
+template <typename T, int CW>
+__global__ void __launch_bounds__(kSkinnyThreads)
     gemm_skinny_kernel(int64_t M, int64_t rows, int N, int K, const T* __restrict__ A, int64_t lda, int64_t sA,
                        bool conjA, const T* __restrict__ B, int64_t ldb, int64_t sB, int opB, T* __restrict__ C,
                        int64_t ldc, int64_t sC, int64_t groups, Scal<T> sc, bool plain) {
   extern __shared__ __align__(16) unsigned char sk_smem[];
-  const int nt = blockDim.x;
-  T* As = (T*)sk_smem;                       // [K][nt]
+  constexpr int R = kSkinnyThreads / CW;     // rows per CTA
+  T* As = (T*)sk_smem;                       // [K][R]
   __shared__ T Bs[32][33];                   // op(B)
   __shared__ T nzv[32][32];                  // non-zeros of each column of op(B)
   __shared__ unsigned char nzk[32][32];      // their row index k
   __shared__ int cnt[32], lead[32];          // their number; exponent of a real power-of-two first one
   constexpr int kNoLead = 1 << 20;
   const bool transB = (opB == OP_T || opB == OP_C), conjB = (opB == OP_C || opB == OP_R);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  const int64_t tiles = (rows + nt - 1) / nt;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = kSkinnyThreads / 32;
+  const int rl = tid % R, cw = tid / R;  // row in the tile, first column
+  const int64_t tiles = (rows + R - 1) / R;
   int64_t listed = -1;
   for (int64_t job = blockIdx.x; job < tiles * groups; job += gridDim.x) {
-    const int64_t g = job / tiles, r = (job % tiles) * nt + tid;
+    const int64_t g = job / tiles, r = (job % tiles) * R + rl;
     const int64_t bz = g + r / M, i = r % M;  // (groups > 1: rows = M, so r / M = 0)
     __syncthreads();  // the previous job's readers are done
     if (g != listed) {
       const T* Bb = B + g * sB;
-      for (int e = tid; e < N * K; e += nt) {
+      for (int e = tid; e < N * K; e += kSkinnyThreads) {
         const int j = transB ? e % N : e / K, k = transB ? e / N : e % K;
         Bs[j][k] = ld(transB ? Bb + j + (int64_t)k * ldb : Bb + k + (int64_t)j * ldb, conjB);
       }
     }
-    T* Ar = As + tid;
+    T* Ar = As + rl;
     if (r < rows) {
       const T* Ab = A + bz * sA + i;
 #pragma unroll 8
-      for (int k = 0; k < K; ++k) Ar[k * nt] = ld(Ab + (int64_t)k * lda, conjA);
+      for (int k = cw; k < K; k += CW) Ar[k * R] = ld(Ab + (int64_t)k * lda, conjA);
     }
     __syncthreads();
     if (g != listed) {
@@ -354,20 +360,20 @@ __global__ void __launch_bounds__(256)
     }
     if (r < rows) {
       T* Cb = C + bz * sC + i;
-      for (int j = 0; j < N; ++j) {
+      for (int j = cw; j < N; j += CW) {
         const int c = cnt[j];
         T acc;
         zero(acc);
         int t = 0;
         if (c > 0) {
-          const T a = Ar[nzk[j][0] * nt];
+          const T a = Ar[nzk[j][0] * R];
           if (lead[j] != kNoLead)
             acc = mul_pow2(a, lead[j], nzv[j][0]);
           else
             mac(acc, a, nzv[j][0]);
           t = 1;
         }
-        for (; t < c; ++t) mac(acc, Ar[nzk[j][t] * nt], nzv[j][t]);
+        for (; t < c; ++t) mac(acc, Ar[nzk[j][t] * R], nzv[j][t]);
         T* cp = Cb + (int64_t)j * ldc;
         *cp = plain ? acc : sc.epi(acc, cp);
       }
@@ -426,26 +432,37 @@ void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
   const bool cplx = g.dtype == NSG_C128;
   const double flops = double(g.M) * double(g.N) * double(g.K) * double(g.batch) * (cplx ? 8.0 : 2.0);
   if (g.N <= 32 && g.K <= 32 && g.K >= 1 && (g.opA == OP_N || g.opA == OP_R)) {
-    // batch entries that share B are one row space; rows per CTA: the smallest of 64, 128,
-    // 256 with which the rows still take every SM (the list of B's non-zeros is built per CTA)
+    // batch entries that share B are one row space; the columns on as many warps as it
+    // takes to give each SM sub-partition a warp or two (32 rows each)
     const bool shared_b = g.strideB == 0 || g.batch == 1;
     const int64_t groups = shared_b ? 1 : g.batch, rows = shared_b ? g.M * g.batch : g.M;
-    int nt = 64;
-    while (nt < 256 && (rows + nt - 1) / nt * groups > 2 * sms) nt *= 2;
-    const int grid = int(std::min<int64_t>((rows + nt - 1) / nt * groups, sms * 16));
+    int col_warps = 1;
+    while (col_warps < 8 && (rows + 31) / 32 * groups * col_warps < 8 * sms) col_warps *= 2;
     const bool plain = g.alpha_re == 1.0 && g.alpha_im == 0.0 && g.beta_re == 0.0 && g.beta_im == 0.0;
     ProfScope ps(c, NSG_PROF_SIMT_GEMM, flops);
-    auto launch = [&](auto zero_value, auto sc) {
-      using T = decltype(zero_value);
-      ensure_smem_limit((const void*)gemm_skinny_kernel<T>, 32 * 256 * int(sizeof(T)));
-      gemm_skinny_kernel<T><<<grid, nt, size_t(g.K) * nt * sizeof(T), c->stream>>>(
+    auto launch = [&](auto cw, auto sc) {
+      using T = std::remove_reference_t<decltype(sc.a)>;
+      constexpr int CW = decltype(cw)::value, R = kSkinnyThreads / CW;
+      const int grid = int(std::min<int64_t>((rows + R - 1) / R * groups, sms * 16));
+      ensure_smem_limit((const void*)gemm_skinny_kernel<T, CW>, 32 * R * int(sizeof(T)));
+      gemm_skinny_kernel<T, CW><<<grid, kSkinnyThreads, size_t(g.K) * R * sizeof(T), c->stream>>>(
           g.M, rows, int(g.N), int(g.K), (const T*)g.A, g.lda, g.strideA, g.opA == OP_R, (const T*)g.B, g.ldb,
           g.strideB, g.opB, (T*)g.C, g.ldc, g.strideC, groups, sc, plain);
     };
+    auto pick = [&](auto sc) {
+      if (col_warps == 1)
+        launch(std::integral_constant<int, 1>{}, sc);
+      else if (col_warps == 2)
+        launch(std::integral_constant<int, 2>{}, sc);
+      else if (col_warps == 4)
+        launch(std::integral_constant<int, 4>{}, sc);
+      else
+        launch(std::integral_constant<int, 8>{}, sc);
+    };
     if (cplx)
-      launch(double2{}, Scal<double2>{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)});
+      pick(Scal<double2>{make_double2(g.alpha_re, g.alpha_im), make_double2(g.beta_re, g.beta_im)});
     else
-      launch(double{}, Scal<double>{g.alpha_re, g.beta_re});
+      pick(Scal<double>{g.alpha_re, g.beta_re});
     count_launch(c);
     check_launch("gemm_skinny");
     return;
