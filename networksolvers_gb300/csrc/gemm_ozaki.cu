@@ -21,6 +21,7 @@
 // TMA copies (bounded), frees its TMEM and returns.
 #include "nsg_internal.h"
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -106,79 +107,223 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 }
 
 // ---------------------------------------------------------------------------
-// scales: scale[b][r] = 2^ceil(log2 max_k |src(r, k)|) (1 for an all-zero row)
+// scales and slices of the operands of a product:
+//   scale[b][r] = 2^ceil(log2 max_k |src(r, k)|) (1 for an all-zero row),
+//   out[(b*S + s)][r][k] (bf16, K-major, padded with zeros)
+// Work unit: 32 rows x at most 128 of K, read into shared memory with every load of the CTA
+// in flight at once (16 per thread), coalesced along whichever axis is contiguous, and
+// sliced from there with 16-byte stores by integer arithmetic on the numbers' bits (the
+// FP64 pipe is the slow one here).  Two forms:
+//  * depths below 1024: one launch for all operands of the product (up to four: the real and
+//    imaginary parts of both).  A cluster of up to 8 CTAs holds 32 rows over the whole depth,
+//    the row maxima meet through distributed shared memory, and each number is read once.
+//  * deeper: a pass for the row maxima and one for the slices per operand (the maxima of
+//    slabs of kMaxSlab, which the second pass combines).
+// Measured: both operands of an eight-slice product of order 950 in 8.7 us (scale and slice
+// passes per operand that read across rows: 29, in four launches), a 5120 x 1024 operand in
+// 17 + 38 us (38 + 58; one launch of clusters that kept slabs of 416 in shared memory: 105).
 // ---------------------------------------------------------------------------
-__global__ void row_scale_kernel(const double* __restrict__ src, int64_t rows, int64_t K, int64_t rs, int64_t ks,
-                                 int64_t bs, int64_t rows_p, double* __restrict__ scale, int64_t batch) {
-  // one warp per row; lanes stride over k
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = (gridDim.x * (int64_t)blockDim.x) >> 5;
-  for (int64_t t = w; t < rows_p * batch; t += nw) {
-    int64_t r = t % rows_p, b = t / rows_p;
-    double m = 0.0;
-    if (r < rows) {
-      const double* base = src + b * bs + r * rs;
-      for (int64_t k = lane; k < K; k += 32) m = fmax(m, fabs(base[k * ks]));
+struct OzSource {
+  const double* src;
+  int64_t rows, rs, ks, bs;  // element (r, k) of batch entry b at src[b bs + r rs + k ks]
+  int64_t rows_p, batch;
+  double* scale;
+  unsigned* part;            // row maxima of the slabs (deep form)
+  __nv_bfloat16* out;
+  int64_t tile_end;          // 32-row tiles of this and the earlier operands
+};
+struct OzSources {
+  OzSource op[4];
+  int n;
+  int64_t K, K_p;
+  int slab;  // K range of a CTA, a multiple of 32
+};
+constexpr int kSliceThreads = 256, kSliceWarps = kSliceThreads / 32, kSliceRows = 32, kSliceK = 128;
+constexpr int64_t kShallow = 1024, kMaxSlab = 512;
+
+// position of (row, k) in the shared-memory tile: odd row stride, octets of K swizzled
+__device__ __forceinline__ int slice_at(int r, int k) {
+  return r * (kSliceK + 1) + ((k & ~7) | ((k ^ (k >> 3)) & 7));
+}
+__device__ __forceinline__ unsigned magnitude(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+
+// 32 rows x len of K of one operand into `tile`; rowmax[r] takes the largest high word of
+// |row r| over them (zeroed before by the caller, and valid after a barrier).
+__device__ void load_slab(const OzSource& op, const double* base, int64_t r0, int64_t k0, int len, int64_t K, double* tile,
+                          unsigned* rowmax) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int NV = kSliceRows * kSliceK / kSliceThreads;
+  double v[NV];
+  if (op.ks < op.rs) {  // lanes along K: a warp takes rows warp, warp + 8, ..., four chunks of 32 each
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+      const int r = warp + kSliceWarps * (x / 4), k = lane + 32 * (x % 4);
+      v[x] = k < len && r0 + r < op.rows && k0 + k < K ? base[(r0 + r) * op.rs + (k0 + k) * op.ks] : 0.0;
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) {
-      int e = 0;
-      if (m > 0) {
-        frexp(m, &e);  // m = f 2^e, f in [0.5, 1)  ->  m <= 2^e
+#pragma unroll
+    for (int y = 0; y < NV / 4; ++y) {
+      const int r = warp + kSliceWarps * y;
+      unsigned m = 0;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        if (lane + 32 * x < len) tile[slice_at(r, lane + 32 * x)] = v[4 * y + x];
+        m = max(m, magnitude(v[4 * y + x]));
       }
-      // a normal power of two (the slicer inverts it by exponent arithmetic)
-      scale[t] = (m > 0) ? ldexp(1.0, max(e, -1000)) : 1.0;
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) rowmax[r] = m;
     }
+  } else {  // lanes along the rows
+    const bool in = r0 + lane < op.rows;
+    unsigned m = 0;
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+      const int k = warp + kSliceWarps * x;
+      v[x] = in && k < len && k0 + k < K ? base[(r0 + lane) * op.rs + (k0 + k) * op.ks] : 0.0;
+    }
+#pragma unroll
+    for (int x = 0; x < NV; ++x) {
+      const int k = warp + kSliceWarps * x;
+      if (k < len) tile[slice_at(lane, k)] = v[x];
+      m = max(m, magnitude(v[x]));
+    }
+    atomicMax(&rowmax[lane], m);
   }
 }
 
-// slices: out[(b*S + s)][r][k] (bf16, K-major, padded with zeros)
+// Biased exponent of a row's scale: |row| < 2^(e - 1022), e the largest biased exponent;
+// scales stay normal powers of two well inside the range (a row of subnormals takes
+// 2^-1000; a row that is not finite an infinite one, for which the epilogue writes NaN).
+__device__ __forceinline__ unsigned scale_exponent(unsigned m) {
+  const unsigned e = m >> 20;
+  return m == 0 ? 1023u : e == 0x7ffu ? 0x7ffu : max(e + 1, 23u);
+}
+
+// The tile's slices: X = round(v / scale 2^{7S}) from v's bits (the 53-bit significand
+// shifted by the exponents' difference, half to even), then balanced 7-bit digits
+// from the low end, |d| <= 64 (the top one up to 128): X = sum_s d_s 2^{7(S-1-s)} and
+// |v / scale - X 2^{-7S}| <= 2^{-7S-1}.  Lanes take octets of a row: 16-byte stores.
 template <int S>
-__global__ void slice_kernel(const double* __restrict__ src, int64_t rows, int64_t K, int64_t rs, int64_t ks,
-                             int64_t bs, int64_t rows_p, int64_t K_p, const double* __restrict__ scale,
-                             __nv_bfloat16* __restrict__ out, int64_t batch) {
-  __shared__ double tile[32][33];
-  const int64_t tr = rows_p / 32, tk = K_p / 32;
-  const int64_t ntiles = tr * tk * batch;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    int64_t kt = t % tk, rt = (t / tk) % tr, b = t / (tk * tr);
-    const double* base = src + b * bs;
-    if (ks == 1) {
-      for (int i = ty; i < 32; i += 8) {
-        int64_t r = rt * 32 + i, k = kt * 32 + tx;
-        tile[i][tx] = (r < rows && k < K) ? base[r * rs + k] : 0.0;
-      }
-    } else {
-      for (int j = ty; j < 32; j += 8) {
-        int64_t r = rt * 32 + tx, k = kt * 32 + j;
-        tile[tx][j] = (r < rows && k < K) ? base[r * rs + k * ks] : 0.0;
-      }
-    }
-    __syncthreads();
-    for (int i = ty; i < 32; i += 8) {
-      int64_t r = rt * 32 + i, k = kt * 32 + tx;
-      // x = value / sigma_r in [-1, 1] (sigma_r a power of two: the product is exact),
-      // then X = round(x 2^{7S}) in int64 and balanced 7-bit digits of X peeled off from
-      // the top with integer shifts (round half up): X = sum_s d_s 2^{7(S-1-s)}, |d_0| <=
-      // 128, |d_s| <= 64 after it, and |x - X 2^{-7S}| <= 2^{-7S-1}.  Only one FP64
-      // multiply and one conversion per element: the FP64 pipe is the slow one here.
-      // 1 / sigma_r by exponent arithmetic (sigma_r is a normal power of two)
-      const double inv = __longlong_as_double(0x7FE0000000000000ll - __double_as_longlong(scale[b * rows_p + r]));
-      constexpr double kFix = double(1ull << (7 * S));
-      long long X = __double2ll_rn(tile[i][tx] * inv * kFix);
+__device__ void slice_slab(const OzSource& op, int64_t b, int64_t r0, int64_t k0, int len, int64_t K_p, const double* tile,
+                           const unsigned* rowexp) {
+  const int noct = len / 8;
+  for (int t = threadIdx.x; t < kSliceRows * noct; t += kSliceThreads) {
+    const int r = t / noct, q = t % noct;
+    const int re = int(rowexp[r]);
+    uint32_t w[S][4];
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        const int sh = 7 * (S - 1 - s);
-        const long long dgt = sh ? ((X + (1ll << (sh - 1))) >> sh) : X;
-        X -= dgt << sh;
-        size_t o = ((size_t)(b * S + s) * rows_p + r) * K_p + k;
-        out[o] = __float2bfloat16_rn((float)(int)dgt);  // |dgt| <= 128: exact in bf16
+    for (int j = 0; j < 8; ++j) {
+      const long long bits = __double_as_longlong(tile[slice_at(r, q * 8 + j)]);
+      const int e = int((bits >> 52) & 0x7ff);
+      const long long m = (bits & 0xfffffffffffffll) | (e ? 0x10000000000000ll : 0);
+      const int sh = 52 - 7 * S - (max(e, 1) - re);  // m 2^(e - 1075) = X 2^(re - 1023 - 7S)
+      const int up = min(max(sh, 1), 55);
+      long long X = sh <= 0 ? m << min(-sh, 10) : (m + ((1ll << (up - 1)) - 1) + ((m >> up) & 1)) >> up;
+      if (bits < 0) X = -X;
+      // the low four digits and the rest in 32-bit arithmetic
+      int lo = int((X + (1ll << 27)) & ((1ll << 28) - 1)) - (1 << 27);
+      int hi = int((X - lo) >> 28);
+#pragma unroll
+      for (int s = S - 1; s >= 0; --s) {
+        int& part = s >= S - 4 ? lo : hi;
+        int d = part;
+        if (s > 0) {
+          d = ((part + 64) & 127) - 64;
+          part = (part - d) >> 7;
+          if (s == S - 4) hi += part;  // (the last carry out of the low digits)
+        }
+        // an integer of at most 128 as bf16: the upper half of its float
+        const uint32_t f = __float_as_uint(__int_as_float(0x4b400000 + d) - 12582912.f);
+        w[s][j / 2] = (j & 1) ? __byte_perm(w[s][j / 2], f, 0x7632) : f;
       }
     }
-    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+      *(uint4*)(op.out + ((size_t)(b * S + s) * op.rows_p + r0 + r) * K_p + k0 + q * 8) =
+          make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
   }
+}
+
+constexpr int kTileBytes = kSliceRows * (kSliceK + 1) * 8;
+
+template <int S>
+__global__ void __launch_bounds__(kSliceThreads) oz_slice_shallow_kernel(const __grid_constant__ OzSources P) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double tile[kTileBytes / 8];
+  __shared__ unsigned rowmax[kSliceRows], rowexp[kSliceRows];
+  const int C = int(cluster.num_blocks()), rank = int(cluster.block_rank()), tid = threadIdx.x;
+  int64_t t = blockIdx.x / C;
+  int o = 0;
+  while (t >= P.op[o].tile_end) ++o;
+  const OzSource& op = P.op[o];
+  if (o > 0) t -= P.op[o - 1].tile_end;
+  const int64_t rt = op.rows_p / kSliceRows, b = t / rt, r0 = (t % rt) * kSliceRows;
+  const int64_t k0 = (int64_t)rank * P.slab;
+  const int len = int(max(int64_t(0), min((int64_t)P.slab, P.K_p - k0)));
+  if (tid < kSliceRows) rowmax[tid] = 0;
+  __syncthreads();
+  load_slab(op, op.src + b * op.bs, r0, k0, len, P.K, tile, rowmax);
+  cluster.sync();  // every CTA's maxima are published
+  if (tid < kSliceRows) {
+    unsigned m = 0;
+    for (int c = 0; c < C; ++c) m = max(m, *cluster.map_shared_rank(&rowmax[tid], c));
+    rowexp[tid] = scale_exponent(m);
+    if (rank == 0) op.scale[b * op.rows_p + r0 + tid] = __hiloint2double(int(rowexp[tid] << 20), 0);
+  }
+  cluster.sync();  // the peers have read this CTA's maxima; rowexp is published
+  slice_slab<S>(op, b, r0, k0, len, P.K_p, tile, rowexp);
+}
+
+// blockIdx.x = 32-row tile (over the batch), blockIdx.y = slab of kMaxSlab
+__global__ void __launch_bounds__(kSliceThreads) oz_row_max_kernel(const __grid_constant__ OzSource op, int64_t K) {
+  __shared__ unsigned rowmax[kSliceRows];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t rt = op.rows_p / kSliceRows, b = blockIdx.x / rt, r0 = (blockIdx.x % rt) * kSliceRows;
+  const double* base = op.src + b * op.bs;
+  const int64_t k0 = blockIdx.y * kMaxSlab, k1 = min(K, k0 + kMaxSlab);
+  if (tid < kSliceRows) rowmax[tid] = 0;
+  __syncthreads();
+  if (op.ks < op.rs) {
+    for (int r = warp; r < kSliceRows; r += kSliceWarps) {
+      unsigned m = 0;
+      if (r0 + r < op.rows)
+#pragma unroll 16
+        for (int64_t k = k0 + lane; k < k1; k += 32) m = max(m, magnitude(base[(r0 + r) * op.rs + k * op.ks]));
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) rowmax[r] = m;
+    }
+  } else {
+    unsigned m = 0;
+    if (r0 + lane < op.rows)
+#pragma unroll 16
+      for (int64_t k = k0 + warp; k < k1; k += kSliceWarps) m = max(m, magnitude(base[(r0 + lane) * op.rs + k * op.ks]));
+    atomicMax(&rowmax[lane], m);
+  }
+  __syncthreads();
+  if (tid < kSliceRows) op.part[(int64_t)blockIdx.y * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid] = rowmax[tid];
+}
+
+// blockIdx.x = 32-row tile, blockIdx.y = slab of kSliceK
+template <int S>
+__global__ void __launch_bounds__(kSliceThreads)
+    oz_slice_deep_kernel(const __grid_constant__ OzSource op, int64_t K, int64_t K_p, int slabs) {
+  __shared__ double tile[kTileBytes / 8];
+  __shared__ unsigned rowmax[kSliceRows], rowexp[kSliceRows];
+  const int tid = threadIdx.x;
+  const int64_t rt = op.rows_p / kSliceRows, b = blockIdx.x / rt, r0 = (blockIdx.x % rt) * kSliceRows;
+  const int64_t k0 = (int64_t)blockIdx.y * kSliceK;
+  const int len = int(min((int64_t)kSliceK, K_p - k0));
+  if (tid < kSliceRows) {
+    unsigned m = 0;
+    for (int q = 0; q < slabs; ++q) m = max(m, op.part[(int64_t)q * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid]);
+    rowexp[tid] = scale_exponent(m);
+    rowmax[tid] = 0;
+    if (k0 == 0) op.scale[blockIdx.x * kSliceRows + tid] = __hiloint2double(int(rowexp[tid] << 20), 0);
+  }
+  __syncthreads();
+  load_slab(op, op.src + b * op.bs, r0, k0, len, K, tile, rowmax);
+  __syncthreads();
+  slice_slab<S>(op, b, r0, k0, len, K_p, tile, rowexp);
 }
 
 struct OzEpi {
@@ -410,6 +555,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           if (col < ep.N) {
             const int kb = pow2_exponent(ep.sb[(ep.b_batched ? bz : 0) * ep.Np + col]);
             double v = scale_pow2(widen(hi[j]) + widen(lo[j]), ka + kb);
+            if (ka > 1023 || kb > 1023) v = __longlong_as_double(0x7ff8000000000000ll);  // a row that is not finite
             if (Wz) {
               Wz[row + col * ep.M] = v;
             } else {
@@ -475,23 +621,6 @@ CUtensorMap make_map(void* base, int64_t rows_p, int64_t K_p, int64_t planes, in
   return m;
 }
 
-template <int S>
-void slice_operand(nsg_ctx* c, const double* src, int64_t rows, int64_t K, int64_t rs, int64_t ks, int64_t bs,
-                   int64_t batch, int64_t rows_p, int64_t K_p, double* scale, __nv_bfloat16* out) {
-  {
-    int64_t warps = rows_p * batch;
-    int grid = int(std::min<int64_t>((warps * 32 + 255) / 256, (int64_t)c->num_sms * 16));
-    ProfScope ps(c, NSG_PROF_SPLIT, 0.0);
-    row_scale_kernel<<<grid, 256, 0, c->stream>>>(src, rows, K, rs, ks, bs, rows_p, scale, batch);
-  }
-  int64_t ntiles = (rows_p / 32) * (K_p / 32) * batch;
-  int grid = int(std::min<int64_t>(ntiles, (int64_t)c->num_sms * 16));
-  ProfScope ps(c, NSG_PROF_SPLIT, 0.0);
-  slice_kernel<S><<<grid, 256, 0, c->stream>>>(src, rows, K, rs, ks, bs, rows_p, K_p, scale, out, batch);
-  count_launch(c, 2);
-  check_launch("ozaki slices");
-}
-
 // One operand of an Ozaki product, sliced: S bf16 slices [batch][S][rows_p][K_p] and the
 // power-of-two row scales [batch][rows_p].
 struct OzOperand {
@@ -500,23 +629,74 @@ struct OzOperand {
   int64_t rows_p = 0, batch = 1;
 };
 
+// bytes of the slices, the scales and the slabs' row maxima (256-byte aligned each)
+inline size_t oz_align(size_t b) { return (b + 255) & ~size_t(255); }
 template <int S>
 size_t oz_operand_bytes(int64_t rows_p, int64_t K_p, int64_t batch) {
-  return ((2 * size_t(S) * rows_p * K_p * batch + 255) & ~size_t(255)) + ((8 * size_t(rows_p) * batch + 255) & ~size_t(255));
+  const size_t rows = size_t(rows_p) * batch;
+  return oz_align(2 * size_t(S) * rows * K_p) + oz_align(8 * rows) +
+         (K_p >= kShallow ? oz_align(4 * rows * ((K_p + kMaxSlab - 1) / kMaxSlab)) : 0);
 }
 
-// slices of op(X) viewed as rows x K (element (r, k) at src[b bs + r rs + k ks], in doubles)
+// The operands of a product laid out in `mem`, one after the other, and sliced: op(X) viewed
+// as rows x K (element (r, k) at src[b bs + r rs + k ks], in doubles).
 template <int S>
-OzOperand oz_prepare(nsg_ctx* c, unsigned char* mem, const double* src, int64_t rows, int64_t K, int64_t rs,
-                     int64_t ks, int64_t bs, int64_t batch, int64_t rows_p, int64_t K_p) {
-  OzOperand o;
-  o.slices = (__nv_bfloat16*)mem;
-  o.scales = (double*)(mem + ((2 * size_t(S) * rows_p * K_p * batch + 255) & ~size_t(255)));
-  o.rows_p = rows_p;
-  o.batch = batch;
-  slice_operand<S>(c, src, rows, K, rs, ks, bs, batch, rows_p, K_p, o.scales, o.slices);
-  return o;
-}
+struct OzSlicer {
+  nsg_ctx* c;
+  OzSources P{};
+  unsigned char* mem;
+  OzSlicer(nsg_ctx* cc, unsigned char* m, int64_t K, int64_t K_p) : c(cc), mem(m) {
+    P.K = K;
+    P.K_p = K_p;
+  }
+  OzOperand add(const double* src, int64_t rows, int64_t rs, int64_t ks, int64_t bs, int64_t batch, int64_t rows_p) {
+    const size_t all = size_t(rows_p) * batch;
+    OzOperand o;
+    o.slices = (__nv_bfloat16*)mem;
+    o.scales = (double*)(mem + oz_align(2 * size_t(S) * all * P.K_p));
+    o.rows_p = rows_p;
+    o.batch = batch;
+    const int64_t before = P.n > 0 ? P.op[P.n - 1].tile_end : 0;
+    P.op[P.n++] = OzSource{src, rows, rs, ks, bs, rows_p, batch, o.scales, (unsigned*)((char*)o.scales + oz_align(8 * all)),
+                           o.slices, before + rows_p / kSliceRows * batch};
+    mem += oz_operand_bytes<S>(rows_p, P.K_p, batch);
+    return o;
+  }
+  void run() {
+    ProfScope ps(c, NSG_PROF_SPLIT, 0.0);
+    const int64_t tiles = P.op[P.n - 1].tile_end;
+    if (P.K_p < kShallow && tiles * 8 < (1ll << 31)) {
+      int C = 1;
+      while (P.K_p > int64_t(kSliceK) * C) C *= 2;
+      P.slab = int((P.K_p / 32 + C - 1) / C * 32);
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(unsigned(tiles * C));
+      cfg.blockDim = dim3(kSliceThreads);
+      cfg.stream = c->stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = C;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      NSG_CUDA(cudaLaunchKernelEx(&cfg, oz_slice_shallow_kernel<S>, P));
+      count_launch(c);
+    } else {
+      const int slabs = int((P.K_p + kMaxSlab - 1) / kMaxSlab);
+      NSG_CHECK(slabs <= 65535 && P.K_p <= 65535 * int64_t(kSliceK) && tiles < (1ll << 31), NSG_ERR_UNSUPPORTED,
+                "ozaki slices: grid too large");
+      for (int o = 0; o < P.n; ++o) {
+        const unsigned mine = unsigned(P.op[o].rows_p / kSliceRows * P.op[o].batch);
+        oz_row_max_kernel<<<dim3(mine, slabs), kSliceThreads, 0, c->stream>>>(P.op[o], P.K);
+        oz_slice_deep_kernel<S><<<dim3(mine, unsigned((P.K_p + kSliceK - 1) / kSliceK)), kSliceThreads, 0, c->stream>>>(
+            P.op[o], P.K, P.K_p, slabs);
+      }
+      count_launch(c, 2 * P.n);
+    }
+    check_launch("ozaki slices");
+  }
+};
 
 // C (+)= alpha A B^T-form product of two prepared operands into C (stride ldc between
 // columns, sC between batch entries, crs between rows; all in doubles)
@@ -589,8 +769,10 @@ bool gemm_ozaki_impl(nsg_ctx* c, const GemmArgs& g) {
   if (!cplx) {
     ScopedBuf sbuf(c, opA_bytes + opB_bytes);
     unsigned char* buf = (unsigned char*)sbuf.p;
-    OzOperand A = oz_prepare<S>(c, buf, (const double*)g.A, g.M, g.K, ars, aks, g.strideA, ab, Mp, Kp);
-    OzOperand B = oz_prepare<S>(c, buf + opA_bytes, (const double*)g.B, g.N, g.K, brs, bks, g.strideB, bb, Np, Kp);
+    OzSlicer<S> sl(c, buf, g.K, Kp);
+    OzOperand A = sl.add((const double*)g.A, g.M, ars, aks, g.strideA, ab, Mp);
+    OzOperand B = sl.add((const double*)g.B, g.N, brs, bks, g.strideB, bb, Np);
+    sl.run();
     oz_product<S>(c, A, B, g.M, g.N, Kp, g.batch, (double*)g.C, g.ldc, g.strideC, 1, g.alpha_re, g.beta_re, g.K);
     return true;
   }
@@ -603,11 +785,12 @@ bool gemm_ozaki_impl(nsg_ctx* c, const GemmArgs& g) {
   unsigned char* buf = (unsigned char*)sbuf.p;
   const double* Ad = (const double*)g.A;
   const double* Bd = (const double*)g.B;
-  OzOperand Ar = oz_prepare<S>(c, buf, Ad, g.M, g.K, 2 * ars, 2 * aks, 2 * g.strideA, ab, Mp, Kp);
-  OzOperand Ai = oz_prepare<S>(c, buf + opA_bytes, Ad + 1, g.M, g.K, 2 * ars, 2 * aks, 2 * g.strideA, ab, Mp, Kp);
-  OzOperand Br = oz_prepare<S>(c, buf + 2 * opA_bytes, Bd, g.N, g.K, 2 * brs, 2 * bks, 2 * g.strideB, bb, Np, Kp);
-  OzOperand Bi = oz_prepare<S>(c, buf + 2 * opA_bytes + opB_bytes, Bd + 1, g.N, g.K, 2 * brs, 2 * bks,
-                               2 * g.strideB, bb, Np, Kp);
+  OzSlicer<S> sl(c, buf, g.K, Kp);
+  OzOperand Ar = sl.add(Ad, g.M, 2 * ars, 2 * aks, 2 * g.strideA, ab, Mp);
+  OzOperand Ai = sl.add(Ad + 1, g.M, 2 * ars, 2 * aks, 2 * g.strideA, ab, Mp);
+  OzOperand Br = sl.add(Bd, g.N, 2 * brs, 2 * bks, 2 * g.strideB, bb, Np);
+  OzOperand Bi = sl.add(Bd + 1, g.N, 2 * brs, 2 * bks, 2 * g.strideB, bb, Np);
+  sl.run();
   double* Cr = (double*)g.C;
   double* Ci = Cr + 1;
   const int64_t ldc = 2 * g.ldc, sC = 2 * g.strideC;
