@@ -7,11 +7,14 @@
 //   A_ik / sigma_i = sum_{s<S} 2^{-7(s+1)} A^(s)_ik + r,  A^(s) integers, |A^(s)| <= 128,
 // (round-to-nearest digits, |r| <= 2^{-7S-1}); columns of B likewise with tau_j.  Then
 //   (AB)_ij = sigma_i tau_j sum_g 2^{-7(g+2)} sum_{s+t=g} (A^(s) B^(t))_ij,   g <= S-1.
-// The integer slices are exact in BF16, and with g+1 <= 6 products per group and K
-// chunks of 128 every partial sum is an integer below 2^24, so the tcgen05 FP32
-// accumulation of a group over a chunk is exact.  Drain warps add the six group sums
-// of each chunk into double-float (hi, lo) FP32 accumulators; the epilogue widens to
-// FP64 and applies sigma_i tau_j, alpha and beta.  With S = 6 slices the result is
+// The integer slices are exact in BF16 (|A^(0)| <= 128, the others <= 64), and with g+1 <= 8
+// products per group and K chunks of 384 every partial sum is an integer below
+// 384 (2 x 128 x 64 + 6 x 64^2) < 2^24, so the tcgen05 FP32 accumulation of a group over a
+// chunk is exact.  Drain warps add the group sums of each chunk into double-float (hi, lo)
+// FP32 accumulators; the epilogue widens to FP64 and applies sigma_i tau_j, alpha and beta.
+// At the end of a chunk the tensor pipe waits for the accumulators' drain, so chunks are as
+// long as exactness allows: an H_eff product at bond dimension 1024 takes 0.94 ms with
+// chunks of 384, 0.97 with 256 and 1.07 with 128.  With S = 6 slices the result is
 // within ~2^-43 K sigma_i tau_j of A B (dropped slices and products).
 //
 // Kernel layout: 128 x 64 output tile per CTA, 16 drain warps (4 warpgroups, each
@@ -35,7 +38,8 @@ namespace {
 constexpr int BM = 128, BN = 64, BKS = 32;  // K slab: 32 bf16 = 64 bytes
 constexpr int SLICE_A = BM * BKS * 2;       // 8 KB
 constexpr int SLICE_B = BN * BKS * 2;       // 4 KB
-constexpr int CHUNK_SLABS = 4;              // K = 128 per exact chunk
+constexpr int SPLIT_SLABS = 4;              // K is split over CTAs in units of 128
+constexpr int CHUNK_SLABS = 12;             // K = 384 per exact chunk
 constexpr int NDRAIN_WARPS = 16;
 constexpr int NTHREADS = (NDRAIN_WARPS + 1) * 32;
 
@@ -500,24 +504,27 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // three groups' TMEM loads in flight per wait (one wait per group made the drain,
-      // and with it the tensor pipe, wait on the load latency six times per chunk); the
-      // groups are still added in ascending order
+      // and with it the tensor pipe, wait on the load latency six times per chunk).  The
+      // groups are added smallest first: the sums' low parts stay small, so their rounding
+      // does too (K = 777, entries near one, eight slices: largest error 5.6e-12, against
+      // 1.15e-11 largest first).  The last two groups go to the low part with one addition:
+      // its rounding, 2^-24 of a term of 2^-7S, is below what the dropped groups are.
 #pragma unroll
-      for (int g0 = 0; g0 < G; g0 += 3) {
+      for (int g0 = G - 1; g0 >= 0; g0 -= 3) {
         uint32_t r[3][16];
 #pragma unroll
         for (int gg = 0; gg < 3; ++gg) {
-          if (g0 + gg < G)
+          if (g0 - gg >= 0)
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
                 "%13, %14, %15}, [%16];"
                 : "=r"(r[gg][0]), "=r"(r[gg][1]), "=r"(r[gg][2]), "=r"(r[gg][3]), "=r"(r[gg][4]), "=r"(r[gg][5]),
                   "=r"(r[gg][6]), "=r"(r[gg][7]), "=r"(r[gg][8]), "=r"(r[gg][9]), "=r"(r[gg][10]), "=r"(r[gg][11]),
                   "=r"(r[gg][12]), "=r"(r[gg][13]), "=r"(r[gg][14]), "=r"(r[gg][15])
-                : "r"(tmem + lane_base + (uint32_t)((g0 + gg) * BN + 16 * q)));
+                : "r"(tmem + lane_base + (uint32_t)((g0 - gg) * BN + 16 * q)));
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (g0 + 3 >= G) {
+        if (g0 < 3) {
           // the last loads are in registers: release the accumulators before the
           // arithmetic, so the next chunk's products overlap it
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -525,10 +532,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
 #pragma unroll
         for (int gg = 0; gg < 3; ++gg) {
-          if (g0 + gg < G) {
-            const float sc = __int_as_float((127 - 7 * (g0 + gg + 2)) << 23);  // 2^{-7(g+2)}, exact
+          if (g0 - gg >= 0) {
+            const float sc = __int_as_float((127 - 7 * (g0 - gg + 2)) << 23);  // 2^{-7(g+2)}, exact
 #pragma unroll
-            for (int j = 0; j < 16; ++j) two_sum_acc(hi[j], lo[j], __uint_as_float(r[gg][j]) * sc);
+            for (int j = 0; j < 16; ++j) {
+              if (g0 - gg >= G - 2)
+                lo[j] = fmaf(__uint_as_float(r[gg][j]), sc, lo[j]);
+              else
+                two_sum_acc(hi[j], lo[j], __uint_as_float(r[gg][j]) * sc);
+            }
           }
         }
       }
@@ -710,13 +722,13 @@ void oz_product(nsg_ctx* c, const OzOperand& A, const OzOperand& B, int64_t M, i
   ensure_smem_limit((const void*)oz_gemm_kernel<S>, SMEM_BYTES);
   // split K over whole exact chunks when the output tiles would leave most SMs idle
   // (the small products of a converged sweep: 32-64 tiles of 128 x 64 on 152 SMs)
-  const int nk = int(K_p / BKS), nchunk = (nk + CHUNK_SLABS - 1) / CHUNK_SLABS;
+  const int nk = int(K_p / BKS), units = (nk + SPLIT_SLABS - 1) / SPLIT_SLABS;
   const int64_t tiles = (A.rows_p / BM) * (B.rows_p / BN) * batch;
   const int64_t sms = c->num_sms > 0 ? c->num_sms : 152;
   int nsplit = 1;
-  if (tiles * 2 <= sms && nchunk >= 2)
-    nsplit = int(std::min<int64_t>({(int64_t)nchunk, sms / tiles, 16, 65535 / batch}));
-  const int split_slabs = (nchunk + nsplit - 1) / nsplit * CHUNK_SLABS;
+  if (tiles * 2 <= sms && units >= 2)
+    nsplit = int(std::min<int64_t>({(int64_t)units, sms / tiles, 16, 65535 / batch}));
+  const int split_slabs = (units + nsplit - 1) / nsplit * SPLIT_SLABS;
   nsplit = (nk + split_slabs - 1) / split_slabs;
   // the partial products' workspace, only when K is split (freed on every exit)
   struct Partials {

@@ -41,6 +41,23 @@ def test_slices_every_orientation(nsg_ctx, precision, bits, cplx, m, n, k):
         nsg_ctx.set_precision("fp64")
 
 
+@pytest.mark.parametrize("precision,bits", [("ozaki", 42), ("ozaki8", 48)])
+@pytest.mark.parametrize("k", [384, 385, 416, 777])
+def test_chunks_of_one_pass_over_k(nsg_ctx, precision, bits, k):
+    """Depths around the exact chunk's length where K is not split over CTAs (100 output
+    tiles), with every entry's digits near their largest value and of one sign."""
+    rng = np.random.default_rng(k)
+    m, n = 1270, 630
+    a, b = 1.0 - 2.0 ** -40 * rng.random((m, k)), 1.0 - 2.0 ** -9 * (1 + rng.random((k, n)))
+    i, j, l = Index(m), Index(n), Index(k)
+    nsg_ctx.set_precision(precision)
+    try:
+        got = contract([DTensor.from_numpy(a, [i, l]), DTensor.from_numpy(b, [l, j])], out=[i, j]).to_numpy()
+    finally:
+        nsg_ctx.set_precision("fp64")
+    assert np.max(np.abs(got - a @ b)) <= 4 * k * 2.0 ** -bits
+
+
 @pytest.mark.parametrize("precision", ["ozaki", "ozaki8"])
 def test_slices_batched(nsg_ctx, precision):
     rng = np.random.default_rng(4)
