@@ -48,13 +48,14 @@ constexpr double kEps = 2.220446049250313e-16;
 //   dcol       block-local column of deflated pole j
 //   rot_pq, rot_cs   deflation rotations (2 entries each, at 2 lo)
 //   gscr       scratch of blocks above kSmemMerge rows
+//   low        exponent below which an entry of T counts as zero
 // Delta and St hold nb^2 entries per merge at offset mi nbmax^2.
 enum { C_K = 0, C_ROT, C_FLIP, C_L1, C_L2, C_STRIDE = 8 };
 struct DcWork {
   int n, leaf;
   const double *d, *e;
   double *w, *Ds, *zs, *Dk, *zk, *wk, *lam, *zh, *rot_cs, *gscr, *rho, *Delta, *St;
-  int *perm, *kind, *qcol, *l1, *l2, *outp, *dcol, *rot_pq, *counts, *err;
+  int *perm, *kind, *qcol, *l1, *l2, *outp, *dcol, *rot_pq, *counts, *low, *err;
 };
 
 struct Span {
@@ -177,6 +178,12 @@ __device__ __forceinline__ int rank_in(F key, int len, long long k) {
   return lo;
 }
 
+// x, or 0 when its biased exponent is below `low`: a matrix of low rank leaves blocks of T that
+// fall by eps from row to row, and the merges square their entries' differences.
+__device__ __forceinline__ double above(double x, int low) {
+  return ((__double2hiint(x) >> 20) & 0x7ff) < low ? 0.0 : x;
+}
+
 // One leaf (rows [lo, hi), at most 32) by one CTA: two-sided cyclic Jacobi with the
 // round-robin ordering, half the rows' pairs rotated at once; a step is one pass over the
 // rows of independent 2 x 2 blocks plus the eigenvector columns.  The rotation's tangent is
@@ -189,23 +196,33 @@ __device__ __forceinline__ int rank_in(F key, int len, long long k) {
 // after 30 sweeps raises *err.
 __device__ void solve_leaf(const DcWork& W, int lo, int hi, double* Q0, double* Q1) {
   __shared__ double A[kLeafMax][kLeafMax + 1], V[kLeafMax][kLeafMax + 1], cs[kLeafMax / 2], sn[kLeafMax / 2];
-  __shared__ int pos[kLeafMax], moved, expo;
+  __shared__ int pos[kLeafMax], moved, expo, top;
   __shared__ unsigned char pairs[kLeafMax - 1][kLeafMax / 2][2];  // of round r: (lower, upper) index
   const int s = hi - lo, tid = threadIdx.x, nt = blockDim.x;
   if (tid == 0) {
     moved = 0;
     expo = 0;
+    top = 0;
   }
   __syncthreads();
+  // entries below 2^-200 of T's largest count as zero (the same bound in every CTA)
+  int mx = 0;
+  for (int i = tid; i < W.n; i += nt)
+    mx = max(mx, max((__double2hiint(W.d[i]) >> 20) & 0x7ff, i + 1 < W.n ? (__double2hiint(W.e[i]) >> 20) & 0x7ff : 0));
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((tid & 31) == 0) atomicMax(&top, mx);
+  __syncthreads();
+  const int low = max(top - 200, 0);
+  if (tid == 0) *W.low = low;
   for (int t = tid; t < s * s; t += nt) {
     const int i = t % s, j = t / s;
     double a = 0.0;
     if (i == j) {  // the rank-one updates of the splits at both ends are taken off
-      a = W.d[lo + i];
-      if (i == 0 && lo > 0) a -= W.e[lo - 1];
-      if (i == s - 1 && hi < W.n) a -= W.e[hi - 1];
+      a = above(W.d[lo + i], low);
+      if (i == 0 && lo > 0) a -= above(W.e[lo - 1], low);
+      if (i == s - 1 && hi < W.n) a -= above(W.e[hi - 1], low);
     } else if (i == j + 1 || j == i + 1) {
-      a = W.e[lo + min(i, j)];
+      a = above(W.e[lo + min(i, j)], low);
     }
     A[i][j] = a;
     V[i][j] = i == j ? 1.0 : 0.0;
@@ -353,7 +370,7 @@ __device__ void prep_merge(const DcWork& W, const double* Q, int lo, int hi, int
     s_nrot = 0;
   }
   __syncthreads();
-  double rho = W.e[mid - 1];
+  double rho = above(W.e[mid - 1], *W.low);
   const int flip = rho < 0;
   if (flip) rho = -rho;
   // merge of the two ascending halves (both traversed from their top when flipped, values
@@ -1110,7 +1127,7 @@ double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* 
     sq = std::max(sq, nm * nb * nb);
   }
   const size_t N = (size_t(n) + 1) & ~size_t(1), MC = size_t(C_STRIDE) * maxm;
-  const size_t doubles = 13 * N + 2 * sq + maxm + 2, ints = 9 * N + MC;
+  const size_t doubles = 13 * N + 2 * sq + maxm + 2, ints = 9 * N + MC + 2;
   ScopedBuf buf(c, sizeof(double) * doubles + sizeof(int) * ints);
   double* p = (double*)buf.p;
   auto take = [&](size_t m) {
@@ -1143,6 +1160,7 @@ double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* 
   W.l2 = takei(N);
   W.outp = takei(N);
   W.dcol = takei(N);
+  W.low = takei(2);
   W.rot_pq = takei(2 * N);
   W.counts = takei(MC);
   auto prep_smem = [](int nb) { return nb <= kSmemMerge ? nb * kPrepBytes : 0; };

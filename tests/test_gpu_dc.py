@@ -81,6 +81,15 @@ def test_diagonal_and_zero(nsg_ctx, n):
     check(nsg_ctx, np.zeros((n, n)))
 
 
+@pytest.mark.parametrize("n", [50, 140, 300, 500])
+def test_rank_one_falls_by_eps_per_row(nsg_ctx, n):
+    """The reduction of a matrix of ones leaves tridiagonal blocks down to the end of the
+    exponent range."""
+    check(nsg_ctx, np.ones((n, n)))
+    v = np.cos(np.arange(n))
+    check(nsg_ctx, np.outer(v, v) * 1e-60)
+
+
 @pytest.mark.parametrize("precision", ["ozaki", "ozaki8"])
 @pytest.mark.parametrize("n", [257, 400, 530, 700])
 def test_tensor_core_merges(nsg_ctx, n, precision):
