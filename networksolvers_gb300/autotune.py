@@ -6,8 +6,9 @@ Measures on the current GPU, with per-context overrides (nsg_ctx_set_tuning) and
 events around the kernels of the class (nsg_ctx_profile):
 
 * the Householder tridiagonalisation of the truncated factorization, for matrix orders
-  32..576: the grid-wide cooperative kernel against one thread-block cluster of 2, 4, 8
-  and 16 CTAs (where the matrix fits the cluster's shared memory);
+  8..576: the kernel over all SMs against one thread-block cluster of 2, 4, 8 and 16 CTAs
+  (where the matrix fits the cluster's shared memory; a cluster within 15 % of the kernel
+  over all SMs is preferred, since it leaves the other SMs to other streams);
 * the FP64 CUDA-core GEMM of small outputs (the eigensolver's products at small bond
   dimension), for output sizes 32..256 and depths 64..4096: split K into 1..64 slices.
 
@@ -26,7 +27,7 @@ from pathlib import Path
 
 import numpy as np
 
-TRI_ORDERS = [32, 48, 64, 96, 128, 192, 256, 320, 384, 448, 512, 576]
+TRI_ORDERS = [8, 16, 32, 48, 64, 96, 128, 192, 256, 320, 384, 448, 512, 576]
 TRI_PATHS = [-1, 2, 4, 8, 16]
 GEMM_SIZES = [32, 64, 128, 256]
 GEMM_DEPTHS = [64, 128, 256, 512, 1024, 2048, 4096]
@@ -50,6 +51,11 @@ def _median_class_ms(ctx, cls, run, reps):
     return float(np.median(out))
 
 
+def best_path(times):
+    cluster = min((p for p in times if p > 0), key=times.get, default=-1)
+    return cluster if cluster > 0 and times[cluster] <= 1.15 * times[-1] else -1
+
+
 def tune_tridiag(ctx, reps):
     from .itensors import DTensor, Index, factorize
     rng = np.random.default_rng(3)
@@ -66,7 +72,7 @@ def tune_tridiag(ctx, reps):
             times[path] = _median_class_ms(ctx, "tridiag", lambda: factorize(T, [l], cutoff=1e-12, maxdim=n // 2),
                                            reps)
         ctx.set_tuning("tridiag", 0)
-        best = min(times, key=times.get)
+        best = best_path(times)
         rows.append({"order": n, "ms": {str(k): v for k, v in times.items()}, "best": best})
         print(json.dumps(rows[-1]), file=sys.stderr, flush=True)
     return rows
@@ -140,8 +146,8 @@ def header(tri, split, device_name):
         "namespace tuning {",
         "",
         "// Householder tridiagonalisation by matrix order: orders up to max_order use `path`",
-        "// (2..16: one thread-block cluster of that many CTAs; 0: the grid-wide cooperative",
-        "// kernel).  Orders above the last entry use the grid kernel.",
+        "// (2..16: one thread-block cluster of that many CTAs; 0: the kernel over all",
+        "// SMs).  Orders above the last entry use the kernel over all SMs.",
         "struct TriEntry {",
         "  int max_order;",
         "  int path;",

@@ -1,8 +1,8 @@
 // Dense Hermitian eigensolver for the truncated factorizations:
-//   1. Householder reduction to a real symmetric tridiagonal T: one thread-block
-//      cluster holding the matrix in distributed shared memory (orders up to the tuning
-//      table's limit), else one cooperative kernel over all SMs with one grid barrier
-//      per column (the matrix stays L2-resident),
+//   1. Householder reduction to a real symmetric tridiagonal T with the matrix in shared
+//      memory, of one thread-block cluster (orders up to the tuning table's limit) or of
+//      all SMs (real orders to ~1770, complex ~1210); beyond that one cooperative kernel
+//      with one grid barrier per column (the matrix stays L2-resident),
 //   2. Cuppen divide and conquer on T (dc.cu),
 //   3. back-transformation of the kept eigenvectors with the Householder reflectors
 //      in blocks of 64 (compact WY, three GEMMs per block; every block's T factor is
@@ -59,11 +59,6 @@ template <>
 __device__ __forceinline__ double cone<double>() { return 1.0; }
 template <>
 __device__ __forceinline__ double2 cone<double2>() { return make_double2(1.0, 0.0); }
-__device__ __forceinline__ double cdiv(double a, double b) { return a / b; }
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
-  double den = b.x * b.x + b.y * b.y;
-  return make_double2((a.x * b.x + a.y * b.y) / den, (a.y * b.x - a.x * b.y) / den);
-}
 
 // v - a b - c d and acc + conj(a) b as chains of fused multiply-adds (two FP64
 // operations per real element: the FP64 pipe bounds the tridiagonalisation)
@@ -99,35 +94,9 @@ struct Barrier {
 // and whose further entries have squared norm xnorm2: beta = -sign(Re alpha) times the
 // column's norm, tau = (beta - alpha) / beta and the scale 1 / (alpha - beta) that turns
 // the column into the reflector v (v[0] = 1).  A zero tail under a real alpha needs no
-// reflection (tau = 0, beta = alpha).
-template <typename T>
-__device__ __forceinline__ void hh_scalars(T alpha, double xnorm2, T& tk, T& scale, double& beta, bool& active) {
-  const double ar = cre(alpha);
-  double ai = 0.0;
-  if constexpr (sizeof(T) == 16) ai = ((double2&)alpha).y;
-  tk = czero<T>();
-  scale = czero<T>();
-  beta = ar;
-  active = !(xnorm2 == 0.0 && ai == 0.0);
-  if (active) {
-    const double nrm = sqrt(ar * ar + ai * ai + xnorm2);
-    beta = ar >= 0 ? -nrm : nrm;
-    if constexpr (sizeof(T) == 16) {
-      double2 t2 = make_double2((beta - ar) / beta, -ai / beta);
-      tk = *(T*)&t2;
-      double2 inv = cdiv(make_double2(1.0, 0.0), make_double2(ar - beta, ai));
-      scale = *(T*)&inv;
-    } else {
-      double t1 = (beta - ar) / beta, s1 = 1.0 / (ar - beta);
-      tk = *(T*)&t1;
-      scale = *(T*)&s1;
-    }
-  }
-}
-
-// hh_scalars by one warp, its quotients spread over lanes (each lane runs the same
-// division on its own operands: one division sequence instead of two, or four for
-// complex data); lane 0 stores the results.  Same values as hh_scalars.
+// reflection (tau = 0, beta = alpha).  By one warp, the quotients spread over lanes (each
+// lane runs the same division on its own operands: one division sequence instead of two,
+// or four for complex data); lane 0 stores the results.
 template <typename T>
 __device__ __forceinline__ void hh_scalars_warp(T alpha, double xnorm2, int lane, T& tk, T& scale, double& beta,
                                                 bool& active) {
@@ -523,192 +492,480 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
-// Householder tridiagonalisation of a Hermitian matrix of moderate order (n <= ~640) by
-// one thread-block cluster: the matrix is held in the cluster's distributed shared
-// memory (column j in CTA j mod C, C <= 16), so a step's data never leaves the SMs and
-// its synchronisation is the hardware cluster barrier instead of a grid barrier over
-// global memory.  Same reflectors, tau, d and e as tridiag_kernel (the back-
-// transformation reads v_k below the subdiagonal of A's column k).
-// Step k: every CTA reads the pivot column from its owner (DSMEM), forms the reflector
-// (identically in every CTA: same data, same reduction order); each CTA forms
-// x_j = tau A22[:, j]^H v for its own columns; barrier; every CTA gathers x, forms
-// w = x - tau/2 (x^H v) v and applies A22 -= v w^H + w v^H to its own columns; barrier.
-constexpr int kClusterTriThreads = 256;
+// Householder tridiagonalisation with the matrix resident in shared memory: column j lives
+// in CTA j mod C for the whole reduction, so a step moves only one row of the matrix and the
+// vector x between SMs.  The CTAs are one thread-block cluster (both pushed to the peers'
+// shared memory, one cluster barrier per step) or, GRID, up to one per SM (exchanged through
+// L2 in 16-byte pieces that carry the step's number beside the value, so a consumer polls the
+// data itself: no counter, no fence, and no second round trip for the data after a barrier).
+// Same reflectors, tau, d and e as tridiag_kernel.
+//
+// Step k, with the rank-2 update of step k-1 pending (reflector v, x = tau A v):
+//   p = Re x^H v,  c = -|tau|^2 / Re(tau) p,  w'_j = x_j + c v_j:  A -= v w'^H + x v^H
+//   (the usual w = x + c/2 v enters both products; here all of c v v^H goes to the first, so
+//   w' is needed only at the CTA's own columns);
+//   a = the pivot column with the update applied, in every CTA (same data, same order);
+//   one pass over the own trailing columns applies the update and forms S_j = A[:, j]^H a;
+//   x_j = conj(A_k+1,j) - S_j / beta, sent with A_k+1,j, which the others take as the next
+//   pivot column (A is Hermitian).
+// v = scale a but for v_0 = 1, and tau scale = -1 / beta: the new x needs a reciprocal square
+// root and nothing else, and the column a is kept as it is, with scale in the coefficients.
+// A thread keeps the same rows (from the last one up, so that finished rows leave whole
+// iterations) through every phase of a step, so the vectors need no barrier of their own.
+//
+// Bound: the dependent chain of a step (gather, sum, pivot column, pass, publication; about
+// 5500 cycles at order 128), and from about order 700 the FP64 pipe (3 operations an
+// element).  An FP64 instruction of a warp holds its SM sub-partition for 64 cycles whatever
+// its active lanes, so the count of such instructions on the chain is what costs: one pass
+// warp per sub-partition (it fills the pipe with independent elements, and leaves less to sum
+// over the CTA), a further warp for the sums and scalars beside the pass, no loop unrolled
+// past the rows a thread has.  us per column, over all SMs against tridiag_kernel (above
+// order 384) or a cluster that read the pivot column and x from its peers in two barriers a
+// step: real order 128 2.8 / 4.2, 256 3.2 / 5.7, 512 4.4 / 7.8, 950 6.9 / 9.3; complex 128
+// 4.3 / 6.9, 256 6.1 / 11.9, 950 15.9 / 25.3.  One cluster: real 24 3.3 / 3.9, 64 3.2 / 3.8.
+// (Tried and slower: sums in exact integer arithmetic, 1050 cycles against 720 by shuffles;
+// the messages in several copies; x and the pivot column interleaved, twice the sectors.)
+constexpr int kResWarps = 4;                // pass warps
+constexpr int kResPass = 32 * kResWarps;    // pass threads
+constexpr int kResThreads = kResPass + 32;  // and the scalar warp
+constexpr int kResCols = 128;               // own columns of a CTA, at most
+constexpr int kPollDelay = 500;             // cycles between publishing and the first poll (order
+                                            // 256: 820 us, with none 1380, 300 875, 800 845)
 
-template <typename T>
-__global__ void __launch_bounds__(kClusterTriThreads)
-    tridiag_cluster_kernel(T* __restrict__ A, int n, double* __restrict__ d, double* __restrict__ e,
-                           T* __restrict__ tau, double2* __restrict__ phase) {
+__device__ __forceinline__ void put_tagged(ulonglong2* p, double v, unsigned long long tag) {
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ bool get_tagged(const ulonglong2* p, unsigned long long tag, double& v) {
+  unsigned long long a, b;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
+               : "=l"(a), "=l"(b)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double((long long)a);
+  return b == tag;
+}
+// row r's message, S_r and the next pivot column's entry, in two runs of n rows
+__device__ __forceinline__ void put_row(ulonglong2* buf, int n, int r, double S, double a, unsigned long long tag) {
+  put_tagged(buf + r, S, tag);
+  put_tagged(buf + n + r, a, tag);
+}
+__device__ __forceinline__ void put_row(ulonglong2* buf, int n, int r, double2 S, double2 a, unsigned long long tag) {
+  put_tagged(buf + 2 * r, S.x, tag);
+  put_tagged(buf + 2 * r + 1, S.y, tag);
+  put_tagged(buf + 2 * (n + r), a.x, tag);
+  put_tagged(buf + 2 * (n + r) + 1, a.y, tag);
+}
+__device__ __forceinline__ bool get_row(const ulonglong2* buf, int n, int r, unsigned long long tag, double& S, double& a) {
+  const bool k0 = get_tagged(buf + r, tag, S), k1 = get_tagged(buf + n + r, tag, a);
+  return k0 && k1;
+}
+__device__ __forceinline__ bool get_row(const ulonglong2* buf, int n, int r, unsigned long long tag, double2& S, double2& a) {
+  const bool k0 = get_tagged(buf + 2 * r, tag, S.x), k1 = get_tagged(buf + 2 * r + 1, tag, S.y);
+  const bool k2 = get_tagged(buf + 2 * (n + r), tag, a.x), k3 = get_tagged(buf + 2 * (n + r) + 1, tag, a.y);
+  return k0 && k1 && k2 && k3;
+}
+__device__ __forceinline__ double shfl_x(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ double2 shfl_x(double2 v, int o) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+// x + c v for a real c
+__device__ __forceinline__ double caxpy(double c, double v, double x) { return fma(c, v, x); }
+__device__ __forceinline__ double2 caxpy(double c, double2 v, double2 x) {
+  return make_double2(fma(c, v.x, x.x), fma(c, v.y, x.y));
+}
+// v - a b
+__device__ __forceinline__ double cfnma(double v, double a, double b) { return fma(-a, b, v); }
+__device__ __forceinline__ double2 cfnma(double2 v, double2 a, double2 b) {
+  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, v.x)), fma(-a.y, b.x, fma(-a.x, b.y, v.y)));
+}
+// s + |a|^2
+__device__ __forceinline__ double sqacc(double s, double a) { return fma(a, a, s); }
+__device__ __forceinline__ double sqacc(double s, double2 a) { return fma(a.y, a.y, fma(a.x, a.x, s)); }
+
+// barriers between the pass warps and the scalar warp: a side that has nothing to wait for
+// only arrives
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ bool not_zero(double a) { return (__double_as_longlong(a) << 1) != 0; }
+__device__ __forceinline__ bool not_zero(double2 a) { return not_zero(a.x) || not_zero(a.y); }
+
+// The pass over NB own columns from cols: update, dot products with a, and their sums over
+// the warp (part[b]; the values are reduced together: the first levels of the butterfly halve
+// those a lane holds, so that eight take 9 additions).  Rows rtop, rtop - kResPass, .. rlow.
+template <typename T, int NB>
+__device__ __forceinline__ void resident_pass(T* cols, int n, const T* wpc, const T* vpc, const T* uu, const T* xx,
+                                              const T* aa, int rtop, int rlow, int lane, T* part) {
+  constexpr int NP = NB > 4 ? 8 : NB > 2 ? 4 : NB;  // rounded to a power of two
+  T w[NB], v0[NB], acc[NP], nxt[NB];
+#pragma unroll
+  for (int b = 0; b < NP; ++b) acc[b] = czero<T>();
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    w[b] = wpc[b];
+    v0[b] = vpc[b];
+    nxt[b] = rtop >= rlow ? cols[(size_t)b * n + rtop] : czero<T>();
+  }
+  for (int r = rtop; r >= rlow; r -= kResPass) {
+    T val[NB];
+    const T ur = uu[r], xr = xx[r], ar = aa[r];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      val[b] = nxt[b];
+      if (r - kResPass >= rlow) nxt[b] = cols[(size_t)b * n + r - kResPass];
+    }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) val[b] = fnms2(val[b], ur, w[b], xr, v0[b]);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      acc[b] = fcma(acc[b], val[b], ar);
+      cols[(size_t)b * n + r] = val[b];
+    }
+  }
+  int o = 16;
+#pragma unroll
+  for (int h = NP / 2; h >= 1; h /= 2, o /= 2) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < h; ++i) {
+      const T send = up ? acc[i] : acc[i + h], keep = up ? acc[i + h] : acc[i];
+      acc[i] = cadd(keep, shfl_x(send, o));
+    }
+  }
+  for (; o > 0; o /= 2) acc[0] = cadd(acc[0], shfl_x(acc[0], o));
+  constexpr int kLow = 32 / NP;  // lanes that hold the same column's sum
+  if (lane % kLow == 0 && lane / kLow < NB) part[lane / kLow] = acc[0];
+}
+
+// A thread's rows of the messages with tag k, PU requested together; scalars() once, before
+// the first row is taken.  False when the wait gives up.
+template <typename T, int PU, typename Scalars, typename Take>
+__device__ __forceinline__ bool resident_gather(const ulonglong2* in, int n, int rtop, int k, Barrier* bar,
+                                                Scalars scalars, Take take) {
+  bool good = true, first = true;
+  for (int r0 = rtop; first || r0 >= k; r0 -= PU * kResPass, first = false) {
+    T S[PU], raw[PU];
+    for (int polls = 0;; ++polls) {
+      bool ok = true;
+#pragma unroll
+      for (int u = 0; u < PU; ++u) {
+        const int r = r0 - u * kResPass;
+        if (r >= k) ok = get_row(in, n, r, (unsigned long long)k, S[u], raw[u]) && ok;
+      }
+      if (ok) break;
+      if (polls > (1 << 22) || ((polls & 255) == 255 && *(volatile int*)&bar->err)) {
+        atomicExch(&bar->err, 1);
+        good = false;
+        break;
+      }
+    }
+    if (first) scalars();
+#pragma unroll
+    for (int u = 0; u < PU; ++u) {
+      const int r = r0 - u * kResPass;
+      if (r >= k) take(r, S[u], raw[u]);
+    }
+  }
+  return good;
+}
+
+template <typename T, bool GRID>
+__global__ void __launch_bounds__(kResThreads)
+    tridiag_resident_kernel(T* __restrict__ A, int n, double* __restrict__ d, double* __restrict__ e,
+                            T* __restrict__ tau, double2* __restrict__ phase, ulonglong2* xch, Barrier* bar) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  const int C = int(cluster.num_blocks());
-  const int rank = int(cluster.block_rank());
+  const int C = GRID ? int(gridDim.x) : int(cluster.num_blocks());
+  const int rank = GRID ? int(blockIdx.x) : int(cluster.block_rank());
   const int ncol = (n - rank + C - 1) / C;  // columns j = rank + C q, q < ncol
-  const int ncmax = (n + C - 1) / C;        // the layout is the same in every CTA (remote
-                                            // reads address a peer's arrays by this offset)
+  const int ncmax = (n + C - 1) / C;        // the layout is the same in every CTA (peers address it)
+  constexpr bool cplx = sizeof(T) == 16;
+  constexpr int kBatch = cplx ? 4 : 8;      // columns of one pass over the rows
+  constexpr int kScalars = 1, kSum = 2, kUpdate = 3, kNorm = 4, kColumns = 5;  // barriers
   extern __shared__ __align__(16) unsigned char ct_smem[];
   T* cols = (T*)ct_smem;               // own columns, n rows each
-  T* vcur = cols + (size_t)ncmax * n;  // reflector (rows k+1..n-1 at offsets 0..m-1)
-  T* xloc = vcur + n;                  // x_j of own columns (by global column index)
-  T* xall = xloc + n;                  // gathered x (rows k+1.. at offsets 0..)
-  T* wv = xall + n;                    // w
-  __shared__ T red[kClusterTriThreads / 32];
-  __shared__ double redd[kClusterTriThreads / 32];
+  T* abuf = cols + (size_t)ncmax * n;  // pivot columns of this step and the last, by step parity
+  T* xg = abuf + 2 * n;                // x; with the peers as writers of S by step parity, then
+                                       // the next pivot column likewise
+  __shared__ double psum[2][kResPass];
+  __shared__ T part[kResWarps][kResCols], wpc[kResCols], vpc[kResCols];
+  __shared__ T s_w0, s_scale;
+  __shared__ double s_c, s_f;
+  __shared__ int s_fail, s_tail;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = kClusterTriThreads / 32;
-  static_assert(NW >= 2 && (NW & (NW - 1)) == 0, "warp 0 plus dot-product warps, a power of two");
+  const bool scalar_warp = warp == kResWarps;
+  // the thread's rows: rtop - i kResPass; the last rows to the last pass warp, so that the
+  // warp beside the scalar warp on its sub-partition has the fewest
+  const int rtop = n - 1 - (tid ^ (kResPass - 32));
   for (int q = 0; q < ncol; ++q) {
     const T* src = A + (size_t)(rank + C * q) * n;
-    for (int r = tid; r < n; r += blockDim.x) cols[(size_t)q * n + r] = src[r];
+    for (int r = tid; r < n; r += kResThreads) cols[(size_t)q * n + r] = src[r];
   }
-  cluster.sync();
-  // block sums end in one warp (the warps' sums added in warp order), which also forms
-  // the step's scalars: on this GPU a warp-wide FP64 instruction holds a sub-partition's
-  // FP64 pipe for ~64 cycles, so a scalar chain repeated by every warp would take the
-  // CTA's FP64 issue for a step of its own
-  __shared__ T s_tk, s_scl, s_alpha2;
-  __shared__ double s_beta;
-  __shared__ bool s_active;
-  auto warp_sum_t = [&](T v) {
-    for (int o = 16; o > 0; o >>= 1) {
-      if constexpr (sizeof(T) == 8) {
-        v += __shfl_xor_sync(0xffffffffu, v, o);
-      } else {
-        double2 t2;
-        t2.x = __shfl_xor_sync(0xffffffffu, ((double2&)v).x, o);
-        t2.y = __shfl_xor_sync(0xffffffffu, ((double2&)v).y, o);
-        v = cadd(v, *(T*)&t2);
-      }
-    }
-    return v;
-  };
-  for (int k = 0; k < n - 2; ++k) {
-    const int m = n - k - 1;
-    const int owner = k % C;
-    const T* pcol = cluster.map_shared_rank(cols, owner) + (size_t)(k / C) * n;
-    // 1. the reflector from column k (rows k+1..n-1), in every CTA
-    double ss = 0.0;
-    for (int r = tid; r < m; r += blockDim.x) {
-      const T a = pcol[k + 1 + r];
-      vcur[r] = a;
-      if (r > 0) ss += cabs2(a);
-    }
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) redd[warp] = ss;
-    __syncthreads();  // publishes vcur (the column a, unscaled) and the warp sums
-    // warp 0 forms the reflector's scalars while the other warps form the dot products
-    // S_j = sum_i conj(A_ij) a_i of the own trailing columns with the column as it is
-    // (one warp per column): with v_0 = 1, v_i = scale a_i (i > 0) and
-    // alpha - beta = 1 / scale, A^H v = scale (S - beta conj(A_0,:))
-    if (warp == 0) {
-      // a tree over the warps' sums (lane 0 ends with the total; hh_scalars_warp takes
-      // lane 0's operands for every lane)
-      double xnorm2 = lane < NW ? redd[lane] : 0.0;
-      for (int o = NW / 2; o > 0; o >>= 1) xnorm2 += __shfl_xor_sync(0xffffffffu, xnorm2, o);
-      hh_scalars_warp(vcur[0], xnorm2, lane, s_tk, s_scl, s_beta, s_active);
-      if (rank == owner && lane == 0) {
-        d[k] = cre(pcol[k]);
-        e[k] = s_active ? s_beta : cre(vcur[0]);
-        tau[k] = s_tk;
-      }
-    }
-    // 2. x_j = tau sum_i conj(A_ij) v_i for the own trailing columns, one warp per column
-    //    on the warps other than warp 0
-    const int q0 = (k + 1 - rank + C - 1) / C;  // first own column index with j >= k+1
-    for (int q = warp > 0 ? q0 + warp - 1 : ncol; q < ncol; q += NW - 1) {
-      const int j = rank + C * q;
-      const T* cj = cols + (size_t)q * n + (k + 1);
-      T acc = czero<T>(), acc1 = czero<T>();
-      int r = lane;
-      for (; r + 32 < m; r += 64) {
-        acc = fcma(acc, cj[r], vcur[r]);
-        acc1 = fcma(acc1, cj[r + 32], vcur[r + 32]);
-      }
-      if (r < m) acc = fcma(acc, cj[r], vcur[r]);
-      acc = cadd(acc, acc1);
-      for (int o = 16; o > 0; o >>= 1) {
-        if constexpr (sizeof(T) == 8) {
-          acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        } else {
-          double2 t2;
-          t2.x = __shfl_xor_sync(0xffffffffu, ((double2&)acc).x, o);
-          t2.y = __shfl_xor_sync(0xffffffffu, ((double2&)acc).y, o);
-          acc = cadd(acc, *(T*)&t2);
-        }
-      }
-      if (lane == 0) xloc[j] = acc;
-    }
-    __syncthreads();  // publishes the scalars and the dot products
-    const T tk = s_tk, scl = s_scl;
-    const bool active = s_active;
-    {
-      const double beta = s_beta;
-      const T ts = cmulv(tk, scl);
-      for (int q = q0 + tid; q < ncol; q += blockDim.x) {
-        const int j = rank + C * q;
-        xloc[j] = cmulv(ts, csub(xloc[j], cscale(cconj(cols[(size_t)q * n + (k + 1)]), beta)));
-      }
-    }
-    for (int r = tid; r < m; r += blockDim.x) vcur[r] = (r == 0) ? cone<T>() : cmulv(vcur[r], scl);
-    cluster.sync();  // publishes x to the peers and the scaled reflector within the CTA
-    if (rank == owner) {
-      T* gcol = A + (size_t)k * n + (k + 1);
-      for (int r = tid + 1; r < m; r += blockDim.x) gcol[r] = vcur[r];
-    }
-    if (active) {
-      // 3. gather x, x^H v, w = x - tau/2 (x^H v) v
-      T pv = czero<T>();
-      for (int r = tid; r < m; r += blockDim.x) {
-        const int j = k + 1 + r;
-        const T xj = cluster.map_shared_rank(xloc, j % C)[j];
-        xall[r] = xj;
-        pv = cadd(pv, cmulv(cconj(xj), vcur[r]));
-      }
-      pv = warp_sum_t(pv);
-      if (lane == 0) red[warp] = pv;
-      __syncthreads();
-      if (warp == 0) {
-        T xv = lane < NW ? red[lane] : czero<T>();  // a tree over the warps' sums (lane 0)
-        for (int o = NW / 2; o > 0; o >>= 1) {
-          if constexpr (sizeof(T) == 8) {
-            xv += __shfl_xor_sync(0xffffffffu, xv, o);
-          } else {
-            double2 t2;
-            t2.x = __shfl_xor_sync(0xffffffffu, ((double2&)xv).x, o);
-            t2.y = __shfl_xor_sync(0xffffffffu, ((double2&)xv).y, o);
-            xv = cadd(xv, *(T*)&t2);
-          }
-        }
-        if (lane == 0) s_alpha2 = cscale(cmulv(tk, xv), -0.5);
-      }
-      __syncthreads();
-      const T alpha2 = s_alpha2;
-      for (int r = tid; r < m; r += blockDim.x) wv[r] = cadd(xall[r], cmulv(alpha2, vcur[r]));
-      __syncthreads();
-      // 4. A22 -= v w^H + w v^H on the own trailing columns
-      for (int q = q0 + warp; q < ncol; q += NW) {
-        const int jr = rank + C * q - (k + 1);
-        T* cj = cols + (size_t)q * n + (k + 1);
-        const T wj = cconj(wv[jr]), vj = cconj(vcur[jr]);
-        for (int r = lane; r < m; r += 32) cj[r] = fnms2(cj[r], vcur[r], wj, wv[r], vj);
-      }
-    }
+  for (int r = tid; r < n; r += kResThreads) abuf[n + r] = czero<T>();  // no update is pending at step 0
+  if (tid == 0) s_fail = s_tail = 0;
+  // the scalar warp's state of the pending update: scale, ctau = |tau|^2 / Re(tau) and
+  // m1 = -ctau scale
+  T scale = czero<T>(), m1 = czero<T>();
+  double ctau = 0.0;
+  if constexpr (GRID)
+    __syncthreads();
+  else
     cluster.sync();
-  }
-  // the last 2 x 2 block
-  if (n >= 2) {
-    const int o2 = (n - 2) % C, o1 = (n - 1) % C;
-    if (rank == o2 && tid == 0) {
-      const T* c2 = cols + (size_t)((n - 2) / C) * n;
-      const T a11 = c2[n - 2], a21 = c2[n - 1];
-      d[n - 2] = cre(a11);
-      e[n - 2] = last_offdiagonal(a21, phase);
+  auto warp_sum = [&](const double* v) {  // of kResPass values, on every lane of the scalar warp
+    static_assert(kResPass == 128, "four values per lane");
+    double s = (v[lane] + v[lane + 32]) + (v[lane + 64] + v[lane + 96]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+  };
+  for (int k = 0; k < n - 1; ++k) {
+    const int q0 = (k + 1 - rank + C - 1) / C, nown = ncol - q0;  // own trailing columns (j > k)
+    const bool last = k == n - 2;  // the final 2 x 2 block: nothing left to reflect
+    if (nown <= 0) {
+      if constexpr (GRID) return;
+      if (!last) cluster.sync();
+      continue;
     }
-    if (rank == o1 && tid == 0) d[n - 1] = cre(cols[(size_t)((n - 1) / C) * n + (n - 1)]);
-  } else if (rank == 0 && tid == 0) {
-    d[0] = cre(cols[0]);
+    const bool stores = rank == min(k + 1 + C / 2, n - 1) % C;  // this step's results are written by one CTA
+    T* aa = abuf + (k & 1) * n;
+    T* uu = abuf + ((k + 1) & 1) * n;
+    T* xx = GRID ? xg : xg + ((k + 1) & 1) * n;
+    if (scalar_warp) {
+      // c = -ctau (Re x_k + Re scale sum conj(x) a), and scale conj(w') at the own columns and
+      // (the last lane) at the pivot, whose v is 1; what does not need x comes before the wait
+      const bool at_pivot = lane == 31;
+      T vj = czero<T>(), sv = czero<T>();
+      int j = k;
+      auto own = [&](int q) {
+        j = rank + C * (q0 + q);
+        vj = cconj(cmulv(scale, uu[j]));
+        sv = cmulv(scale, vj);
+      };
+      if (at_pivot)
+        sv = scale;
+      else if (lane < nown)
+        own(lane);
+      bar_sync(kSum, kResThreads);
+      if (GRID && s_fail) {
+        bar_arrive(kUpdate, kResThreads);
+        return;
+      }
+      const double m0 = -ctau * cre(xx[k]);
+      T xj = cmulv(scale, cconj(xx[j]));
+      double c;
+      if constexpr (cplx)
+        c = fma(m1.x, warp_sum(psum[0]), fma(-m1.y, warp_sum(psum[1]), m0));
+      else
+        c = fma(m1, warp_sum(psum[0]), m0);
+      {
+        const T w = caxpy(c, sv, xj);
+        if (at_pivot) {
+          s_w0 = w;
+          s_c = c;
+        } else if (lane < nown) {
+          vpc[lane] = vj;
+          wpc[lane] = w;
+        }
+      }
+      for (int q = 31 + lane; q < nown; q += 32) {
+        own(q);
+        vpc[q] = vj;
+        wpc[q] = caxpy(c, sv, cmulv(scale, cconj(xx[j])));
+      }
+      bar_arrive(kUpdate, kResThreads);
+      // the scalars of column k's reflector, beside the pass
+      bar_sync(kNorm, kResThreads);
+      const T alpha = aa[k + 1];
+      if (last) {
+        if (stores && lane == 0) e[k] = last_offdiagonal(alpha, phase);
+        break;
+      }
+      const double x2 = warp_sum(psum[0]), ar = cre(alpha);
+      double ai = 0.0;
+      if constexpr (cplx) ai = alpha.y;
+      // (a norm whose square is subnormal has lost its digits, and H its orthogonality)
+      const bool active = __double2hiint(x2) >= 0x00100000 && (s_tail || not_zero(ai));
+      const double rr = active ? rsqrt(x2) : 0.0;
+      const bool neg = __double2hiint(ar) < 0;
+      __syncwarp();
+      if (lane == 0) {
+        s_f = neg ? -rr : rr;  // -1 / beta, or 0 for no reflection
+        s_tail = 0;
+      }
+      bar_arrive(kScalars, kResThreads);
+      T tk = czero<T>();
+      double beta = ar;
+      scale = czero<T>();
+      ctau = 0.0;
+      if (active) {
+        double nrm = x2 * rr;
+        nrm = fma(0.5 * rr, fma(-nrm, nrm, x2), nrm);
+        const double sg = neg ? -1.0 : 1.0, big = fabs(ar) + nrm;  // alpha - beta = (sg big, ai)
+        beta = neg ? nrm : -nrm;
+        if constexpr (cplx) {
+          const double inv = 1.0 / fma(ai, ai, big * big);
+          scale = make_double2(sg * big * inv, -ai * inv);
+          tk = make_double2(fma(fabs(ar), rr, 1.0), sg * ai * rr);
+          ctau = (tk.x * tk.x + tk.y * tk.y) / tk.x;
+        } else {
+          scale = sg / big;
+          tk = fma(fabs(ar), rr, 1.0);
+          ctau = tk;
+        }
+      }
+      m1 = cscale(scale, -ctau);
+      if (lane == 0) {
+        s_scale = scale;
+        if (stores) {
+          e[k] = beta;
+          tau[k] = tk;
+        }
+      }
+      if constexpr (!GRID) cluster.sync();
+      continue;
+    }
+    // 1. the pending update's x; sum of conj(x) a
+    T p = czero<T>();
+    double f = 0.0;
+    auto take = [&](int r, T S, T raw) {
+      const T x = not_zero(f) ? caxpy(f, S, raw) : czero<T>();
+      xx[r] = x;
+      aa[r] = not_zero(f) ? S : raw;
+      if (r > k) p = fcma(p, x, uu[r]);
+    };
+    if (k == 0) {
+      for (int r = rtop; r >= 0; r -= kResPass) take(r, czero<T>(), A[r]);
+    } else if constexpr (GRID) {
+      const ulonglong2* in = xch + (size_t)((k + 1) & 1) * (cplx ? 4 : 2) * n;
+      // polls that come before the messages slow down the stores they wait for
+      for (const long long t0 = clock64(); clock64() - t0 < kPollDelay;) {
+      }
+      bool ok = true;
+      const int nr = (n - k + kResPass - 1) / kResPass;  // rows of a thread, at most
+      auto scalars = [&] {
+        bar_sync(kScalars, kResThreads);
+        f = s_f;
+      };
+      if (nr == 1)
+        ok = resident_gather<T, 1>(in, n, rtop, k, bar, scalars, take);
+      else if (nr == 2)
+        ok = resident_gather<T, 2>(in, n, rtop, k, bar, scalars, take);
+      else if (nr <= 4 || cplx)
+        ok = resident_gather<T, 4>(in, n, rtop, k, bar, scalars, take);
+      else
+        ok = resident_gather<T, cplx ? 4 : 8>(in, n, rtop, k, bar, scalars, take);
+      if (!ok) s_fail = 1;
+    } else {
+      bar_sync(kScalars, kResThreads);
+      f = s_f;
+      const T* raw = xg + (2 + ((k + 1) & 1)) * n;
+      for (int r = rtop; r >= k; r -= kResPass) take(r, xx[r], raw[r]);
+    }
+    if constexpr (cplx) {
+      psum[0][tid] = p.x;
+      psum[1][tid] = p.y;
+    } else {
+      psum[0][tid] = p;
+    }
+    bar_arrive(kSum, kResThreads);
+    // 2. the pivot column: A_r,k - x_r = -f S_r without the term in v (v_k = 1), which comes
+    //    with c; its squared norm
+    if (not_zero(f))
+      for (int r = rtop; r >= k; r -= kResPass) aa[r] = cscale(aa[r], -f);
+    bar_sync(kUpdate, kResThreads);
+    if (GRID && s_fail) return;
+    const T w0 = s_w0, sc = s_scale;
+    bool tail = false;
+    double ss = 0.0;
+    for (int r = rtop; r > k; r -= kResPass) {
+      const T a = cfnma(aa[r], uu[r], w0);
+      aa[r] = a;
+      ss = sqacc(ss, a);
+      tail = tail || (r > k + 1 && not_zero(a));
+    }
+    psum[0][tid] = ss;
+    if (tail) s_tail = 1;
+    bar_arrive(kNorm, kResThreads);
+    // 3. the pass over the own columns
+    const bool rows = n - 1 - 32 * (kResWarps - 1 - warp) > k;  // does the warp hold trailing rows?
+    const int nbat = (nown + kBatch - 1) / kBatch, per = (nown + nbat - 1) / nbat;
+    for (int q = 0; q < nown; q += per) {
+      T* cq = cols + (size_t)(q0 + q) * n;
+      const int nb = min(per, nown - q);
+      if (!rows) {
+        if (lane < nb) part[warp][q + lane] = czero<T>();
+        continue;
+      }
+#define NSG_RESIDENT_PASS(NB) \
+  case NB:                    \
+    resident_pass<T, NB>(cq, n, wpc + q, vpc + q, uu, xx, aa, rtop, k + 1, lane, &part[warp][q]); \
+    break
+      switch (nb) {
+        NSG_RESIDENT_PASS(1);
+        NSG_RESIDENT_PASS(2);
+        NSG_RESIDENT_PASS(3);
+        NSG_RESIDENT_PASS(4);
+        default:
+          if constexpr (!cplx) {
+            switch (nb) {
+              NSG_RESIDENT_PASS(5);
+              NSG_RESIDENT_PASS(6);
+              NSG_RESIDENT_PASS(7);
+              NSG_RESIDENT_PASS(8);
+            }
+          }
+      }
+#undef NSG_RESIDENT_PASS
+    }
+    if (last) {
+      if (rtop == n - 1) d[n - 1] = cre(cols[(size_t)(ncol - 1) * n + n - 1]);
+    } else {
+      bar_sync(kColumns, kResPass);
+      // 4. S and row k+1 at the own columns, to everyone
+      auto sum_of = [&](int q, T& a0) {
+        static_assert(kResWarps == 4, "the tree below");
+        a0 = cconj(cols[(size_t)(q0 + q) * n + k + 1]);
+        return cadd(cadd(part[0][q], part[1][q]), cadd(part[2][q], part[3][q]));
+      };
+      if constexpr (GRID) {
+        ulonglong2* out = xch + (size_t)(k & 1) * (cplx ? 4 : 2) * n;
+        for (int q = tid; q < nown; q += kResPass) {
+          T a0;
+          const T S = sum_of(q, a0);
+          put_row(out, n, rank + C * (q0 + q), S, a0, (unsigned long long)(k + 1));
+        }
+      } else {
+        for (int i = tid; i < nown * C; i += kResPass) {
+          const int q = i / C, peer = i - q * C, j = rank + C * (q0 + q);
+          T a0;
+          const T S = sum_of(q, a0);
+          T* out = cluster.map_shared_rank(xg, peer) + (k & 1) * n;
+          out[j] = S;
+          out[2 * n + j] = a0;
+        }
+        cluster.barrier_arrive();
+      }
+    }
+    // d_k, and the last reflector to its place below the subdiagonal of column k-1 (column 0
+    // of A has been read by every CTA: each has published since)
+    if (stores) {
+      if ((rtop - k) % kResPass == 0) d[k] = cre(aa[k]) - (cre(xx[k]) + s_c);  // the thread that holds row k
+      if (k > 0) {
+        T* gcol = A + (size_t)(k - 1) * n;
+        for (int r = rtop; r > k; r -= kResPass) gcol[r] = cmulv(uu[r], sc);
+      }
+    }
+    if (last) break;
+    if constexpr (!GRID) cluster.barrier_wait();
   }
-  cluster.sync();  // no CTA leaves while another may still read its shared memory
+  if constexpr (!GRID) cluster.sync();  // no CTA leaves while another may still write its shared memory
 }
 
 // Eigenvectors first, first + step, ... of T (columns of Q) as the columns of Z, the last
@@ -941,10 +1198,9 @@ void BackTransform<T>::apply(T* Z, int64_t ldz, int64_t k) {
 
 // Cluster tridiagonalisation when the matrix fits the distributed shared memory of one
 // cluster (up to 16 CTAs of ~200 KB).  The cluster size comes from the tuning table by
-// order (measured: the reduction is FP64-bound on its C SMs, and a CTA's remote reads
-// per step do not grow with C; orders above the table take the grid kernel), or from the
-// context's override; it is raised until the columns fit.  Returns false (nothing
-// launched) for the grid kernel or when no cluster shape fits.
+// order (orders above the table take the kernel over all SMs), or from the context's
+// override; it is raised until the columns fit.  Returns false (nothing launched) when the
+// table or the override says so or when no cluster shape fits.
 template <typename T>
 static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* tau, double2* phase) {
   if (n < 3 || c->tune_tri == -1) return false;
@@ -958,16 +1214,17 @@ static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* ta
       }
     if (C == 0) return false;
   }
-  auto kfn = tridiag_cluster_kernel<T>;
+  auto kfn = tridiag_resident_kernel<T, false>;
+  static_assert(kResCols >= 111, "own columns of a CTA: order 222 on two");
   for (; C <= 16; C *= 2) {
     const size_t ncol = (size_t(n) + C - 1) / C;
-    const size_t smem = (ncol * n + 4 * size_t(n)) * eb;
-    if (smem > 200 * 1024) continue;
+    const size_t smem = (ncol * n + 6 * size_t(n)) * eb;
+    if (smem - 2 * size_t(n) * eb > 200 * 1024) continue;
     ensure_smem_limit((const void*)kfn, int(smem));
     if (C > 8) NSG_CUDA(cudaFuncSetAttribute((const void*)kfn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kClusterTriThreads);
+    cfg.blockDim = dim3(kResThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
@@ -983,12 +1240,37 @@ static bool tridiag_cluster(nsg_ctx* c, int n, T* A, double* d, double* e, T* ta
       continue;
     }
     ProfScope ps(c, NSG_PROF_TRIDIAG, (sizeof(T) == 16 ? 16.0 : 4.0) / 3.0 * double(n) * n * n);
-    NSG_CUDA(cudaLaunchKernelEx(&cfg, kfn, A, n, d, e, tau, phase));
+    NSG_CUDA(cudaLaunchKernelEx(&cfg, kfn, A, n, d, e, tau, phase, (ulonglong2*)nullptr, (Barrier*)nullptr));
     count_launch(c);
     check_launch("tridiag (cluster)");
     return true;
   }
   return false;
+}
+
+// The resident kernel over all SMs, when every CTA's columns fit its shared memory (real
+// orders up to ~1770, complex ~1210).  Returns false with nothing launched when they do not.
+template <typename T>
+static bool tridiag_resident(nsg_ctx* c, int n, T* A, double* d, double* e, T* tau, double2* phase, Barrier* bar) {
+  if (n < 3 || c->num_sms < 1) return false;
+  const int C = std::min(c->num_sms, n);
+  const size_t ncol = (size_t(n) + C - 1) / C, smem = (ncol * n + 3 * size_t(n)) * sizeof(T);
+  if (ncol > size_t(kResCols) || smem > 208 * 1024) return false;
+  auto kfn = tridiag_resident_kernel<T, true>;
+  ensure_smem_limit((const void*)kfn, int(smem));
+  int per_sm = 0;
+  NSG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, kResThreads, smem));
+  if (per_sm < 1) return false;
+  const size_t xbytes = sizeof(ulonglong2) * 4 * size_t(n) * (sizeof(T) / sizeof(double));
+  DevBuf xch(c, xbytes);
+  NSG_CUDA(cudaMemsetAsync(xch.p, 0, xbytes, c->stream));
+  ulonglong2* px = xch.as<ulonglong2>();
+  void* args[] = {&A, &n, &d, &e, &tau, &phase, &px, &bar};
+  ProfScope ps(c, NSG_PROF_TRIDIAG, (sizeof(T) == 16 ? 16.0 : 4.0) / 3.0 * double(n) * n * n);
+  NSG_CUDA(cudaLaunchCooperativeKernel((void*)kfn, dim3(C), dim3(kResThreads), args, smem, c->stream));
+  count_launch(c);
+  check_launch("tridiag (resident)");
+  return true;
 }
 
 // Hermitian eigen-decomposition of A (n x n, consumed).  Eigenvalues ascending into
@@ -1021,8 +1303,8 @@ static void syevd_dc_impl(nsg_ctx* c, int dtype, int n, T* A, std::vector<double
     const double2 one = make_double2(1.0, 0.0);
     NSG_CUDA(cudaMemcpyAsync(pph, &one, sizeof(double2), cudaMemcpyHostToDevice, c->stream));
     NSG_CUDA(cudaStreamSynchronize(c->stream));  // `one` leaves scope
-  } else if (!tridiag_cluster<T>(c, n, A, pd, pe, pt, pph)) {
-    // cooperative tridiagonalisation
+  } else if (!tridiag_cluster<T>(c, n, A, pd, pe, pt, pph) && !tridiag_resident<T>(c, n, A, pd, pe, pt, pph, &st->bar)) {
+    // cooperative tridiagonalisation, the matrix in L2
     int max_blocks = 0;
     size_t shm = eb * 3 * n;
     NSG_CHECK(shm <= 200 * 1024, NSG_ERR_UNSUPPORTED, "tridiagonalisation: matrix order too large");

@@ -9,14 +9,14 @@ namespace nsg {
 namespace tuning {
 
 // Householder tridiagonalisation by matrix order: orders up to max_order use `path`
-// (2..16: one thread-block cluster of that many CTAs; 0: the grid-wide cooperative
-// kernel).  Orders above the last entry use the grid kernel.
+// (2..16: one thread-block cluster of that many CTAs; 0: the kernel over all
+// SMs).  Orders above the last entry use the kernel over all SMs.
 struct TriEntry {
   int max_order;
   int path;
 };
 constexpr TriEntry kTri[] = {
-    {48, 8}, {384, 16},
+    {16, 8}, {64, 16},
 };
 
 // FP64 CUDA-core GEMM: number of K slices (split K) for products whose output has
