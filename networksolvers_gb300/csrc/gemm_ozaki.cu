@@ -13,8 +13,8 @@
 // chunk is exact.  Drain warps add the group sums of each chunk into double-float (hi, lo)
 // FP32 accumulators; the epilogue widens to FP64 and applies sigma_i tau_j, alpha and beta.
 // At the end of a chunk the tensor pipe waits for the accumulators' drain, so chunks are as
-// long as exactness allows: an H_eff product at bond dimension 1024 takes 0.94 ms with
-// chunks of 384, 0.97 with 256 and 1.07 with 128.  With S = 6 slices the result is
+// long as exactness allows: an H_eff product at bond dimension 1024 took 0.94 ms with
+// chunks of 384, 0.97 with 256 and 1.07 with 128 (0.78 since the epilogue below).  With S = 6 slices the result is
 // within ~2^-43 K sigma_i tau_j of A B (dropped slices and products).
 //
 // Kernel layout: 128 x 64 output tile per CTA, 16 drain warps (4 warpgroups, each
@@ -341,31 +341,33 @@ struct OzEpi {
   int a_batched, b_batched;
   int* err;
   // split K: grid z = batch x nsplit, split s takes K slabs [s split_slabs, ..) (whole
-  // exact chunks) and writes its scaled partial product to W[z] (M x N, column-major);
+  // multiples of 128) and writes its scaled partial product to W[z] (M x N, column-major);
   // oz_split_reduce_kernel adds the splits in order and applies alpha and beta
   int nsplit, split_slabs;
   double* W;
 };
 
-// float -> double by exponent re-bias (exact for normal floats; zero, subnormals, inf and
-// NaN take the conversion instruction)
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t b = __float_as_uint(f);
-  const uint32_t e = (b >> 23) & 0xFFu;
-  if (e == 0u || e == 0xFFu) return (double)f;
-  const uint64_t d = ((uint64_t)(b >> 31) << 63) | ((uint64_t)(e + 896u) << 52) | ((uint64_t)(b & 0x7FFFFFu) << 29);
-  return __longlong_as_double((long long)d);
-}
 // exponent k of a normal power of two 2^k
 __device__ __forceinline__ int pow2_exponent(double p) {
   return int((__double_as_longlong(p) >> 52) & 0x7FF) - 1023;
 }
-// v * 2^k by adding k to the exponent field when the result stays normal
-__device__ __forceinline__ double scale_pow2(double v, int k) {
-  const long long b = __double_as_longlong(v);
-  const int e = int((b >> 52) & 0x7FF);
-  if (e == 0 || e == 0x7FF || e + k <= 0 || e + k >= 0x7FF) return v * ldexp(1.0, k);
-  return __longlong_as_double(b + ((long long)k << 52));
+// f as a double, for a normal f or a zero: the exponent re-biased by integer arithmetic (a
+// conversion is one more operation of the FP64 pipe, which holds an SM sub-partition for 64
+// cycles per operation of a warp)
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), m = (b & 0x7fffffffu) >> 3;
+  const uint32_t hi = (b & 0x7f800000u) == 0 ? 0u : (b & 0x80000000u) | (m + (896u << 20));
+  return __hiloint2double(int(hi), int(b << 29));
+}
+// (hi + lo) 2^k: one FP64 operation, the scale added to the exponent field; out of the normal
+// range by two multiplications
+__device__ __forceinline__ double join_pow2(float hi, float lo, int k) {
+  const double v = widen(hi) + widen(lo);
+  const int vh = __double2hiint(v), e = (vh >> 20) & 0x7ff;
+  if (e == 0) return 0.0;  // both zero: the terms are multiples of 2^-7(S+1)
+  if (e + k < 1 || e + k > 2046)
+    return v * __hiloint2double((1023 + k / 2) << 20, 0) * __hiloint2double((1023 + k - k / 2) << 20, 0);
+  return __hiloint2double(vh + (k << 20), __double2loint(v));
 }
 
 __device__ __forceinline__ void two_sum_acc(float& hi, float& lo, float x) {
@@ -382,6 +384,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                    OzEpi ep) {
   constexpr int S = Oz<S_>::S, G = Oz<S_>::G, STAGES = Oz<S_>::STAGES, STAGE_BYTES = Oz<S_>::STAGE_BYTES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ int s_exp[BM + BN];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
   uint64_t* empty = full + STAGES;
@@ -396,6 +399,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int nkl = min(nk - tb, ep.split_slabs);  // its slabs; the pipeline counts from 0
   const int nchunks = (nkl + CHUNK_SLABS - 1) / CHUNK_SLABS;
 
+  if (tid == NDRAIN_WARPS * 32) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
+  }
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full[s], 1);
@@ -495,6 +502,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 #pragma unroll
     for (int j = 0; j < 16; ++j) hi[j] = lo[j] = 0.f;
     const uint32_t lane_base = (uint32_t)(wl * 32) << 16;
+    // the scales' exponents, for the epilogue
+    if (tid < BM)
+      s_exp[tid] = pow2_exponent(ep.sa[(ep.a_batched ? bz : 0) * ep.Mp + m0 + tid]);
+    else if (tid < BM + BN)
+      s_exp[tid] = pow2_exponent(ep.sb[(ep.b_batched ? bz : 0) * ep.Np + n0 + tid - BM]);
+    asm volatile("bar.sync 1, %0;" ::"n"(NDRAIN_WARPS * 32) : "memory");
     bool ok = true;
     for (int c = 0; c < nchunks; ++c) {
       if (!mbar_wait(accfull, c & 1, fail)) {
@@ -552,30 +565,41 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
     if (ok) {
-      // Epilogue with as few FP64-pipe operations as possible (GB300 runs FP64 at ~2 per
-      // clock per SM, and this loop touches every output): the FP32 pair is widened by
-      // exponent arithmetic, added with one DADD, and the power-of-two scales sigma_i tau_j
-      // are applied to the exponent field; alpha = 1 costs nothing further.
+      // Epilogue: no load between the stores (the scales' exponents are in shared memory) and
+      // one FP64 operation per output (GB300 runs FP64 at ~2 per clock per SM) but for alpha and
+      // beta: 6900 cycles a tile.  With the scales loaded between the stores, and conversions
+      // and multiplications the compiler ran for every value, it took 34000 of the 46000 cycles
+      // of a tile of depth 128 (integer arithmetic alone, correctly rounded: 9000).
       const int64_t row = m0 + wl * 32 + lane;
-      if (row < ep.M) {
-        const int ka = pow2_exponent(ep.sa[(ep.a_batched ? bz : 0) * ep.Mp + row]);
-        const bool unit_alpha = ep.alpha == 1.0;
-        double* Wz = ep.nsplit > 1 ? ep.W + (size_t)blockIdx.z * ep.M * ep.N : nullptr;
+      const int ka = s_exp[wl * 32 + lane];
+      double* Wz = ep.nsplit > 1 ? ep.W + (size_t)blockIdx.z * ep.M * ep.N : nullptr;
+      const int ncol = int(min((int64_t)16, ep.N - (n0 + 16 * q)));
+      if (row < ep.M && ncol > 0) {
+        double* cp = Wz ? Wz + row + (n0 + 16 * q) * ep.M : ep.C + bz * ep.sC + row * ep.crs + (n0 + 16 * q) * ep.ldc;
+        const int64_t step = Wz ? ep.M : ep.ldc;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int64_t col = n0 + 16 * q + j;
-          if (col < ep.N) {
-            const int kb = pow2_exponent(ep.sb[(ep.b_batched ? bz : 0) * ep.Np + col]);
-            double v = scale_pow2(widen(hi[j]) + widen(lo[j]), ka + kb);
-            if (ka > 1023 || kb > 1023) v = __longlong_as_double(0x7ff8000000000000ll);  // a row that is not finite
-            if (Wz) {
-              Wz[row + col * ep.M] = v;
-            } else {
-              if (!unit_alpha) v *= ep.alpha;
-              double* cp = ep.C + bz * ep.sC + row * ep.crs + col * ep.ldc;
-              *cp = (ep.beta == 0.0) ? v : fma(ep.beta, *cp, v);
-            }
+        for (int h = 0; h < 16; h += 8) {
+          double v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int kb = s_exp[BM + 16 * q + h + j];
+            v[j] = join_pow2(hi[h + j], lo[h + j], ka + kb);
+            if (ka > 1023 || kb > 1023) v[j] = __longlong_as_double(0x7ff8000000000000ll);  // a row that is not finite
           }
+          if (!Wz && ep.alpha != 1.0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] *= ep.alpha;
+          }
+          if (!Wz && ep.beta != 0.0) {
+            double old[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) old[j] = h + j < ncol ? cp[(h + j) * step] : 0.0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = fma(ep.beta, old[j], v[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (h + j < ncol) cp[(h + j) * step] = v[j];
         }
       }
     }
