@@ -162,11 +162,13 @@ void lanczos_step(nsg_ctx* c, nsg_linmap* m, std::vector<nsg_tensor*>& V, int j,
 // passes' coefficients and the sum of squares of w stay in `scal` (one block of
 // 4 (j + 1) + 2 doubles per step j, at step_offset(j)) and the next basis vector is
 // normalised by a kernel that reads that sum of squares, so the cycle issues no host
-// synchronisation; the host reads every scalar back once.  The kernels and the operand
-// order are those of lanczos_step, hence the same vectors.  All K steps run; steps after
-// a breakdown are discarded by the caller.
+// synchronisation; the host reads every scalar back once.  A step's vector work is one launch
+// (lanczos.cu), in the operations of lanczos_step; beyond the vectors that launch takes, the
+// kernels of lanczos_step.  All K steps run; steps after a breakdown are discarded by the
+// caller.
 static size_t step_offset(int j) { return size_t(2) * j * (j + 1) + size_t(2) * j; }  // sum_{i<j} (4 (i+1) + 2)
-void lanczos_cycle_dev(nsg_ctx* c, nsg_linmap* m, std::vector<nsg_tensor*>& V, int K, nsg_tensor* w, double* scal) {
+void lanczos_cycle_dev(nsg_ctx* c, nsg_linmap* m, LanczosVectors& lv, std::vector<nsg_tensor*>& V, int K, nsg_tensor* w,
+                       double* scal) {
   const int dt = w->dtype;
   const int64_t n = w->size;
   std::vector<const void*> ptrs;
@@ -176,9 +178,11 @@ void lanczos_cycle_dev(nsg_ctx* c, nsg_linmap* m, std::vector<nsg_tensor*>& V, i
     double* co2 = blk + 2 * (j + 1);
     double* ss = blk + 4 * (j + 1);
     linmap_apply(c, m, V[j], w);
-    if (j > 0) axpby_devscalar(c, dt, n, scal + step_offset(j - 1) + 4 * j, 1, V[j - 1]->data, w->data);
+    const double* prev = j > 0 ? scal + step_offset(j - 1) + 4 * j : nullptr;
     ptrs.assign(j + 1, nullptr);
     for (int i = 0; i <= j; ++i) ptrs[i] = V[i]->data;
+    if (lv.step(j + 1, ptrs.data(), w->data, prev, co1, co2, ss, j + 1 < K ? V[j + 1]->data : nullptr)) continue;
+    if (j > 0) axpby_devscalar(c, dt, n, prev, 1, V[j - 1]->data, w->data);
     multi_dot_dev(c, dt, n, j + 1, ptrs.data(), w->data, co1);
     multi_axpy_devcoef(c, dt, n, j + 1, ptrs.data(), co1, -1.0, w->data);
     multi_dot_dev(c, dt, n, j + 1, ptrs.data(), w->data, co2);
@@ -218,10 +222,9 @@ int nsg_eigsolve(nsg_ctx* c, nsg_linmap* m, nsg_tensor* x, int krylovdim, int ma
     ScopedBuf sb(c, sizeof(double) * nscal);
     double* scal = (double*)sb.p;
     double* sx = scal + step_offset(krylovdim);
-    const void* xp[1] = {x->data};
-    multi_dot_dev(c, dt, n, 1, xp, x->data, sx);
-    axpby_devscalar(c, dt, n, sx, 0, x->data, V[0]->data);
-    lanczos_cycle_dev(c, m, V, krylovdim, w, scal);
+    LanczosVectors lv(c, dt, n);
+    lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, V[0]->data);
+    lanczos_cycle_dev(c, m, lv, V, krylovdim, w, scal);
     std::vector<double> hs(nscal);
     NSG_CUDA(cudaMemcpyAsync(hs.data(), scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, c->stream));
     NSG_CUDA(cudaStreamSynchronize(c->stream));
@@ -255,9 +258,7 @@ int nsg_eigsolve(nsg_ctx* c, nsg_linmap* m, nsg_tensor* x, int krylovdim, int ma
       for (int j = 0; j < k; ++j) ptrs[j] = V[j]->data;
       NSG_CUDA(cudaMemsetAsync(x->data, 0, x->bytes, c->stream));
       multi_axpy(c, dt, n, k, ptrs.data(), coef.data(), x->data);
-      const void* xq[1] = {x->data};
-      multi_dot_dev(c, dt, n, 1, xq, x->data, sx);
-      axpby_devscalar(c, dt, n, sx, 0, x->data, x->data);
+      lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, x->data);
       *eigval = lam;
       if (numops) *numops = ops;
       check_device_flag(c);
@@ -353,10 +354,9 @@ int nsg_exponentiate(nsg_ctx* c, nsg_linmap* m, double t_re, double t_im, nsg_te
       ScopedBuf sb(c, sizeof(double) * nscal);
       double* scal = (double*)sb.p;
       double* sx = scal + step_offset(spec);
-      const void* xp[1] = {x->data};
-      multi_dot_dev(c, dt, n, 1, xp, x->data, sx);
-      axpby_devscalar(c, dt, n, sx, 0, x->data, V[0]->data);
-      lanczos_cycle_dev(c, m, V, spec, w, scal);
+      LanczosVectors lv(c, dt, n);
+      lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, V[0]->data);
+      lanczos_cycle_dev(c, m, lv, V, spec, w, scal);
       std::vector<double> hs(nscal);
       NSG_CUDA(cudaMemcpyAsync(hs.data(), scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, c->stream));
       NSG_CUDA(cudaStreamSynchronize(c->stream));

@@ -208,6 +208,24 @@ void multi_axpy_devcoef(nsg_ctx* c, int dtype, int64_t n, int nv, const void* co
 // y = x / sqrt(s) (mode 0) or y -= sqrt(s) x (mode 1), s = s_dev[0]
 void axpby_devscalar(nsg_ctx* c, int dtype, int64_t n, const double* s_dev, int mode, const void* x, void* y);
 double norm2(nsg_ctx* c, int dtype, int64_t n, const void* x);
+// The vector work of Lanczos steps on vectors of one length (lanczos.cu): w -= prev[1] v[nv-2]
+// (prev: the step before's ss; null: nothing), two Gram-Schmidt passes against v[0..nv) whose coefficients
+// (2 doubles each) go to co1 and co2, ss = {|w|^2, |w|}, next = w / |w| (unless null).  nv = 0:
+// w is only read.  Returns false, with nothing launched, for more vectors than it takes.
+struct LanczosVectors {
+  nsg_ctx* c;
+  int dtype;
+  int64_t n;
+  int grid = 1;
+  void* msg = nullptr;
+  size_t bytes = 0;
+  uint64_t tag = 1;
+  LanczosVectors(nsg_ctx* ctx, int dt, int64_t len);
+  ~LanczosVectors();
+  LanczosVectors(const LanczosVectors&) = delete;
+  LanczosVectors& operator=(const LanczosVectors&) = delete;
+  bool step(int nv, const void* const* v, void* w, const double* prev, double* co1, double* co2, double* ss, void* next);
+};
 double amax(nsg_ctx* c, int dtype, int64_t n, const void* x);  // max |component|
 void scale(nsg_ctx* c, int dtype, int64_t n, double ar, double ai, void* x);
 void copy_columns(nsg_ctx* c, int dtype, int64_t rows, int64_t ncols, const void* src,

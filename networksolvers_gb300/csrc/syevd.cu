@@ -14,6 +14,7 @@
 // Every wait in these kernels is bounded: the grid barrier gives up after ~2^26
 // polls, raises an error flag and the host reports NSG_ERR_TIMEOUT.
 #include "nsg_internal.h"
+#include "tagged.h"
 #include "tuning_table.h"
 
 #include <cooperative_groups.h>
@@ -532,20 +533,6 @@ constexpr int kResCols = 128;               // own columns of a CTA, at most
 constexpr int kPollDelay = 500;             // cycles between publishing and the first poll (order
                                             // 256: 820 us, with none 1380, 300 875, 800 845)
 
-__device__ __forceinline__ void put_tagged(ulonglong2* p, double v, unsigned long long tag) {
-  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}\n" ::"l"(p),
-               "l"(__double_as_longlong(v)), "l"(tag)
-               : "memory");
-}
-__device__ __forceinline__ bool get_tagged(const ulonglong2* p, unsigned long long tag, double& v) {
-  unsigned long long a, b;
-  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}\n"
-               : "=l"(a), "=l"(b)
-               : "l"(p)
-               : "memory");
-  v = __longlong_as_double((long long)a);
-  return b == tag;
-}
 // row r's message, S_r and the next pivot column's entry, in two runs of n rows
 __device__ __forceinline__ void put_row(ulonglong2* buf, int n, int r, double S, double a, unsigned long long tag) {
   put_tagged(buf + r, S, tag);
