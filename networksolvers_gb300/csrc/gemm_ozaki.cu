@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int nkl = min(nk - tb, ep.split_slabs);  // its slabs; the pipeline counts from 0
   const int nchunks = (nkl + CHUNK_SLABS - 1) / CHUNK_SLABS;
 
+  asm volatile("griddepcontrol.launch_dependents;");
   if (tid == NDRAIN_WARPS * 32) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
@@ -564,6 +565,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         hi[j] = s;
       }
     }
+    // a chained product updates C after the products before it, and ends after them; a partial
+    // product is its own and need not wait to be written
+    if (ep.nsplit == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (ok) {
       // Epilogue: no load between the stores (the scales' exponents are in shared memory) and
       // one FP64 operation per output (GB300 runs FP64 at ~2 per clock per SM) but for alpha and
@@ -603,24 +607,37 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         }
       }
     }
+    if (ep.nsplit > 1) asm volatile("griddepcontrol.wait;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
 }
 
-// C = alpha sum_s W[b nsplit + s] + beta C, the splits added in order
-__global__ void oz_split_reduce_kernel(const double* __restrict__ W, int nsplit, int64_t M, int64_t N,
-                                       int64_t batch, double* __restrict__ C, int64_t ldc, int64_t sC, int64_t crs,
-                                       double alpha, double beta) {
+// Products of one shape, C_t = alpha_t A_t B_t^T + beta_t C_t, in order (the parts of a complex
+// product; two of them share a C)
+struct OzTerms {
+  int n;
+  double* C[4];
+  double alpha[4], beta[4];
+};
+
+// C_t = alpha_t sum_s W[t][b nsplit + s] + beta_t C_t for the terms from `first` on, the splits
+// added in order
+__global__ void oz_split_reduce_kernel(const double* __restrict__ W, int nsplit, int64_t M, int64_t N, int64_t batch,
+                                       const __grid_constant__ OzTerms terms, int first, int64_t ldc, int64_t sC,
+                                       int64_t crs) {
   const int64_t MN = M * N, tot = MN * batch;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / MN, r = e - b * MN, row = r % M, col = r / M;
-    double acc = 0.0;
-    for (int sp = 0; sp < nsplit; ++sp) acc += W[(b * nsplit + sp) * MN + r];
-    const double v = alpha == 1.0 ? acc : acc * alpha;
-    double* cp = C + b * sC + row * crs + col * ldc;
-    *cp = (beta == 0.0) ? v : fma(beta, *cp, v);
+    for (int t = first; t < terms.n; ++t) {
+      const double* Wt = W + (t - first) * nsplit * tot;
+      double acc = 0.0;
+      for (int sp = 0; sp < nsplit; ++sp) acc += Wt[(b * nsplit + sp) * MN + r];
+      const double v = terms.alpha[t] == 1.0 ? acc : acc * terms.alpha[t];
+      double* cp = terms.C[t] + b * sC + row * crs + col * ldc;
+      *cp = (terms.beta[t] == 0.0) ? v : fma(terms.beta[t], *cp, v);
+    }
   }
 }
 
@@ -734,27 +751,30 @@ struct OzSlicer {
   }
 };
 
-// C (+)= alpha A B^T-form product of two prepared operands into C (stride ldc between
-// columns, sC between batch entries, crs between rows; all in doubles)
+// The terms' products of prepared operands (A[t], B[t]) into their C (stride ldc between
+// columns, sC between batch entries, crs between rows; all in doubles).  The launches after
+// the first are chained: they start while the one before still runs, on the SMs it leaves, and
+// wait for it before their epilogue (a complex product with its slicing, 640 x 512 x 128, 40
+// tiles a term: 104 us one term after the other, 77 chained; 4096 x 1024 x 1024: 909, 804).
 template <int S>
-void oz_product(nsg_ctx* c, const OzOperand& A, const OzOperand& B, int64_t M, int64_t N, int64_t K_p, int64_t batch,
-                double* C, int64_t ldc, int64_t sC, int64_t crs, double alpha, double beta, int64_t flop_k) {
+void oz_products(nsg_ctx* c, const OzOperand* const* A, const OzOperand* const* B, const OzTerms& terms, int64_t M,
+                 int64_t N, int64_t K_p, int64_t batch, int64_t ldc, int64_t sC, int64_t crs, int64_t flop_k) {
   constexpr int SMEM_BYTES = Oz<S>::SMEM_BYTES;
-  CUtensorMap mA = make_map(A.slices, A.rows_p, K_p, S * A.batch, BM, S),
-              mB = make_map(B.slices, B.rows_p, K_p, S * B.batch, BN, S);
+  const int64_t Mp = A[0]->rows_p, Np = B[0]->rows_p;
   int* err = device_flag(c);  // checked once at the end of the public call
   ensure_smem_limit((const void*)oz_gemm_kernel<S>, SMEM_BYTES);
-  // split K over whole exact chunks when the output tiles would leave most SMs idle
-  // (the small products of a converged sweep: 32-64 tiles of 128 x 64 on 152 SMs)
+  // split K when the output tiles would leave most SMs idle (the small products of a
+  // converged sweep: 32-64 tiles of 128 x 64 on 152 SMs)
   const int nk = int(K_p / BKS), units = (nk + SPLIT_SLABS - 1) / SPLIT_SLABS;
-  const int64_t tiles = (A.rows_p / BM) * (B.rows_p / BN) * batch;
+  const int64_t tiles = (Mp / BM) * (Np / BN) * batch;
   const int64_t sms = c->num_sms > 0 ? c->num_sms : 152;
   int nsplit = 1;
   if (tiles * 2 <= sms && units >= 2)
     nsplit = int(std::min<int64_t>({(int64_t)units, sms / tiles, 16, 65535 / batch}));
   const int split_slabs = (units + nsplit - 1) / nsplit * SPLIT_SLABS;
   nsplit = (nk + split_slabs - 1) / split_slabs;
-  // the partial products' workspace, only when K is split (freed on every exit)
+  // the partial products' workspace, only when K is split (freed on every exit): of all terms,
+  // reduced together, or where that does not fit of one term at a time
   struct Partials {
     nsg_ctx* c;
     void* p;
@@ -766,24 +786,51 @@ void oz_product(nsg_ctx* c, const OzOperand& A, const OzOperand& B, int64_t M, i
       }
     }
   } wbuf{c, nullptr, 0};
+  const size_t term_w = size_t(nsplit) * size_t(batch) * size_t(M) * size_t(N);
+  bool together = terms.n > 1;
   if (nsplit > 1) {
-    wbuf.bytes = sizeof(double) * size_t(nsplit) * size_t(batch) * size_t(M) * size_t(N);
-    wbuf.p = dalloc(c, wbuf.bytes);
-  }
-  OzEpi ep{C,        ldc,         sC,          M,     N,     crs,  alpha, beta, A.scales, B.scales, A.rows_p, B.rows_p,
-           A.batch > 1, B.batch > 1, err, nsplit, split_slabs, (double*)wbuf.p};
-  dim3 grid(unsigned(A.rows_p / BM), unsigned(B.rows_p / BN), unsigned(batch * nsplit));
-  {
-    ProfScope ps(c, NSG_PROF_TC_GEMM, 2.0 * double(M) * double(N) * double(flop_k) * double(batch));
-    oz_gemm_kernel<S><<<grid, NTHREADS, SMEM_BYTES, c->stream>>>(mA, mB, nk, ep);
-    if (nsplit > 1) {
-      const int64_t tot = M * N * batch;
-      const int rg = int(std::min<int64_t>((tot + 255) / 256, sms * 8));
-      oz_split_reduce_kernel<<<rg, 256, 0, c->stream>>>((const double*)wbuf.p, nsplit, M, N, batch, C, ldc, sC, crs,
-                                                        alpha, beta);
+    for (;;) {
+      const size_t bytes = sizeof(double) * term_w * (together ? terms.n : 1);
+      try {
+        wbuf.p = dalloc(c, bytes);
+        wbuf.bytes = bytes;
+        break;
+      } catch (const Error& e) {
+        if (!together || e.code != NSG_ERR_OOM) throw;
+        together = false;
+      }
     }
   }
-  count_launch(c, nsplit > 1 ? 2 : 1);
+  for (int t = 0; t < terms.n; ++t) {
+    const CUtensorMap mA = make_map(A[t]->slices, Mp, K_p, S * A[t]->batch, BM, S),
+                      mB = make_map(B[t]->slices, Np, K_p, S * B[t]->batch, BN, S);
+    double* W = nsplit > 1 ? (double*)wbuf.p + (together ? t * term_w : 0) : nullptr;
+    const OzEpi ep{terms.C[t],       ldc,          sC,           M,            N,   crs, terms.alpha[t], terms.beta[t],
+                   A[t]->scales,     B[t]->scales, Mp,           Np,           A[t]->batch > 1, B[t]->batch > 1,
+                   err,              nsplit,       split_slabs,  W};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(Mp / BM), unsigned(Np / BN), unsigned(batch * nsplit));
+    cfg.blockDim = dim3(NTHREADS);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = t > 0 && (nsplit == 1 || together) ? 1 : 0;
+    const bool reduce = nsplit > 1 && (!together || t + 1 == terms.n);
+    ProfScope ps(c, NSG_PROF_TC_GEMM, 2.0 * double(M) * double(N) * double(flop_k) * double(batch));
+    NSG_CUDA(cudaLaunchKernelEx(&cfg, oz_gemm_kernel<S>, mA, mB, nk, ep));
+    if (reduce) {
+      const int64_t tot = M * N * batch;
+      const int rg = int(std::min<int64_t>((tot + 255) / 256, sms * 8));
+      OzTerms upto = terms;
+      upto.n = t + 1;
+      oz_split_reduce_kernel<<<rg, 256, 0, c->stream>>>((const double*)wbuf.p, nsplit, M, N, batch, upto,
+                                                        together ? 0 : t, ldc, sC, crs);
+    }
+    count_launch(c, reduce ? 2 : 1);
+  }
   check_launch("oz_gemm");
 }
 
@@ -809,7 +856,9 @@ bool gemm_ozaki_impl(nsg_ctx* c, const GemmArgs& g) {
     OzOperand A = sl.add((const double*)g.A, g.M, ars, aks, g.strideA, ab, Mp);
     OzOperand B = sl.add((const double*)g.B, g.N, brs, bks, g.strideB, bb, Np);
     sl.run();
-    oz_product<S>(c, A, B, g.M, g.N, Kp, g.batch, (double*)g.C, g.ldc, g.strideC, 1, g.alpha_re, g.beta_re, g.K);
+    const OzOperand *pa[1] = {&A}, *pb[1] = {&B};
+    const OzTerms terms{1, {(double*)g.C}, {g.alpha_re}, {g.beta_re}};
+    oz_products<S>(c, pa, pb, terms, g.M, g.N, Kp, g.batch, g.ldc, g.strideC, 1, g.K);
     return true;
   }
   // complex: A = Ar + i sa Ai, B = Br + i sb Bi (sa, sb = -1 for conjugated operands), as
@@ -828,13 +877,10 @@ bool gemm_ozaki_impl(nsg_ctx* c, const GemmArgs& g) {
   OzOperand Bi = sl.add(Bd + 1, g.N, 2 * brs, 2 * bks, 2 * g.strideB, bb, Np);
   sl.run();
   double* Cr = (double*)g.C;
-  double* Ci = Cr + 1;
-  const int64_t ldc = 2 * g.ldc, sC = 2 * g.strideC;
   const double al = g.alpha_re, be = g.beta_re;
-  oz_product<S>(c, Ar, Br, g.M, g.N, Kp, g.batch, Cr, ldc, sC, 2, al, be, g.K);
-  oz_product<S>(c, Ai, Bi, g.M, g.N, Kp, g.batch, Cr, ldc, sC, 2, -sa * sbs * al, 1.0, g.K);
-  oz_product<S>(c, Ar, Bi, g.M, g.N, Kp, g.batch, Ci, ldc, sC, 2, sbs * al, be, g.K);
-  oz_product<S>(c, Ai, Br, g.M, g.N, Kp, g.batch, Ci, ldc, sC, 2, sa * al, 1.0, g.K);
+  const OzOperand *pa[4] = {&Ar, &Ai, &Ar, &Ai}, *pb[4] = {&Br, &Bi, &Bi, &Br};
+  const OzTerms terms{4, {Cr, Cr, Cr + 1, Cr + 1}, {al, -sa * sbs * al, sbs * al, sa * al}, {be, 1.0, be, 1.0}};
+  oz_products<S>(c, pa, pb, terms, g.M, g.N, Kp, g.batch, 2 * g.ldc, 2 * g.strideC, 2, g.K);
   return true;
 }
 

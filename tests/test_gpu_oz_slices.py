@@ -99,3 +99,27 @@ def test_zero_extreme_and_non_finite_rows(nsg_ctx, precision):
             assert np.array_equal(got2[keep], got[keep])
     finally:
         nsg_ctx.set_precision("fp64")
+
+
+def test_partial_products_of_one_term_at_a_time(nsg_ctx):
+    """A complex product whose K is split keeps the partial products of its four terms; where the
+    budget has no room for them, of one term at a time, with the same result."""
+    from networksolvers_gb300 import _native
+    rng = np.random.default_rng(3)
+    m, n, k = 512, 128, 1280
+    a, b = rnd(rng, (m, k), True), rnd(rng, (k, n), True)
+    i, j, l = Index(m), Index(n), Index(k)
+    got, budget = [], 0
+    try:
+        for _ in range(2):
+            ctx = _native.Context(0, hbm_budget=budget, precision="ozaki")
+            _native.set_default_context(ctx)
+            A, B = DTensor.from_numpy(a, [i, l]), DTensor.from_numpy(b, [l, j])
+            C = contract([A, B], out=[i, j])
+            got.append(C.to_numpy())
+            budget = ctx.memory()[1] - 2 * 8 * 2 * m * n  # two terms' partial products, of two splits or more
+            del A, B, C
+    finally:
+        _native.set_default_context(nsg_ctx)
+    assert np.array_equal(got[0], got[1])
+    assert np.max(np.abs(got[0] - a @ b)) < 8 * k * 2.0 ** -42 * np.abs(a).max() * np.abs(b).max()
