@@ -3,6 +3,7 @@
 //
 // All reductions are two-stage with a fixed summation order, so results are
 // bit-reproducible run to run (no floating-point atomics).
+#include "chained.h"
 #include "nsg_internal.h"
 
 #include <cmath>
@@ -36,7 +37,9 @@ struct PermParams {
 
 template <typename T, bool CONJ>
 __global__ void __launch_bounds__(kThreads)
-    permute_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t n, PermParams p) {
+    permute_kernel(const T* __restrict__ in_, T* __restrict__ out, int64_t n, PermParams p) {
+  chained_start();
+  const T* __restrict__ in = after_start(in_);
   for (int64_t o = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; o < n; o += int64_t(gridDim.x) * blockDim.x) {
     int64_t rem = o, src = 0;
     for (int k = 0; k < p.rank; ++k) {
@@ -55,7 +58,9 @@ __global__ void __launch_bounds__(kThreads)
 // case where the fastest output axis group is not the fastest input group.
 template <typename T, bool CONJ>
 __global__ void __launch_bounds__(kThreads)
-    transpose3_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t A, int64_t B, int64_t Cn) {
+    transpose3_kernel(const T* __restrict__ in_, T* __restrict__ out, int64_t A, int64_t B, int64_t Cn) {
+  chained_start();
+  const T* __restrict__ in = after_start(in_);
   __shared__ T tile[32][33];
   int64_t ntA = (A + 31) / 32, ntB = (B + 31) / 32;
   int64_t ntiles = ntA * ntB * Cn;
@@ -324,7 +329,7 @@ void launch_permute(nsg_ctx* c, const nsg_tensor* x, nsg_tensor* out, const int*
       int64_t cap = int64_t(c->num_sms) * 16;
       int grid = int(tiles < cap ? tiles : cap);
       if (grid < 1) grid = 1;
-      transpose3_kernel<T, CONJ><<<grid, kThreads, 0, c->stream>>>((const T*)x->data, (T*)out->data, A, B, Cn);
+      launch_chained(c, transpose3_kernel<T, CONJ>, grid, kThreads, 0, (const T*)x->data, (T*)out->data, A, B, Cn);
       count_launch(c);
       check_launch("transpose3");
       return;
@@ -336,8 +341,8 @@ void launch_permute(nsg_ctx* c, const nsg_tensor* x, nsg_tensor* out, const int*
     p.odims[k] = x->dims[perm[k]];
     p.istride[k] = instr[perm[k]];
   }
-  permute_kernel<T, CONJ><<<grid_for(c, x->size), kThreads, 0, c->stream>>>((const T*)x->data, (T*)out->data,
-                                                                          x->size, p);
+  launch_chained(c, permute_kernel<T, CONJ>, grid_for(c, x->size), kThreads, 0, (const T*)x->data, (T*)out->data,
+                 x->size, p);
   count_launch(c);
   check_launch("permute");
 }

@@ -7,6 +7,7 @@
 // others, and a row-per-thread form for products with a sparse operator tensor.  Loads
 // are mapped so that consecutive threads touch consecutive addresses for either operand
 // orientation.
+#include "chained.h"
 #include "nsg_internal.h"
 
 #include <cooperative_groups.h>
@@ -307,10 +308,14 @@ __global__ void __launch_bounds__(kTileThreads)
 constexpr int kSkinnyThreads = 256;
 template <typename T, int CW>
 __global__ void __launch_bounds__(kSkinnyThreads)
-    gemm_skinny_kernel(int64_t M, int64_t rows, int N, int K, const T* __restrict__ A, int64_t lda, int64_t sA,
-                       bool conjA, const T* __restrict__ B, int64_t ldb, int64_t sB, int opB, T* __restrict__ C,
+    gemm_skinny_kernel(int64_t M, int64_t rows, int N, int K, const T* __restrict__ A_, int64_t lda, int64_t sA,
+                       bool conjA, const T* __restrict__ B_, int64_t ldb, int64_t sB, int opB, T* __restrict__ C,
                        int64_t ldc, int64_t sC, int64_t groups, Scal<T> sc, bool plain) {
   extern __shared__ __align__(16) unsigned char sk_smem[];
+  // (many rows, CW = 1: not chained, and the loads through the read-only path)
+  if constexpr (CW > 1) chained_start();
+  const T* __restrict__ A = CW > 1 ? after_start(A_) : A_;
+  const T* __restrict__ B = CW > 1 ? after_start(B_) : B_;
   constexpr int R = kSkinnyThreads / CW;     // rows per CTA
   T* As = (T*)sk_smem;                       // [K][R]
   __shared__ T Bs[32][33];                   // op(B)
@@ -445,9 +450,15 @@ void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
       constexpr int CW = decltype(cw)::value, R = kSkinnyThreads / CW;
       const int grid = int(std::min<int64_t>((rows + R - 1) / R * groups, sms * 16));
       ensure_smem_limit((const void*)gemm_skinny_kernel<T, CW>, 32 * R * int(sizeof(T)));
-      gemm_skinny_kernel<T, CW><<<grid, kSkinnyThreads, size_t(g.K) * R * sizeof(T), c->stream>>>(
-          g.M, rows, int(g.N), int(g.K), (const T*)g.A, g.lda, g.strideA, g.opA == OP_R, (const T*)g.B, g.ldb,
-          g.strideB, g.opB, (T*)g.C, g.ldc, g.strideC, groups, sc, plain);
+      const auto launch = [&](auto... args) {
+        const size_t smem = size_t(g.K) * R * sizeof(T);
+        if constexpr (CW > 1)
+          launch_chained(c, gemm_skinny_kernel<T, CW>, grid, kSkinnyThreads, smem, args...);
+        else
+          gemm_skinny_kernel<T, CW><<<grid, kSkinnyThreads, smem, c->stream>>>(args...);
+      };
+      launch(g.M, rows, int(g.N), int(g.K), (const T*)g.A, g.lda, g.strideA, g.opA == OP_R, (const T*)g.B, g.ldb,
+             g.strideB, g.opB, (T*)g.C, g.ldc, g.strideC, groups, sc, plain);
     };
     auto pick = [&](auto sc) {
       if (col_warps == 1)

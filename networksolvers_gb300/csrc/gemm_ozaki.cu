@@ -22,6 +22,7 @@
 // holding all six slices of A and B (SWIZZLE_64B); 6 x 64 TMEM accumulator columns.
 // All mbarrier waits are bounded; on time-out the CTA raises the error flag, drains its
 // TMA copies (bounded), frees its TMEM and returns.
+#include "chained.h"
 #include "nsg_internal.h"
 
 #include <cooperative_groups.h>
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_shallow_kernel(const _
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double tile[kTileBytes / 8];
   __shared__ unsigned rowmax[kSliceRows], rowexp[kSliceRows];
+  chained_start();
   const int C = int(cluster.num_blocks()), rank = int(cluster.block_rank()), tid = threadIdx.x;
   int64_t t = blockIdx.x / C;
   int o = 0;
@@ -345,6 +347,7 @@ struct OzEpi {
   // oz_split_reduce_kernel adds the splits in order and applies alpha and beta
   int nsplit, split_slabs;
   double* W;
+  int chained;  // the slices were complete before the launch before this one
 };
 
 // exponent k of a normal power of two 2^k
@@ -399,7 +402,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   const int nkl = min(nk - tb, ep.split_slabs);  // its slabs; the pipeline counts from 0
   const int nchunks = (nkl + CHUNK_SLABS - 1) / CHUNK_SLABS;
 
-  asm volatile("griddepcontrol.launch_dependents;");
+  if (ep.chained) asm volatile("griddepcontrol.launch_dependents;");
   if (tid == NDRAIN_WARPS * 32) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapA) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&mapB) : "memory");
@@ -422,6 +425,11 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  // the first product's slices come from the kernel before it
+  if (!ep.chained) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+  }
   const uint32_t tmem = *tmem_slot;
 
   if (warp == NDRAIN_WARPS) {
@@ -624,9 +632,10 @@ struct OzTerms {
 
 // C_t = alpha_t sum_s W[t][b nsplit + s] + beta_t C_t for the terms from `first` on, the splits
 // added in order
-__global__ void oz_split_reduce_kernel(const double* __restrict__ W, int nsplit, int64_t M, int64_t N, int64_t batch,
+__global__ void oz_split_reduce_kernel(const double* W, int nsplit, int64_t M, int64_t N, int64_t batch,
                                        const __grid_constant__ OzTerms terms, int first, int64_t ldc, int64_t sC,
                                        int64_t crs) {
+  chained_start();
   const int64_t MN = M * N, tot = MN * batch;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < tot; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t b = e / MN, r = e - b * MN, row = r % M, col = r / M;
@@ -726,13 +735,13 @@ struct OzSlicer {
       cfg.gridDim = dim3(unsigned(tiles * C));
       cfg.blockDim = dim3(kSliceThreads);
       cfg.stream = c->stream;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = C;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
+      cudaLaunchAttribute attr[2] = {chained_attribute()};
+      attr[1].id = cudaLaunchAttributeClusterDimension;
+      attr[1].val.clusterDim.x = C;
+      attr[1].val.clusterDim.y = 1;
+      attr[1].val.clusterDim.z = 1;
       cfg.attrs = attr;
-      cfg.numAttrs = 1;
+      cfg.numAttrs = 2;
       NSG_CUDA(cudaLaunchKernelEx(&cfg, oz_slice_shallow_kernel<S>, P));
       count_launch(c);
     } else {
@@ -807,17 +816,15 @@ void oz_products(nsg_ctx* c, const OzOperand* const* A, const OzOperand* const* 
     double* W = nsplit > 1 ? (double*)wbuf.p + (together ? t * term_w : 0) : nullptr;
     const OzEpi ep{terms.C[t],       ldc,          sC,           M,            N,   crs, terms.alpha[t], terms.beta[t],
                    A[t]->scales,     B[t]->scales, Mp,           Np,           A[t]->batch > 1, B[t]->batch > 1,
-                   err,              nsplit,       split_slabs,  W};
+                   err,              nsplit,       split_slabs,  W,            t > 0 && (nsplit == 1 || together)};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(Mp / BM), unsigned(Np / BN), unsigned(batch * nsplit));
     cfg.blockDim = dim3(NTHREADS);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = c->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[1] = {chained_attribute()};
     cfg.attrs = attr;
-    cfg.numAttrs = t > 0 && (nsplit == 1 || together) ? 1 : 0;
+    cfg.numAttrs = 1;
     const bool reduce = nsplit > 1 && (!together || t + 1 == terms.n);
     ProfScope ps(c, NSG_PROF_TC_GEMM, 2.0 * double(M) * double(N) * double(flop_k) * double(batch));
     NSG_CUDA(cudaLaunchKernelEx(&cfg, oz_gemm_kernel<S>, mA, mB, nk, ep));
@@ -826,8 +833,8 @@ void oz_products(nsg_ctx* c, const OzOperand* const* A, const OzOperand* const* 
       const int rg = int(std::min<int64_t>((tot + 255) / 256, sms * 8));
       OzTerms upto = terms;
       upto.n = t + 1;
-      oz_split_reduce_kernel<<<rg, 256, 0, c->stream>>>((const double*)wbuf.p, nsplit, M, N, batch, upto,
-                                                        together ? 0 : t, ldc, sC, crs);
+      launch_chained(c, oz_split_reduce_kernel, rg, 256, 0, (const double*)wbuf.p, nsplit, M, N, batch, upto,
+                     together ? 0 : t, ldc, sC, crs);
     }
     count_launch(c, reduce ? 2 : 1);
   }
