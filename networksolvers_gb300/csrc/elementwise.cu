@@ -246,38 +246,6 @@ __global__ void axpby_devscalar_kernel(int64_t n, const double* __restrict__ s_d
   }
 }
 
-template <typename T>
-__global__ void copy_columns_kernel(int64_t rows, int64_t ncols, const T* __restrict__ src, int64_t lds,
-                                    const int* __restrict__ colidx, T* __restrict__ dst, int64_t ldd) {
-  int64_t n = rows * ncols;
-  for (int64_t e = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; e < n; e += int64_t(gridDim.x) * blockDim.x) {
-    int64_t i = e % rows, k = e / rows;
-    int64_t sc = colidx ? colidx[k] : k;
-    dst[i + k * ldd] = src[i + sc * lds];
-  }
-}
-
-template <bool CPLX>
-__global__ void row_norms_kernel(int64_t rows, int64_t cols, const void* A_, int64_t lda, double* out) {
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < rows; i += int64_t(gridDim.x) * blockDim.x) {
-    double s = 0.0;
-    if constexpr (CPLX) {
-      const double2* A = (const double2*)A_;
-      for (int64_t j = 0; j < cols; ++j) {
-        double2 a = A[i + j * lda];
-        s = fma(a.x, a.x, fma(a.y, a.y, s));
-      }
-    } else {
-      const double* A = (const double*)A_;
-      for (int64_t j = 0; j < cols; ++j) {
-        double a = A[i + j * lda];
-        s = fma(a, a, s);
-      }
-    }
-    out[i] = s;
-  }
-}
-
 __global__ void amax_partial_kernel(int64_t n, const double* __restrict__ x, double* __restrict__ partial) {
   __shared__ double red[kThreads];
   double m = 0.0;
@@ -483,28 +451,6 @@ double norm2(nsg_ctx* c, int dtype, int64_t n, const void* x) {
   return mx * std::sqrt(out[0] > 0 ? out[0] : 0.0);
 }
 
-void copy_columns(nsg_ctx* c, int dtype, int64_t rows, int64_t ncols, const void* src, int64_t lds,
-                  const int* d_colidx, void* dst, int64_t ldd) {
-  if (rows * ncols == 0) return;
-  int grid = grid_for(c, rows * ncols);
-  if (dtype == NSG_C128)
-    copy_columns_kernel<double2><<<grid, kThreads, 0, c->stream>>>(rows, ncols, (const double2*)src, lds, d_colidx,
-                                                                  (double2*)dst, ldd);
-  else
-    copy_columns_kernel<double><<<grid, kThreads, 0, c->stream>>>(rows, ncols, (const double*)src, lds, d_colidx,
-                                                                 (double*)dst, ldd);
-  count_launch(c);
-  check_launch("copy_columns");
-}
-
-void copy_rows(nsg_ctx* c, int dtype, int64_t nrows_out, int64_t ncols, const void* src, int64_t lds, void* dst,
-               int64_t ldd) {
-  // rows [0, nrows_out) of a column-major matrix = a strided 2-D copy
-  size_t eb = elem_bytes(dtype);
-  NSG_CUDA(cudaMemcpy2DAsync(dst, ldd * eb, src, lds * eb, nrows_out * eb, ncols, cudaMemcpyDeviceToDevice,
-                             c->stream));
-}
-
 double amax(nsg_ctx* c, int dtype, int64_t n, const void* x) {
   // complex: max over real and imaginary parts (a factor sqrt(2) of the modulus at most)
   int64_t nd = dtype == NSG_C128 ? 2 * n : n;
@@ -519,16 +465,6 @@ double amax(nsg_ctx* c, int dtype, int64_t n, const void* x) {
   double m = 0.0;
   for (double v : h) m = std::fmax(m, v);
   return m;
-}
-
-void row_norms2(nsg_ctx* c, int dtype, int64_t rows, int64_t cols, const void* A, int64_t lda, double* out_dev) {
-  int grid = grid_for(c, rows);
-  if (dtype == NSG_C128)
-    row_norms_kernel<true><<<grid, kThreads, 0, c->stream>>>(rows, cols, A, lda, out_dev);
-  else
-    row_norms_kernel<false><<<grid, kThreads, 0, c->stream>>>(rows, cols, A, lda, out_dev);
-  count_launch(c);
-  check_launch("row_norms");
 }
 
 }  // namespace nsg

@@ -228,12 +228,6 @@ struct LanczosVectors {
 };
 double amax(nsg_ctx* c, int dtype, int64_t n, const void* x);  // max |component|
 void scale(nsg_ctx* c, int dtype, int64_t n, double ar, double ai, void* x);
-void copy_columns(nsg_ctx* c, int dtype, int64_t rows, int64_t ncols, const void* src,
-                  int64_t lds, const int* d_colidx, void* dst, int64_t ldd);
-void copy_rows(nsg_ctx* c, int dtype, int64_t nrows_out, int64_t ncols, const void* src,
-               int64_t lds, void* dst, int64_t ldd);
-void row_norms2(nsg_ctx* c, int dtype, int64_t rows, int64_t cols, const void* A, int64_t lda,
-                double* out_dev);
 
 // Eigen-decomposition of the real symmetric tridiagonal (d, e) on the device (dc.cu):
 // eigenvalues ascending into w, eigenvectors into the returned one of the n x n buffers Q0
