@@ -162,7 +162,7 @@ class Context:
 
     def set_tuning(self, param, value):
         """Launch-choice override (0 restores the compiled-in tuning table): param
-        "splitk" (FP64 GEMM K slices, 1..64), "tridiag" (-1 grid kernel, 2..16 cluster)
+        "splitk" (64 x 64-tile FP64 products, 1..64 K slices), "tridiag" (-1 all SMs, 2..16 cluster)
         or "dc_leaf" (divide and conquer leaf order, 4..32)."""
         code = {"splitk": 0, "tridiag": 1, "dc_leaf": 2}[param]
         self.check(self.L.nsg_ctx_set_tuning(self.h, code, int(value)))
