@@ -130,7 +130,8 @@ struct PairPlan {
   bool batched_b() const { return lb.contiguous && lb.s > 0 && lb.s + K.n < b.n; }
 };
 
-PairPlan plan_pair(const Labs& labA, double sizeA, const Labs& labB, double sizeB) {
+template <typename Dim>  // dim(label): its extent
+PairPlan plan_pair(const Labs& labA, double sizeA, const Labs& labB, double sizeB, Dim dim) {
   PairPlan p;
   p.a = labA;
   p.b = labB;
@@ -164,6 +165,22 @@ PairPlan plan_pair(const Labs& labA, double sizeA, const Labs& labB, double size
   } else if (!p.lb.contiguous) {
     canon_B(p.la.korder);
   }
+  // A batched product is as wide as the batched operand's first free labels: a site label of
+  // extent 2 there leaves a tensor-core tile 2 columns (and an FP64 tile 2 of its 16).  One
+  // permutation makes it wide: products 256 x 2 x 1280 by 512 of the environments took two
+  // thirds of the FP64 time of a sweep (N = 22, bonds to 256: FP64 products 101 ms of four
+  // sweeps, 46 with the permutation).
+  auto extent = [&](const Labs& x, int from, int to) {
+    double e = 1;
+    for (int k = from; k < to; ++k) e *= double(dim(x.v[k]));
+    return e;
+  };
+  auto thin = [&](const Labs& x, const Layout& L) {
+    const double inner = extent(x, 0, L.s), batch = extent(x, L.s + p.K.n, x.n);
+    return inner < 32 && inner * batch >= 64 && extent(p.K, 0, p.K.n) >= 64;
+  };
+  if (p.batched_a() && thin(p.a, p.la)) canon_A(p.lb.korder);
+  if (p.batched_b() && thin(p.b, p.lb)) canon_B(p.la.korder);
   if (p.batched_a() && p.batched_b()) {
     if (sizeA <= sizeB)
       canon_A(p.lb.korder);
@@ -210,14 +227,14 @@ int with_conj(int op, bool conj) {
 static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_order, nsg_tensor* into) {
   NSG_CHECK(A.t->dtype == B.t->dtype, NSG_ERR_INVALID, "contract: dtype mismatch");
   const int dtype = A.t->dtype;
-  const PairPlan plan = plan_pair(A.lab, double(A.t->size), B.lab, double(B.t->size));
-  const Labs& K = plan.K;
-  const Layout &la = plan.la, &lb = plan.lb;
   auto dim_of = [&](int l) -> int64_t {
     int p = pos_of(A.lab, l);
     if (p >= 0) return A.t->dims[p];
     return B.t->dims[pos_of(B.lab, l)];
   };
+  const PairPlan plan = plan_pair(A.lab, double(A.t->size), B.lab, double(B.t->size), dim_of);
+  const Labs& K = plan.K;
+  const Layout &la = plan.la, &lb = plan.lb;
   for (int l : K)
     NSG_CHECK(A.t->dims[pos_of(A.lab, l)] == B.t->dims[pos_of(B.lab, l)], NSG_ERR_INVALID,
               "contract: dimension mismatch on a shared label");
@@ -491,7 +508,7 @@ static Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
             const Cand &ca = st[A].cands[swap ? j : i], &cb = st[B].cands[swap ? i : j];
             Cand q;
             q.moved = ca.moved + cb.moved;
-            const PairPlan p = plan_pair(ca.order, st[A].size, cb.order, st[B].size);
+            const PairPlan p = plan_pair(ca.order, st[A].size, cb.order, st[B].size, [&](int l) { return dims.at(l); });
             if (p.perm_a) q.moved += st[A].size + kPermLaunch;
             if (p.perm_b) q.moved += st[B].size + kPermLaunch;
             q.order = p.out;
@@ -707,7 +724,7 @@ int nsg_linmap_create(nsg_ctx* c, int n_fixed, nsg_tensor* const* fixed, const i
     LT r = eval_node(c, m, int(ni), dummy, nullptr, nullptr);
     // in the order in which every application will read it
     const Node &l = m->tree.nodes[up->left], &rt = m->tree.nodes[up->right];
-    const PairPlan plan = plan_pair(l.order, l.size, rt.order, rt.size);
+    const PairPlan plan = plan_pair(l.order, l.size, rt.order, rt.size, [&](int x) { return dims.at(x); });
     const bool is_left = up->left == int(ni);
     if (is_left ? plan.perm_a : plan.perm_b) {
       LT q = permute_to(c, r, (is_left ? plan.a : plan.b).list());

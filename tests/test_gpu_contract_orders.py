@@ -100,3 +100,25 @@ def test_linear_map_layouts(nsg_ctx, seed, cplx):
         ref = einsum(legs + [x], arrays + [v], out)
         mag = einsum(legs + [x], [np.abs(t) for t in arrays] + [np.abs(v)], out)
         assert np.all(np.abs(got - ref) <= 1e-12 * mag + 1e-300)
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-13), ("ozaki", 1e-10)])
+@pytest.mark.parametrize("d,k,b", [(2, 64, 32), (2, 80, 40), (31, 64, 3), (32, 64, 5), (2, 63, 40), (2, 80, 31)])
+def test_thin_batched_products(nsg_ctx, precision, tol, d, k, b):
+    """The contracted label between a small free label and a large one, on either side (a batched
+    product d columns wide, or one wide product of the permuted operand), at the edges of the rule."""
+    rng = np.random.default_rng(d + k + b)
+    m = 96
+    p, q, s, r = Index(m), Index(k), Index(d), Index(b)
+    x, y = rng.standard_normal((m, k)), rng.standard_normal((d, k, b))
+    nsg_ctx.set_precision(precision)
+    try:
+        X, Y = DTensor.from_numpy(x, [p, q]), DTensor.from_numpy(y, [s, q, r])
+        got = contract([X, Y], out=[p, s, r]).to_numpy()
+        swapped = contract([Y, X], out=[s, r, p]).to_numpy()
+    finally:
+        nsg_ctx.set_precision("fp64")
+    ref = np.einsum("pq,sqr->psr", x, y)
+    bound = tol * np.abs(x).max() * np.abs(y).max() * k
+    assert np.max(np.abs(got - ref)) < bound
+    assert np.max(np.abs(swapped - ref.transpose(1, 2, 0))) < bound
