@@ -539,15 +539,25 @@ int nsg_eigh(nsg_ctx* c, const nsg_tensor* rho, const int* row_axes, int n_row, 
   NSG_CHECK(m == ncol, NSG_ERR_INVALID, "eigh: row and column spaces differ in size");
   const int dt = rho->dtype;
   const size_t eb = elem_bytes(dt);
+  // The reduction squares column norms and takes a subnormal square for no coupling: entries
+  // far from 1 (densities of un-normalised networks) are brought there by a power of two,
+  // which changes no digit, and the eigenvalues scaled back.
+  const double mx = amax(c, dt, M->size, M->data);
+  int ex = 0;
+  if (mx > 0 && std::isfinite(mx)) std::frexp(mx, &ex);
+  ex = std::abs(ex) > 256 ? std::max(-1000, std::min(1000, ex)) : 0;
   void* A = dalloc(c, eb * m * m);
   NSG_CUDA(cudaMemcpyAsync(A, M->data, eb * m * m, cudaMemcpyDeviceToDevice, c->stream));
   if (owned) free_tensor(c, M);
+  if (ex != 0) scale(c, dt, m * m, std::ldexp(1.0, -ex), 0.0, A);
   double err = 0.0;
   int64_t k = 0;
   nsg_tensor* Ut = nullptr;
   std::vector<double> P, w;
   PickFn pick = [&](const std::vector<double>& wa, void** Z, int64_t* ldz) {
     P.assign(wa.rbegin(), wa.rend());
+    if (ex != 0)
+      for (double& x : P) x = std::ldexp(x, ex);
     k = truncate_rule(P, m, cutoff, maxdim, mindim, &err);
     std::vector<int64_t> udims = rdims;
     udims.push_back(k);

@@ -78,3 +78,12 @@ def test_non_finite(nsg_ctx, path, bad):
     with pytest.raises(NsgError):
         check(nsg_ctx, A, path, vectors=False)
     check(nsg_ctx, hermitian(np.random.default_rng(2), 200, False), path)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("n", [40, 140])
+def test_norms_whose_squares_leave_the_range(nsg_ctx, n, cplx):
+    full = hermitian(np.random.default_rng(n), n, cplx)
+    for path in (4, -1):
+        for s in (1e-155, 1e-160, 1e-200, 1e-280, 1e160, 1e280):
+            check(nsg_ctx, full * s, path)
