@@ -83,9 +83,9 @@ static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_or
     if (p >= 0) return A.t->dims[p];
     return B.t->dims[pos_of(B.lab, l)];
   };
-  const PairPlan plan = plan_pair(A.lab, double(A.t->size), B.lab, double(B.t->size), dim_of);
-  const Labs& K = plan.K;
-  const Layout &la = plan.la, &lb = plan.lb;
+  const PairPlan<int> plan = plan_pair<int>(A.lab, double(A.t->size), B.lab, double(B.t->size), dim_of);
+  const Labs<int>& K = plan.K;
+  const Layout<int> &la = plan.la, &lb = plan.lb;
   for (int l : K)
     NSG_CHECK(A.t->dims[pos_of(A.lab, l)] == B.t->dims[pos_of(B.lab, l)], NSG_ERR_INVALID,
               "contract: dimension mismatch on a shared label");
@@ -408,7 +408,7 @@ int nsg_linmap_create(nsg_ctx* c, int n_fixed, nsg_tensor* const* fixed, const i
     LT r = eval_node(c, m, int(ni), dummy, nullptr, nullptr);
     // in the order in which every application will read it
     const Node &l = m->tree.nodes[up->left], &rt = m->tree.nodes[up->right];
-    const PairPlan plan = plan_pair(l.order, l.size, rt.order, rt.size, [&](int x) { return dims.at(x); });
+    const PairPlan<int> plan = plan_pair(l.order, l.size, rt.order, rt.size, [&](int x) { return dims.at(x); });
     const bool is_left = up->left == int(ni);
     if (is_left ? plan.perm_a : plan.perm_b) {
       LT q = permute_to(c, r, (is_left ? plan.a : plan.b).list());

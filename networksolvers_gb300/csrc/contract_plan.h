@@ -7,31 +7,35 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <functional>
+#include <iterator>
 #include <unordered_map>
 #include <vector>
 
 namespace nsg {
 
-// A short list of labels without an allocation (the planning below forms thousands).
+// A short list of labels without an allocation (the planning below forms thousands).  V: int
+// for the caller's labels, a byte for the search's own numbering of them.
+template <typename V>
 struct Labs {
   int n = 0;
-  int v[2 * NSG_MAX_RANK];
+  V v[2 * NSG_MAX_RANK];
   Labs() {}
   Labs(const std::vector<int>& x) {
     NSG_CHECK(x.size() <= 2 * NSG_MAX_RANK, NSG_ERR_UNSUPPORTED, "contract: result rank above 16");
-    for (int l : x) push_back(l);
+    for (int l : x) push_back(V(l));
   }
-  void push_back(int l) {
+  void push_back(V l) {
     NSG_CHECK(n < 2 * NSG_MAX_RANK, NSG_ERR_UNSUPPORTED, "contract: result rank above 16");
     v[n++] = l;
   }
   void append(const Labs& o, int from, int to) {
     for (int k = from; k < to; ++k) push_back(o.v[k]);
   }
-  const int* begin() const { return v; }
-  const int* end() const { return v + n; }
-  int at(int l) const {
+  const V* begin() const { return v; }
+  const V* end() const { return v + n; }
+  int at(V l) const {
     for (int k = 0; k < n; ++k)
       if (v[k] == l) return k;
     return -1;
@@ -42,14 +46,16 @@ struct Labs {
 };
 
 // Where the contracted labels sit inside an operand: [F1, K, F2] with K contiguous.
+template <typename V>
 struct Layout {
   bool contiguous = false;
-  int s = 0;     // first K position
-  Labs korder;   // K labels in stored order
+  int s = 0;       // first K position
+  Labs<V> korder;  // K labels in stored order
 };
 
-inline Layout classify(const Labs& lab, const Labs& K) {
-  Layout L;
+template <typename V>
+Layout<V> classify(const Labs<V>& lab, const Labs<V>& K) {
+  Layout<V> L;
   if (K.n == 0) {
     L.contiguous = true;
     L.s = lab.n;
@@ -69,35 +75,36 @@ inline Layout classify(const Labs& lab, const Labs& K) {
 
 // How two labelled operands are contracted over their shared labels K: the order each is
 // brought to first (its own when it is used in place) and the result's label order.
+template <typename V>
 struct PairPlan {
-  Labs K, a, b, out;
-  Layout la, lb;
+  Labs<V> K, a, b, out;
+  Layout<V> la, lb;
   bool perm_a = false, perm_b = false;
   bool batched_a() const { return la.contiguous && la.s > 0 && la.s + K.n < a.n; }
   bool batched_b() const { return lb.contiguous && lb.s > 0 && lb.s + K.n < b.n; }
 };
 
-template <typename Dim>  // dim(label): its extent
-PairPlan plan_pair(const Labs& labA, double sizeA, const Labs& labB, double sizeB, Dim dim) {
-  PairPlan p;
+template <typename V, typename Dim>  // dim(label): its extent
+PairPlan<V> plan_pair(const Labs<V>& labA, double sizeA, const Labs<V>& labB, double sizeB, Dim dim) {
+  PairPlan<V> p;
   p.a = labA;
   p.b = labB;
-  for (int l : labA)
+  for (V l : labA)
     if (labB.at(l) >= 0) p.K.push_back(l);
   p.la = classify(p.a, p.K);
   p.lb = classify(p.b, p.K);
-  auto canon_A = [&](const Labs& korder) {
-    Labs ord;
-    for (int l : p.a)
+  auto canon_A = [&](const Labs<V>& korder) {
+    Labs<V> ord;
+    for (V l : p.a)
       if (p.K.at(l) < 0) ord.push_back(l);
     ord.append(korder, 0, korder.n);
     p.a = ord;
     p.perm_a = true;
     p.la = classify(p.a, p.K);
   };
-  auto canon_B = [&](const Labs& korder) {
-    Labs ord = korder;
-    for (int l : p.b)
+  auto canon_B = [&](const Labs<V>& korder) {
+    Labs<V> ord = korder;
+    for (V l : p.b)
       if (p.K.at(l) < 0) ord.push_back(l);
     p.b = ord;
     p.perm_b = true;
@@ -117,12 +124,12 @@ PairPlan plan_pair(const Labs& labA, double sizeA, const Labs& labB, double size
   // permutation makes it wide: products 256 x 2 x 1280 by 512 of the environments took two
   // thirds of the FP64 time of a sweep (N = 22, bonds to 256: FP64 products 101 ms of four
   // sweeps, 46 with the permutation).
-  auto extent = [&](const Labs& x, int from, int to) {
+  auto extent = [&](const Labs<V>& x, int from, int to) {
     double e = 1;
     for (int k = from; k < to; ++k) e *= double(dim(x.v[k]));
     return e;
   };
-  auto thin = [&](const Labs& x, const Layout& L) {
+  auto thin = [&](const Labs<V>& x, const Layout<V>& L) {
     const double inner = extent(x, 0, L.s), batch = extent(x, L.s + p.K.n, x.n);
     return inner < 32 && inner * batch >= 64 && extent(p.K, 0, p.K.n) >= 64;
   };
@@ -168,7 +175,7 @@ struct Node {
   int leaf = -1;          // tensor index for leaves
   int left = -1, right = -1;
   uint32_t mask = 0;
-  Labs order;              // labels of the intermediate, as contract_pair leaves them
+  Labs<int> order;         // labels of the intermediate, as contract_pair leaves them
   double size = 1;         // its elements
   double flops = 0;        // MACs of this step
 };
@@ -177,6 +184,7 @@ struct Tree {
   std::vector<Node> nodes;
   int root = -1;
   double total_macs = 0;
+  double moved = 0;        // what its permutations cost
 };
 
 // Exact flop-optimal pairwise order (dynamic programming over subsets).  Trees of equal
@@ -184,65 +192,95 @@ struct Tree {
 // differ in the permutations that contract_pair needs: among them one that moves little
 // data is taken, a permutation counting as its elements plus kPermLaunch for the launch.
 // For that a subset keeps, of its flop-optimal trees, the cheapest per order of its result
-// (up to kOrders of them, and none that a permutation of the cheapest would beat).  (Taking
-// the first tree cost a permutation of the 168 MB intermediate per application at bond
-// dimension 1024: 0.6 of 3.5 ms.)
+// (none that a permutation of the cheapest would beat).  (Taking the first tree cost a
+// permutation of the 168 MB intermediate per application at bond dimension 1024: 0.6 of
+// 3.5 ms.)
+//
+// Where bonds are equal, or 1 as in a product state, almost every tree ties.  The search is
+// cut to a number of pair plans that takes no longer than the dynamic programming itself:
+// fewer splits per subset, and fewer orders, the more trees tie.  Planning times, host of the
+// GPU machine's class: H_eff of a chain 8 us, environment at a vertex of degree 6 0.3 ms, twelve
+// tensors with bonds 1 7 ms; without the limit 13 us, 3.7 ms, 6 s as a chain and 56 s as a star.
 constexpr double kPermLaunch = 2e4;
-constexpr size_t kOrders = 6;
+struct SearchLimit {
+  int splits, orders;
+};
+constexpr SearchLimit kSearch[] = {{1 << 12, 6}, {4, 6}, {3, 3}, {2, 2}, {1, 1}};
 
 inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::vector<int>& out_labels,
                          const std::unordered_map<int, int64_t>& dims) {
+  using L = Labs<uint8_t>;
   const int n = int(labs.size());
   NSG_CHECK(n >= 1 && n <= 12, NSG_ERR_UNSUPPORTED, "contract: 1..12 tensors");
   const uint32_t full = (1u << n) - 1;
-  // labels: the tensors that hold each, its dimension, whether it is in the result
+  // labels, numbered: the tensors that hold each, its dimension, whether it is in the result
   struct Label {
+    int name;
     uint32_t where = 0;
     double dim = 1;
     bool out = false;
   };
   std::vector<Label> lab;
+  std::vector<L> of(n);
+  L result;
   {
     std::unordered_map<int, int> index;
-    auto label_of = [&](int l) -> Label& {
+    auto number = [&](int l) {
       auto it = index.emplace(l, int(lab.size()));
-      if (it.second) {
-        lab.push_back(Label());
-        lab.back().dim = double(dims.at(l));
-      }
-      return lab[it.first->second];
+      if (it.second) lab.push_back(Label{l, 0, double(dims.at(l)), false});
+      return it.first->second;  // (12 tensors of 16 labels and 16 of the result at most)
     };
     for (int i = 0; i < n; ++i)
-      for (int l : labs[i]) label_of(l).where |= 1u << i;
-    for (int l : out_labels) label_of(l).out = true;
+      for (int l : labs[i]) {
+        const int k = number(l);
+        lab[k].where |= 1u << i;
+        of[i].push_back(uint8_t(k));
+      }
+    for (int l : out_labels) {
+      const int k = number(l);
+      lab[k].out = true;
+      result.push_back(uint8_t(k));
+    }
   }
-  auto open_in = [&](const Label& l, uint32_t S) { return (l.where & S) && ((l.where & ~S & full) || l.out); };
+  auto dim = [&](uint8_t l) { return lab[l].dim; };
+  // labels open in a subset, as a bit set
+  constexpr int kWords = 4;
+  const int words = int(lab.size() + 63) / 64;
+  struct Set {
+    uint64_t w[kWords] = {};
+  };
+  auto extent = [&](const Set& a, const Set& b) {  // of the union
+    double e = 1;
+    for (int k = 0; k < words; ++k)
+      for (uint64_t m = a.w[k] | b.w[k]; m; m &= m - 1) e *= lab[64 * k + __builtin_ctzll(m)].dim;
+    return e;
+  };
   struct Cand {
     double moved = 0;
-    Labs order;
+    L order;
     uint32_t left = 0, right = 0;
     int ci = 0, cj = 0;  // the parts' candidates
   };
   struct State {
     double flops = 0, size = 1;
+    Set open;
     std::vector<uint32_t> splits;  // of the least flops: the larger part
     std::vector<Cand> cands;
+    int reached = 0;  // by the limit numbered so
   };
   std::vector<State> st(size_t(1) << n);
   for (uint32_t S = 1; S <= full; ++S) {
     State& s = st[S];
-    for (const Label& l : lab)
-      if (open_in(l, S)) s.size *= l.dim;
+    for (size_t l = 0; l < lab.size(); ++l)
+      if ((lab[l].where & S) && ((lab[l].where & ~S & full) || lab[l].out)) s.open.w[l / 64] |= uint64_t(1) << (l % 64);
+    s.size = extent(s.open, s.open);
     if ((S & (S - 1)) == 0) continue;
     s.flops = INFINITY;
     for (uint32_t S1 = (S - 1) & S; S1 > 0; S1 = (S1 - 1) & S) {
       const uint32_t S2 = S & ~S1;
-      if (S1 < S2) continue;
+      if (S1 < S2) break;  // (descending: the rest are the mirrored splits)
       // multiply-adds of the step: the labels open in either part
-      double f = 1;
-      for (const Label& l : lab)
-        if (open_in(l, S1) || open_in(l, S2)) f *= l.dim;
-      f += st[S1].flops + st[S2].flops;
+      const double f = extent(st[S1].open, st[S2].open) + st[S1].flops + st[S2].flops;
       if (f > s.flops * (1 + 1e-9)) continue;
       if (f < s.flops * (1 - 1e-9)) {
         s.flops = f;
@@ -251,20 +289,35 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
       s.splits.push_back(S1);
     }
   }
-  const Labs result(out_labels);
+  auto single = [](uint32_t S) { return (S & (S - 1)) == 0; };
+  // pair plans that a limit takes at most, over the subsets below S not yet counted
+  std::function<double(uint32_t, SearchLimit, int)> pairs = [&](uint32_t S, SearchLimit lim, int mark) -> double {
+    if (single(S) || st[S].reached == mark) return 0.0;
+    st[S].reached = mark;
+    double c = 0;
+    for (int k = 0; k < std::min(lim.splits, int(st[S].splits.size())); ++k) {
+      const uint32_t S1 = st[S].splits[k], S2 = S & ~S1;
+      c += 2.0 * (single(S1) ? 1 : lim.orders) * (single(S2) ? 1 : lim.orders);
+      c += pairs(S1, lim, mark) + pairs(S2, lim, mark);
+    }
+    return c;
+  };
+  SearchLimit lim = kSearch[0];
+  for (int k = 0; k < int(std::size(kSearch)); ++k) {
+    lim = kSearch[k];
+    if (pairs(full, lim, k + 1) <= std::max(200.0, std::min(std::pow(3.0, n) / 4, 2e4))) break;
+  }
   std::function<void(uint32_t)> plan = [&](uint32_t S) {
     State& s = st[S];
     if (!s.cands.empty()) return;
-    if ((S & (S - 1)) == 0) {
-      int i = 0;
-      while (!((S >> i) & 1)) ++i;
+    if (single(S)) {
       Cand leaf;
-      leaf.order = Labs(labs[i]);
+      leaf.order = of[__builtin_ctz(S)];
       s.cands.push_back(leaf);
       return;
     }
-    for (uint32_t S1 : s.splits) {
-      const uint32_t S2 = S & ~S1;
+    for (int k = 0; k < std::min(lim.splits, int(s.splits.size())); ++k) {
+      const uint32_t S1 = s.splits[k], S2 = S & ~S1;
       plan(S1);
       plan(S2);
       for (int i = 0; i < int(st[S1].cands.size()); ++i)
@@ -274,13 +327,13 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
             const Cand &ca = st[A].cands[swap ? j : i], &cb = st[B].cands[swap ? i : j];
             Cand q;
             q.moved = ca.moved + cb.moved;
-            const PairPlan p = plan_pair(ca.order, st[A].size, cb.order, st[B].size, [&](int l) { return dims.at(l); });
+            const auto p = plan_pair(ca.order, st[A].size, cb.order, st[B].size, dim);
             if (p.perm_a) q.moved += st[A].size + kPermLaunch;
             if (p.perm_b) q.moved += st[B].size + kPermLaunch;
             q.order = p.out;
             if (S == full && p.out != result) {
               // (a plain product in the swapped order is formed transposed)
-              Labs t;
+              L t;
               t.append(p.b, 0, p.lb.s);
               t.append(p.b, p.lb.s + p.K.n, p.b.n);
               t.append(p.a, 0, p.la.s);
@@ -301,7 +354,7 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     }
     std::stable_sort(s.cands.begin(), s.cands.end(), [](const Cand& x, const Cand& y) { return x.moved < y.moved; });
     const double most = s.cands[0].moved + s.size + kPermLaunch;
-    while (s.cands.size() > kOrders || s.cands.back().moved >= most) s.cands.pop_back();
+    while (s.cands.size() > size_t(lim.orders) || s.cands.back().moved >= most) s.cands.pop_back();
   };
   plan(full);
   Tree T;
@@ -309,12 +362,10 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     const Cand& q = st[S].cands[k];
     Node nd;
     nd.mask = S;
-    nd.order = q.order;
+    for (uint8_t l : q.order) nd.order.push_back(lab[l].name);
     nd.size = st[S].size;
-    if ((S & (S - 1)) == 0) {
-      int i = 0;
-      while (!((S >> i) & 1)) ++i;
-      nd.leaf = i;
+    if (single(S)) {
+      nd.leaf = __builtin_ctz(S);
     } else {
       nd.left = build(q.left, q.ci);
       nd.right = build(q.right, q.cj);
@@ -324,6 +375,7 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     T.nodes.push_back(nd);
     return int(T.nodes.size()) - 1;
   };
+  T.moved = st[full].cands[0].moved;
   T.root = build(full, 0);
   return T;
 }
