@@ -187,7 +187,8 @@ struct Tree {
   double moved = 0;        // what its permutations cost
 };
 
-// Exact flop-optimal pairwise order (dynamic programming over subsets).  Trees of equal
+// Exact flop-optimal pairwise order (dynamic programming over subsets) among those whose
+// intermediates have no more labels than a tensor holds.  Trees of equal
 // flops are common (both ends of a chain's H_eff, either operand of a step first), and
 // differ in the permutations that contract_pair needs: among them one that moves little
 // data is taken, a permutation counting as its elements plus kPermLaunch for the launch.
@@ -276,12 +277,15 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     s.size = extent(s.open, s.open);
     if ((S & (S - 1)) == 0) continue;
     s.flops = INFINITY;
+    int rank = 0;
+    for (int k = 0; k < words; ++k) rank += __builtin_popcountll(s.open.w[k]);
+    if (rank > NSG_MAX_RANK) continue;
     for (uint32_t S1 = (S - 1) & S; S1 > 0; S1 = (S1 - 1) & S) {
       const uint32_t S2 = S & ~S1;
       if (S1 < S2) break;  // (descending: the rest are the mirrored splits)
       // multiply-adds of the step: the labels open in either part
       const double f = extent(st[S1].open, st[S2].open) + st[S1].flops + st[S2].flops;
-      if (f > s.flops * (1 + 1e-9)) continue;
+      if (f == INFINITY || f > s.flops * (1 + 1e-9)) continue;
       if (f < s.flops * (1 - 1e-9)) {
         s.flops = f;
         s.splits.clear();
@@ -289,6 +293,7 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
       s.splits.push_back(S1);
     }
   }
+  NSG_CHECK(st[full].flops < INFINITY, NSG_ERR_UNSUPPORTED, "contract: result rank above 16");
   auto single = [](uint32_t S) { return (S & (S - 1)) == 0; };
   // pair plans that a limit takes at most, over the subsets below S not yet counted
   std::function<double(uint32_t, SearchLimit, int)> pairs = [&](uint32_t S, SearchLimit lim, int mark) -> double {

@@ -134,3 +134,18 @@ def test_ties_do_not_blow_the_planning_up(plan):
     for net, got in zip(nets, plan(nets)):
         assert got[0] == len(net[0]) - 1 or 4 in net[2].values()
         assert got[2] < 0.15
+
+
+def test_intermediates_fit_a_tensors_rank(plan):
+    # trees of equal flops, some of them through an intermediate of more than 16 labels
+    labs = [[9, 8, 5, 3, 1, 6, 0, 7, 2, 4],
+            [0, 15, 16, 18, 12, 25, 17, 14, 1, 13, 10, 11],
+            [21, 10, 2, 22, 3, 19, 20, 11, 26],
+            [13, 19, 4, 27, 24, 23, 12, 20],
+            [16, 5, 24, 7, 15, 6, 14, 23],
+            [21, 8, 18, 22, 17, 9]]
+    two = [2, 5, 6, 7, 8, 9, 10, 12, 17, 19]
+    net = labs, [25, 26, 27], {l: 2 if l in two else 1 for t in labs for l in t}
+    got, wide = plan([net, ([[*range(10)], [*range(10, 20)]], [*range(20)], dict.fromkeys(range(20), 1))])
+    assert got[3] <= 16 and got[0] == least_macs(net)
+    assert wide == "error 7"
