@@ -335,7 +335,7 @@ int nsg_contract(nsg_ctx* c, int n, nsg_tensor* const* tensors, const int32_t* l
     m.fixed.assign(tensors, tensors + n - 1);
     m.labs = labs;
     for (int i = 0; i < n; ++i) m.conj.push_back(conj ? conj[i] : 0);
-    m.tree = optimal_tree(labs, outl, dims);
+    m.tree = optimal_tree(labs, outl, dims, c->precision, dtype);
     LT x;
     x.t = tensors[n - 1];
     x.lab = labs[n - 1];
@@ -392,7 +392,7 @@ int nsg_linmap_create(nsg_ctx* c, int n_fixed, nsg_tensor* const* fixed, const i
     dims[xl] = d;
     if (!dims.count(yl)) dims[yl] = d;
   }
-  m->tree = optimal_tree(m->labs, m->y_labels, dims);
+  m->tree = optimal_tree(m->labs, m->y_labels, dims, c->precision, m->dtype);
   m->flops = m->tree.total_macs * (m->dtype == NSG_C128 ? 8.0 : 2.0);
   // precompute fixed-only subtrees (largest ones only: a node whose parent contains x)
   uint32_t xbit = 1u << n_fixed;

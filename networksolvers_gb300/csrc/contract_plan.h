@@ -82,6 +82,18 @@ struct PairPlan {
   bool perm_a = false, perm_b = false;
   bool batched_a() const { return la.contiguous && la.s > 0 && la.s + K.n < a.n; }
   bool batched_b() const { return lb.contiguous && lb.s > 0 && lb.s + K.n < b.n; }
+  // rows and columns of the product, of each batch entry
+  template <typename Dim>
+  void free_sizes(Dim dim, double* M, double* N) const {
+    auto extent = [&](const Labs<V>& x, const Layout<V>& L, bool one) {  // one: the batched operand's first group
+      double e = 1;
+      for (int q = 0; q < x.n; ++q)
+        if (q < L.s || (q >= L.s + K.n && !one)) e *= double(dim(x.v[q]));
+      return e;
+    };
+    *M = extent(a, la, batched_a());
+    *N = extent(b, lb, batched_b());
+  }
 };
 
 template <typename V, typename Dim>  // dim(label): its extent
@@ -185,31 +197,42 @@ struct Tree {
   int root = -1;
   double total_macs = 0;
   double moved = 0;        // what its permutations cost
+  double fp64_macs = 0;    // MACs of the products below the tensor-core form's sizes
 };
 
 // Exact flop-optimal pairwise order (dynamic programming over subsets) among those whose
-// intermediates have no more labels than a tensor holds.  Trees of equal
-// flops are common (both ends of a chain's H_eff, either operand of a step first), and
-// differ in the permutations that contract_pair needs: among them one that moves little
-// data is taken, a permutation counting as its elements plus kPermLaunch for the launch.
-// For that a subset keeps, of its flop-optimal trees, the cheapest per order of its result
-// (none that a permutation of the cheapest would beat).  (Taking the first tree cost a
-// permutation of the 168 MB intermediate per application at bond dimension 1024: 0.6 of
-// 3.5 ms.)
+// intermediates have no more labels than a tensor holds.  Trees of equal flops are common
+// (both ends of a chain's H_eff, either operand of a step first), and differ in the
+// permutations that contract_pair needs and, in the split precisions, in the products that
+// miss the tensor-core form's least sizes.  Among them one of little predicted time is taken,
+// in units of an element's permutation (16 bytes of HBM traffic, 2.4 ps; twice both for
+// complex data): a permutation costs its elements plus kPermLaunch, a multiply-add 0.7 on the
+// FP64 cores (two per clock and SM) and 0.02 as a split product (4096 x 1024 x 1024 in 0.17
+// ms), twice those for complex data, whose elements take two and whose multiply-adds four
+// times as long; a split product costs kSplitLaunch beyond that (an eigensolve with bonds 40 and
+// 100 takes 376 us with the 3.2 million multiply-adds of one product of its H_eff on the FP64
+// cores and 400 with them split; 63 and 100, 7.9 million: 426 and 415).  For that a subset
+// keeps, of its flop-optimal trees, the cheapest per order of its result (none that a
+// permutation of the cheapest would beat).  Taking the first tree cost a permutation of the
+// 168 MB intermediate per application at bond dimension 1024, 0.6 of 3.5 ms; counting
+// permutations alone left 25 % of the multiply-adds of an H_eff with bonds 60 and 240 to the
+// FP64 cores and 45 % with bonds 63 and 100, where 6 % and 11 % need be (eigensolves with bonds
+// 60 and 240: 543 us and 482; 60 and 1000: 551 and 470).
 //
 // Where bonds are equal, or 1 as in a product state, almost every tree ties.  The search is
 // cut to a number of pair plans that takes no longer than the dynamic programming itself:
 // fewer splits per subset, and fewer orders, the more trees tie.  Planning times, host of the
 // GPU machine's class: H_eff of a chain 8 us, environment at a vertex of degree 6 0.3 ms, twelve
 // tensors with bonds 1 7 ms; without the limit 13 us, 3.7 ms, 6 s as a chain and 56 s as a star.
-constexpr double kPermLaunch = 2e4;
+constexpr double kPermLaunch = 2e4, kSplitLaunch = 4e6;
 struct SearchLimit {
   int splits, orders;
 };
 constexpr SearchLimit kSearch[] = {{1 << 12, 6}, {4, 6}, {3, 3}, {2, 2}, {1, 1}};
 
 inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::vector<int>& out_labels,
-                         const std::unordered_map<int, int64_t>& dims) {
+                         const std::unordered_map<int, int64_t>& dims, int precision = NSG_PREC_FP64,
+                         int dtype = NSG_F64) {
   using L = Labs<uint8_t>;
   const int n = int(labs.size());
   NSG_CHECK(n >= 1 && n <= 12, NSG_ERR_UNSUPPORTED, "contract: 1..12 tensors");
@@ -257,7 +280,7 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     return e;
   };
   struct Cand {
-    double moved = 0;
+    double cost = 0, moved = 0, fp64 = 0;
     L order;
     uint32_t left = 0, right = 0;
     int ci = 0, cj = 0;  // the parts' candidates
@@ -307,6 +330,8 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     }
     return c;
   };
+  if (precision == NSG_PREC_TF32X3 && dtype == NSG_C128) precision = NSG_PREC_FP64;  // (real data only)
+  const double mac_scale = dtype == NSG_C128 ? 2.0 : 1.0;
   SearchLimit lim = kSearch[0];
   for (int k = 0; k < int(std::size(kSearch)); ++k) {
     lim = kSearch[k];
@@ -331,11 +356,12 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
             const uint32_t A = swap ? S2 : S1, B = swap ? S1 : S2;
             const Cand &ca = st[A].cands[swap ? j : i], &cb = st[B].cands[swap ? i : j];
             Cand q;
-            q.moved = ca.moved + cb.moved;
             const auto p = plan_pair(ca.order, st[A].size, cb.order, st[B].size, dim);
-            if (p.perm_a) q.moved += st[A].size + kPermLaunch;
-            if (p.perm_b) q.moved += st[B].size + kPermLaunch;
+            double moved = 0;
+            if (p.perm_a) moved += st[A].size + kPermLaunch;
+            if (p.perm_b) moved += st[B].size + kPermLaunch;
             q.order = p.out;
+            bool transposed = false;
             if (S == full && p.out != result) {
               // (a plain product in the swapped order is formed transposed)
               L t;
@@ -343,9 +369,25 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
               t.append(p.b, p.lb.s + p.K.n, p.b.n);
               t.append(p.a, 0, p.la.s);
               t.append(p.a, p.la.s + p.K.n, p.a.n);
-              if (p.batched_a() || p.batched_b() || t != result) q.moved += s.size + kPermLaunch;
+              transposed = !p.batched_a() && !p.batched_b() && t == result;
+              if (!transposed) moved += s.size + kPermLaunch;
               q.order = result;
             }
+            double time = 0, slow = 0;
+            if (precision != NSG_PREC_FP64) {
+              const double macs = s.flops - st[A].flops - st[B].flops;
+              double M, N, K = 1;
+              p.free_sizes(dim, &M, &N);
+              for (uint8_t l : p.K) K *= dim(l);
+              if (transposed) std::swap(M, N);
+              if (tensor_core_sizes(precision, M, N, K))
+                time = kSplitLaunch + 0.02 * mac_scale * macs;
+              else
+                time = 0.7 * mac_scale * (slow = macs);
+            }
+            q.cost = ca.cost + cb.cost + moved + time;
+            q.moved = ca.moved + cb.moved + moved;
+            q.fp64 = ca.fp64 + cb.fp64 + slow;
             q.left = A;
             q.right = B;
             q.ci = swap ? j : i;
@@ -353,13 +395,13 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
             auto same = std::find_if(s.cands.begin(), s.cands.end(), [&](const Cand& x) { return x.order == q.order; });
             if (same == s.cands.end())
               s.cands.push_back(q);
-            else if (q.moved < same->moved)
+            else if (q.cost < same->cost)
               *same = q;
           }
     }
-    std::stable_sort(s.cands.begin(), s.cands.end(), [](const Cand& x, const Cand& y) { return x.moved < y.moved; });
-    const double most = s.cands[0].moved + s.size + kPermLaunch;
-    while (s.cands.size() > size_t(lim.orders) || s.cands.back().moved >= most) s.cands.pop_back();
+    std::stable_sort(s.cands.begin(), s.cands.end(), [](const Cand& x, const Cand& y) { return x.cost < y.cost; });
+    const double most = s.cands[0].cost + s.size + kPermLaunch;
+    while (s.cands.size() > size_t(lim.orders) || s.cands.back().cost >= most) s.cands.pop_back();
   };
   plan(full);
   Tree T;
@@ -381,6 +423,7 @@ inline Tree optimal_tree(const std::vector<std::vector<int>>& labs, const std::v
     return int(T.nodes.size()) - 1;
   };
   T.moved = st[full].cands[0].moved;
+  T.fp64_macs = st[full].cands[0].fp64;
   T.root = build(full, 0);
   return T;
 }

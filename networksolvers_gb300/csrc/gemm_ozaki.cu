@@ -844,7 +844,7 @@ void oz_products(nsg_ctx* c, const OzOperand* const* A, const OzOperand* const* 
 template <int S>
 bool gemm_ozaki_impl(nsg_ctx* c, const GemmArgs& g) {
   if (g.dtype != NSG_F64 && g.dtype != NSG_C128) return false;
-  if (g.M < 64 || g.N < 32 || g.K < 64) return false;
+  if (!tensor_core_sizes(NSG_PREC_OZAKI, double(g.M), double(g.N), double(g.K))) return false;
   if (g.batch > 65535) return false;
   const bool cplx = g.dtype == NSG_C128;
   if (!cplx && (g.opA == OP_C || g.opA == OP_R || g.opB == OP_C || g.opB == OP_R)) return false;

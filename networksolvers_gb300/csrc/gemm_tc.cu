@@ -369,7 +369,7 @@ bool gemm_split_tc(nsg_ctx* c, const GemmArgs& g) {
   if (g.dtype != NSG_F64) return false;
   if (g.opA == OP_C || g.opA == OP_R || g.opB == OP_C || g.opB == OP_R) return false;
   // small products stay on the FP64 path (tensor cores need full 128-row tiles to pay off)
-  if (g.M < 64 || g.N < 64 || g.K < 32) return false;
+  if (!tensor_core_sizes(NSG_PREC_TF32X3, double(g.M), double(g.N), double(g.K))) return false;
   if (g.batch > 65535) return false;
   const int64_t Mp = (g.M + TM - 1) / TM * TM, Np = (g.N + BN - 1) / BN * BN, Kp = (g.K + BK - 1) / BK * BK;
   // A(r, k): op N -> A[r + k*lda]; op T -> A[k + r*lda]

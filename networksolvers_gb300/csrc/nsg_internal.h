@@ -184,6 +184,13 @@ struct GemmArgs {
   int64_t batch;
   double alpha_re = 1.0, alpha_im = 0.0, beta_re = 0.0, beta_im = 0.0;
 };
+// The least sizes of a precision mode's tensor-core form (64 x 32 x 64 for the split into BF16
+// slices, 64 x 64 x 32 for TF32x3): below them padding to the form's tiles costs more than the
+// FP64 cores take.  The forms test them, and the contraction planner counts by them.
+inline bool tensor_core_sizes(int precision, double M, double N, double K) {
+  if (precision == NSG_PREC_TF32X3) return M >= 64 && N >= 64 && K >= 32;
+  return precision != NSG_PREC_FP64 && M >= 64 && N >= 32 && K >= 64;
+}
 // dispatches by the context's precision mode and shape
 void gemm(nsg_ctx* c, const GemmArgs& g);
 void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g);

@@ -8,6 +8,7 @@ from pathlib import Path
 import pytest
 
 from networksolvers_gb300 import build as nb
+from networksolvers_gb300._native import PRECISIONS
 
 MAIN = r"""
 #include "contract_plan.h"
@@ -25,8 +26,8 @@ int main() {
       for (int& x : v) std::cin >> x;
       return v;
     };
-    int n;
-    std::cin >> n;
+    int n, precision;
+    std::cin >> n >> precision;
     std::vector<std::vector<int>> labs(n);
     for (auto& l : labs) l = list();
     const std::vector<int> out = list(), names = list(), sizes = list();
@@ -37,7 +38,7 @@ int main() {
     try {
       for (int rep = 0; rep < 2; ++rep) {
         const auto t0 = std::chrono::steady_clock::now();
-        t = nsg::optimal_tree(labs, out, dims);
+        t = nsg::optimal_tree(labs, out, dims, precision);
         best = std::min(best, std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count());
       }
     } catch (const nsg::Error& e) {
@@ -46,7 +47,7 @@ int main() {
     }
     int rank = 0;
     for (const auto& nd : t.nodes) rank = std::max(rank, nd.order.n);
-    printf("%.17g %.17g %g %d\n", t.total_macs, t.moved, best, rank);
+    printf("%.17g %.17g %g %d %.17g\n", t.total_macs, t.moved, best, rank, t.fp64_macs);
   }
 }
 """
@@ -60,10 +61,10 @@ def plan(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O2", "-w", f"-I{nb.CSRC}", f"-I{cuda}", str(d / "main.cpp"), "-o",
                     str(d / "main")], check=True)
 
-    def run(nets):
+    def run(nets, precision=PRECISIONS["fp64"]):
         words = [len(nets)]
         for labs, out, dims in nets:
-            words.append(len(labs))
+            words += [len(labs), precision]
             for x in (*labs, out, list(dims), list(dims.values())):
                 words += [len(x), *x]
         r = subprocess.run([str(d / "main")], input=" ".join(map(str, words)), capture_output=True, text=True,
@@ -149,3 +150,11 @@ def test_intermediates_fit_a_tensors_rank(plan):
     got, wide = plan([net, ([[*range(10)], [*range(10, 20)]], [*range(20)], dict.fromkeys(range(20), 1))])
     assert got[3] <= 16 and got[0] == least_macs(net)
     assert wide == "error 7"
+
+
+def test_ties_keep_products_on_the_tensor_cores(plan):
+    """H_eff applications in the split precision: in one of the mirrored orders all but the two
+    operator tensors' products (5 x 2 x 5 x 2 of each of 2 a b entries) meet its least sizes."""
+    shapes = [(60, 240), (63, 100), (60, 1000), (100, 63), (240, 60), (128, 128)]
+    for (a, b), got in zip(shapes, plan([heff(a, b) for a, b in shapes], PRECISIONS["ozaki"])):
+        assert got[4] == 2 * 100 * 2 * a * b, (a, b)
