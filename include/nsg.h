@@ -136,10 +136,13 @@ int nsg_ctx_wait_probe(nsg_ctx* ctx, int64_t polls);
  * (-1 all SMs, 2/4/8/16 one thread-block cluster of that size where the matrix fits it, 0
  * the table); NSG_TUNE_DC_LEAF: the divide and conquer's leaf order (4..32; 0 the default 8:
  * larger leaves mean fewer merge levels, so fewer launches per eigensolve above order 128, at
- * a longer leaf solve). */
+ * a longer leaf solve); NSG_TUNE_LANCZOS_POLLS: polls after which a wait inside the Krylov
+ * solvers' launches gives up (1..2^24; 0 the default 2^22; -1 without a poll, for checks of the
+ * giving-up: the solver then repeats its cycle with kernels that wait for nothing). */
 #define NSG_TUNE_SPLITK 0
 #define NSG_TUNE_TRIDIAG 1
 #define NSG_TUNE_DC_LEAF 2
+#define NSG_TUNE_LANCZOS_POLLS 3
 int nsg_ctx_set_tuning(nsg_ctx* ctx, int param, int value);
 
 /* ---- tensors ------------------------------------------------------------- */

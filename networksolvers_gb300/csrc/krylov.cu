@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstring>
 
 namespace nsg {
 void linmap_apply(nsg_ctx* c, nsg_linmap* m, const nsg_tensor* x, nsg_tensor* y);
@@ -165,8 +166,14 @@ void lanczos_step(nsg_ctx* c, nsg_linmap* m, std::vector<nsg_tensor*>& V, int j,
 // synchronisation; the host reads every scalar back once.  A step's vector work is one launch
 // (lanczos.cu), in the operations of lanczos_step; beyond the vectors that launch takes, the
 // kernels of lanczos_step.  All K steps run; steps after a breakdown are discarded by the
-// caller.
+// caller, and all of them when a wait of those launches gave up (the status word behind the
+// scalars, read with them): the cycle is then taken step by step.
 static size_t step_offset(int j) { return size_t(2) * j * (j + 1) + size_t(2) * j; }  // sum_{i<j} (4 (i+1) + 2)
+bool gave_up(const std::vector<double>& scalars) {  // the status word, last
+  int s;
+  std::memcpy(&s, &scalars.back(), sizeof(s));
+  return s != 0;
+}
 void lanczos_cycle_dev(nsg_ctx* c, nsg_linmap* m, LanczosVectors& lv, std::vector<nsg_tensor*>& V, int K, nsg_tensor* w,
                        double* scal) {
   const int dt = w->dtype;
@@ -218,18 +225,19 @@ int nsg_eigsolve(nsg_ctx* c, nsg_linmap* m, nsg_tensor* x, int krylovdim, int ma
     // host read.  Falls through to the synchronous form below when the start vector's or
     // a kept step's sum of squares leaves the range where sqrt(sum) is exact enough
     // (the synchronous norm rescales there) -- the same arithmetic otherwise.
-    const size_t nscal = step_offset(krylovdim) + 2;
+    const size_t nscal = step_offset(krylovdim) + 3;
     ScopedBuf sb(c, sizeof(double) * nscal);
     double* scal = (double*)sb.p;
     double* sx = scal + step_offset(krylovdim);
-    LanczosVectors lv(c, dt, n);
+    NSG_CUDA(cudaMemsetAsync(sx + 2, 0, sizeof(double), c->stream));
+    LanczosVectors lv(c, dt, n, (int*)(sx + 2));
     lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, V[0]->data);
     lanczos_cycle_dev(c, m, lv, V, krylovdim, w, scal);
     std::vector<double> hs(nscal);
     NSG_CUDA(cudaMemcpyAsync(hs.data(), scal, sizeof(double) * nscal, cudaMemcpyDeviceToHost, c->stream));
     NSG_CUDA(cudaStreamSynchronize(c->stream));
     auto in_range = [](double q) { return std::isfinite(q) && q > 1e-280 && q < 1e280; };
-    bool ok = in_range(hs[step_offset(krylovdim)]);
+    bool ok = in_range(hs[step_offset(krylovdim)]) && !gave_up(hs);
     std::vector<double> alpha, beta;
     int k = 0;
     for (int j = 0; j < krylovdim && ok; ++j) {
@@ -258,7 +266,10 @@ int nsg_eigsolve(nsg_ctx* c, nsg_linmap* m, nsg_tensor* x, int krylovdim, int ma
       for (int j = 0; j < k; ++j) ptrs[j] = V[j]->data;
       NSG_CUDA(cudaMemsetAsync(x->data, 0, x->bytes, c->stream));
       multi_axpy(c, dt, n, k, ptrs.data(), coef.data(), x->data);
-      lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, x->data);
+      // (by kernels that wait for nothing: the host does not read anything after them)
+      const void* xq[1] = {x->data};
+      multi_dot_dev(c, dt, n, 1, xq, x->data, sx);
+      axpby_devscalar(c, dt, n, sx, 0, x->data, x->data);
       *eigval = lam;
       if (numops) *numops = ops;
       check_device_flag(c);
@@ -339,22 +350,23 @@ int nsg_exponentiate(nsg_ctx* c, nsg_linmap* m, double t_re, double t_im, nsg_te
     };
     // Speculative device-resident cycle: the number of steps the previous cycle needed
     // (plus one) runs without host synchronisation, then the host replays the stopping
-    // rule on the read-back scalars.  The vectors are those of the step-by-step form
-    // (same kernels and arithmetic), so a rule that stops within the speculated steps
-    // gives the identical result; a rule that has not stopped continues step by step from
-    // there, and a sum of squares outside the range of an exact square root restarts the
-    // cycle step by step.
+    // rule on the read-back scalars.  The vectors are those of the step-by-step form up to
+    // the rounding of its sums (which other kernels add in another order); a rule that has
+    // not stopped continues step by step from there, and a sum of squares outside the range
+    // of an exact square root, or a launch whose wait gave up, restarts the cycle step by
+    // step.
     double beta0 = 0.0;
     const int spec = std::min(krylovdim, std::max(2, c->krylov_hint + 1));
     const int ops_before = ops;
     bool spec_ok = false;  // the stopping rule fired within the speculated steps
     int resume = 0;        // > 0: steps 0..resume-1 are valid, continue from step `resume`
     {
-      const size_t nscal = step_offset(spec) + 2;
+      const size_t nscal = step_offset(spec) + 3;
       ScopedBuf sb(c, sizeof(double) * nscal);
       double* scal = (double*)sb.p;
       double* sx = scal + step_offset(spec);
-      LanczosVectors lv(c, dt, n);
+      NSG_CUDA(cudaMemsetAsync(sx + 2, 0, sizeof(double), c->stream));
+      LanczosVectors lv(c, dt, n, (int*)(sx + 2));
       lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, V[0]->data);
       lanczos_cycle_dev(c, m, lv, V, spec, w, scal);
       std::vector<double> hs(nscal);
@@ -362,8 +374,8 @@ int nsg_exponentiate(nsg_ctx* c, nsg_linmap* m, double t_re, double t_im, nsg_te
       NSG_CUDA(cudaStreamSynchronize(c->stream));
       auto in_range = [](double q) { return std::isfinite(q) && q > 1e-280 && q < 1e280; };
       const double qx = hs[step_offset(spec)];
-      if (qx == 0.0) break;
-      if (in_range(qx)) {
+      if (!gave_up(hs) && qx == 0.0) break;
+      if (!gave_up(hs) && in_range(qx)) {
         beta0 = std::sqrt(qx);
         for (int j = 0; j < spec; ++j) {
           const double* blk = hs.data() + step_offset(j);

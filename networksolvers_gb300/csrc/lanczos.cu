@@ -36,7 +36,8 @@ struct Step {
   double *co1, *co2, *ss;  // coefficients; the sum of squares and its root
   ulonglong2* msg;     // 3 sums x CTAs x kVals
   unsigned long long tag;
-  int* err;
+  int polls;           // of a wait before it gives up; below 0 it does so at once
+  int* gave_up;
 };
 
 __device__ __forceinline__ double fnma(double a, double v, double w) { return fma(-a, v, w); }
@@ -100,12 +101,13 @@ __device__ void all_sums(const Step& s, int area, int nvals, const double (*part
       double t = 0.0;
       for (int b = lane; b < G; b += 32) {
         double x = 0.0;
-        for (int polls = 0; !get_tagged(msg + (size_t)q * G + b, s.tag + area, x);)
-          if (++polls > (1 << 22)) {  // the host sees that the scalars are not finite
-            atomicExch(s.err, 1);
-            x = __longlong_as_double(0x7ff8000000000000ll);
-            break;
-          }
+        int polls = s.polls;
+        bool there = false;
+        while (polls-- > 0 && !there) there = get_tagged(msg + (size_t)q * G + b, s.tag + area, x);
+        if (!there) {
+          atomicExch(s.gave_up, 1);
+          x = __longlong_as_double(0x7ff8000000000000ll);
+        }
         t += x;
       }
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -280,7 +282,8 @@ const void* step_kernel(int nv) {
 
 }  // namespace
 
-LanczosVectors::LanczosVectors(nsg_ctx* ctx, int dt, int64_t len) : c(ctx), dtype(dt), n(len) {
+LanczosVectors::LanczosVectors(nsg_ctx* ctx, int dt, int64_t len, int* gave_up_flag)
+    : c(ctx), dtype(dt), n(len), gave_up(gave_up_flag) {
   // every CTA gathers every CTA's sums, so no more CTAs than pay: a CTA has at least 512
   // elements (2048 instead: TDVP step at bond dimension 128 7 % slower), one CTA per SM, and two
   // from 2^21 elements on, where the loads in flight count (eigensolve at bond dimension 1024,
@@ -316,11 +319,8 @@ bool LanczosVectors::step(int nv, const void* const* v, void* w, const double* p
   s.msg = (ulonglong2*)msg;
   s.tag = tag;
   tag += 4;
-  // a wait that gives up leaves scalars that are not finite, which the host reads anyway: no
-  // check (and no synchronisation) at the end of the call for its sake
-  const bool pending = c->flag_pending;
-  s.err = device_flag(c);
-  c->flag_pending = pending;
+  s.polls = c->tune_lanczos_polls != 0 ? c->tune_lanczos_polls : 1 << 22;
+  s.gave_up = gave_up;
   const void* fn = dtype == NSG_C128 ? step_kernel<double2>(nv) : step_kernel<double>(nv);
   void* args[] = {&s};
   NSG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kT), args, 0, c->stream));

@@ -61,6 +61,7 @@ struct nsg_ctx {
   int tune_splitk = 0;  // FP64 GEMM K slices of the 64 x 64 tiles (> 0 forces both)
   int tune_tri = 0;     // tridiagonalisation: -1 grid kernel, 2..16 cluster size
   int tune_dc_leaf = 0; // divide and conquer leaf order (4..32; 0 the default)
+  int tune_lanczos_polls = 0;  // polls of a Lanczos launch's waits (-1 none; 0 the default)
   // pinned host staging for scalar readback
   double* host_scalars = nullptr;
   size_t host_scalars_cap = 0;
@@ -219,6 +220,8 @@ double norm2(nsg_ctx* c, int dtype, int64_t n, const void* x);
 // (prev: the step before's ss; null: nothing), two Gram-Schmidt passes against v[0..nv) whose coefficients
 // (2 doubles each) go to co1 and co2, ss = {|w|^2, |w|}, next = w / |w| (unless null).  nv = 0:
 // w is only read.  Returns false, with nothing launched, for more vectors than it takes.
+// A wait that gives up sets *gave_up (which the caller zeroes before and reads with the
+// scalars); the vectors and scalars are then not to be used.
 struct LanczosVectors {
   nsg_ctx* c;
   int dtype;
@@ -227,7 +230,8 @@ struct LanczosVectors {
   void* msg = nullptr;
   size_t bytes = 0;
   uint64_t tag = 1;
-  LanczosVectors(nsg_ctx* ctx, int dt, int64_t len);
+  int* gave_up;
+  LanczosVectors(nsg_ctx* ctx, int dt, int64_t len, int* gave_up_flag);
   ~LanczosVectors();
   LanczosVectors(const LanczosVectors&) = delete;
   LanczosVectors& operator=(const LanczosVectors&) = delete;

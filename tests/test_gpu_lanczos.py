@@ -8,7 +8,7 @@ import pytest
 
 from networksolvers_gb300._native import NsgError
 from networksolvers_gb300.itensors import DTensor
-from networksolvers_gb300.sweep import eigsolve_solver
+from networksolvers_gb300.sweep import eigsolve_solver, exponentiate_solver
 from oracle import krylov as ok
 from test_gpu_kernels import _chain_heff, _device_map
 
@@ -70,3 +70,34 @@ def test_extreme_norms(nsg_ctx, scale):
     lam, _ = eigsolve_solver(lm, DTensor.from_numpy(scale * x0, inds), krylovdim=3, maxiter=1)
     ref, _ = ok.eigsolve_lanczos(heff(*H), x0, krylovdim=3, maxiter=1)
     assert abs(lam - ref) <= 1e-12 * abs(ref)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "ozaki"])
+def test_waits_that_give_up(nsg_ctx, precision):
+    """The cycle is repeated step by step, and nothing of it is reported by a later call."""
+    rng = np.random.default_rng(3)
+    lm, inds = _device_map(*_chain_heff(rng, 64, 80))
+    x0 = DTensor.from_numpy(rng.standard_normal((64, 2, 2, 80)), inds)
+
+    def solve():
+        before = nsg_ctx.counters()["launches"]
+        lam, x = eigsolve_solver(lm, x0, krylovdim=3, maxiter=1)
+        y, info = exponentiate_solver(lm, -0.5 / abs(lam), x0, tol=1e-12)
+        assert info["converged"]
+        return lam, x.to_numpy(), y.to_numpy(), nsg_ctx.counters()["launches"] - before
+
+    nsg_ctx.set_precision(precision)
+    try:
+        solve()  # (the exponential's next cycle starts from what the last one needed)
+        lam, x, y, launches = solve()
+        nsg_ctx.set_tuning("lanczos_polls", -1)
+        lam_g, x_g, y_g, launches_g = solve()
+        nsg_ctx.set_tuning("lanczos_polls", 0)
+        assert launches_g > launches
+        assert abs(lam_g - lam) <= 1e-10 * abs(lam)
+        assert np.linalg.norm(x_g - x) < 1e-8 and np.linalg.norm(y_g - y) < 1e-8 * np.linalg.norm(y)
+        assert abs(np.linalg.norm(x_g) - 1) < 1e-13
+        assert solve()[3] == launches
+    finally:
+        nsg_ctx.set_tuning("lanczos_polls", 0)
+        nsg_ctx.set_precision("fp64")
