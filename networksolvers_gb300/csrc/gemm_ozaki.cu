@@ -280,36 +280,42 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_shallow_kernel(const _
   slice_slab<S>(op, b, r0, k0, len, P.K_p, tile, rowexp);
 }
 
-// blockIdx.x = 32-row tile (over the batch), blockIdx.y = slab of kMaxSlab
-__global__ void __launch_bounds__(kSliceThreads) oz_row_max_kernel(const __grid_constant__ OzSource op, int64_t K) {
+// blockIdx.x = 32-row tile (over the batch), blockIdx.y = first of the slabs of kMaxSlab it
+// takes (one, but for depths that exceed a grid's 65535)
+__global__ void __launch_bounds__(kSliceThreads)
+    oz_row_max_kernel(const __grid_constant__ OzSource op, int64_t K, int slabs) {
   __shared__ unsigned rowmax[kSliceRows];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t rt = op.rows_p / kSliceRows, b = blockIdx.x / rt, r0 = (blockIdx.x % rt) * kSliceRows;
   const double* base = op.src + b * op.bs;
-  const int64_t k0 = blockIdx.y * kMaxSlab, k1 = min(K, k0 + kMaxSlab);
-  if (tid < kSliceRows) rowmax[tid] = 0;
-  __syncthreads();
-  if (op.ks < op.rs) {
-    for (int r = warp; r < kSliceRows; r += kSliceWarps) {
+  for (int slab = blockIdx.y; slab < slabs; slab += gridDim.y) {
+    const int64_t k0 = slab * kMaxSlab, k1 = min(K, k0 + kMaxSlab);
+    if (tid < kSliceRows) rowmax[tid] = 0;
+    __syncthreads();
+    if (op.ks < op.rs) {
+      for (int r = warp; r < kSliceRows; r += kSliceWarps) {
+        unsigned m = 0;
+        if (r0 + r < op.rows)
+#pragma unroll 16
+          for (int64_t k = k0 + lane; k < k1; k += 32) m = max(m, magnitude(base[(r0 + r) * op.rs + k * op.ks]));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) rowmax[r] = m;
+      }
+    } else {
       unsigned m = 0;
-      if (r0 + r < op.rows)
+      if (r0 + lane < op.rows)
 #pragma unroll 16
-        for (int64_t k = k0 + lane; k < k1; k += 32) m = max(m, magnitude(base[(r0 + r) * op.rs + k * op.ks]));
-      m = __reduce_max_sync(0xffffffffu, m);
-      if (lane == 0) rowmax[r] = m;
+        for (int64_t k = k0 + warp; k < k1; k += kSliceWarps)
+          m = max(m, magnitude(base[(r0 + lane) * op.rs + k * op.ks]));
+      atomicMax(&rowmax[lane], m);
     }
-  } else {
-    unsigned m = 0;
-    if (r0 + lane < op.rows)
-#pragma unroll 16
-      for (int64_t k = k0 + warp; k < k1; k += kSliceWarps) m = max(m, magnitude(base[(r0 + lane) * op.rs + k * op.ks]));
-    atomicMax(&rowmax[lane], m);
+    __syncthreads();
+    // (a thread clears what it has stored)
+    if (tid < kSliceRows) op.part[(int64_t)slab * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid] = rowmax[tid];
   }
-  __syncthreads();
-  if (tid < kSliceRows) op.part[(int64_t)blockIdx.y * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid] = rowmax[tid];
 }
 
-// blockIdx.x = 32-row tile, blockIdx.y = slab of kSliceK
+// blockIdx.x = 32-row tile, blockIdx.y = first of the slabs of kSliceK it takes
 template <int S>
 __global__ void __launch_bounds__(kSliceThreads)
     oz_slice_deep_kernel(const __grid_constant__ OzSource op, int64_t K, int64_t K_p, int slabs) {
@@ -317,19 +323,20 @@ __global__ void __launch_bounds__(kSliceThreads)
   __shared__ unsigned rowmax[kSliceRows], rowexp[kSliceRows];
   const int tid = threadIdx.x;
   const int64_t rt = op.rows_p / kSliceRows, b = blockIdx.x / rt, r0 = (blockIdx.x % rt) * kSliceRows;
-  const int64_t k0 = (int64_t)blockIdx.y * kSliceK;
-  const int len = int(min((int64_t)kSliceK, K_p - k0));
   if (tid < kSliceRows) {
     unsigned m = 0;
     for (int q = 0; q < slabs; ++q) m = max(m, op.part[(int64_t)q * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid]);
     rowexp[tid] = scale_exponent(m);
     rowmax[tid] = 0;
-    if (k0 == 0) op.scale[blockIdx.x * kSliceRows + tid] = __hiloint2double(int(rowexp[tid] << 20), 0);
+    if (blockIdx.y == 0) op.scale[blockIdx.x * kSliceRows + tid] = __hiloint2double(int(rowexp[tid] << 20), 0);
   }
-  __syncthreads();
-  load_slab(op, op.src + b * op.bs, r0, k0, len, K, tile, rowmax);
-  __syncthreads();
-  slice_slab<S>(op, b, r0, k0, len, K_p, tile, rowexp);
+  for (int64_t k0 = (int64_t)blockIdx.y * kSliceK; k0 < K_p; k0 += (int64_t)gridDim.y * kSliceK) {
+    const int len = int(min((int64_t)kSliceK, K_p - k0));
+    __syncthreads();  // the exponents are there, and the slab before is sliced
+    load_slab(op, op.src + b * op.bs, r0, k0, len, K, tile, rowmax);
+    __syncthreads();
+    slice_slab<S>(op, b, r0, k0, len, K_p, tile, rowexp);
+  }
 }
 
 struct OzEpi {
@@ -746,13 +753,15 @@ struct OzSlicer {
       count_launch(c);
     } else {
       const int slabs = int((P.K_p + kMaxSlab - 1) / kMaxSlab);
-      NSG_CHECK(slabs <= 65535 && P.K_p <= 65535 * int64_t(kSliceK) && tiles < (1ll << 31), NSG_ERR_UNSUPPORTED,
-                "ozaki slices: grid too large");
+      // (a CTA that slices reads the maxima of all slabs: beyond 512 CTAs a row tile they take
+      // several slabs each, so that the reading stays below the slicing)
+      const unsigned ymax = unsigned(std::min(slabs, 65535)),
+                     yslice = unsigned(std::min<int64_t>((P.K_p + kSliceK - 1) / kSliceK, 512));
+      NSG_CHECK(tiles < (1ll << 31), NSG_ERR_UNSUPPORTED, "ozaki slices: grid too large");
       for (int o = 0; o < P.n; ++o) {
         const unsigned mine = unsigned(P.op[o].rows_p / kSliceRows * P.op[o].batch);
-        oz_row_max_kernel<<<dim3(mine, slabs), kSliceThreads, 0, c->stream>>>(P.op[o], P.K);
-        oz_slice_deep_kernel<S><<<dim3(mine, unsigned((P.K_p + kSliceK - 1) / kSliceK)), kSliceThreads, 0, c->stream>>>(
-            P.op[o], P.K, P.K_p, slabs);
+        oz_row_max_kernel<<<dim3(mine, ymax), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, slabs);
+        oz_slice_deep_kernel<S><<<dim3(mine, yslice), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, P.K_p, slabs);
       }
       count_launch(c, 2 * P.n);
     }

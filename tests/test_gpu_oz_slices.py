@@ -123,3 +123,21 @@ def test_partial_products_of_one_term_at_a_time(nsg_ctx):
         _native.set_default_context(nsg_ctx)
     assert np.array_equal(got[0], got[1])
     assert np.max(np.abs(got[0] - a @ b)) < 8 * k * 2.0 ** -42 * np.abs(a).max() * np.abs(b).max()
+
+
+def test_depth_beyond_a_grid(nsg_ctx):
+    """Slices of more slabs of the depth than a grid has rows (65535 of 128), of operands that
+    repeat after 4096."""
+    rng = np.random.default_rng(8)
+    m, n, p, q = 64, 32, 4096, 2049
+    a, b = rng.standard_normal((m, p)), rng.standard_normal((p, n))
+    i, j, l = Index(m), Index(n), Index(p * q)
+    nsg_ctx.set_precision("ozaki")
+    try:
+        A, B = DTensor.from_numpy(np.tile(a.T, (q, 1)).T, [i, l]), DTensor.from_numpy(np.tile(b.T, (1, q)).T, [l, j])
+        got = contract([A, B], out=[i, j]).to_numpy()
+        del A, B
+    finally:
+        nsg_ctx.set_precision("fp64")
+    bound = 4 * p * q * 2.0 ** -42 * np.abs(a).max(1)[:, None] * np.abs(b).max(0)[None]
+    assert np.all(np.abs(got - q * (a @ b)) <= bound)
