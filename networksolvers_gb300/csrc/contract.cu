@@ -72,33 +72,78 @@ int with_conj(int op, bool conj) {
 
 }  // namespace
 
+// An operand that a scope owns, returned to the pool when it ends (also by an error).
+namespace {
+struct ScopedLT {
+  nsg_ctx* c;
+  LT x;
+  ~ScopedLT() {
+    try {
+      release(c, x);
+    } catch (...) {
+    }
+  }
+  LT take() {
+    LT r = x;
+    x = LT();
+    return r;
+  }
+};
+}  // namespace
+
+static LT contract_planned(nsg_ctx* c, LT A, LT B, const PairPlan<int>& plan, const std::vector<int>* final_order,
+                           nsg_tensor* into);
+
 // Contract two labeled tensors over their shared labels.  `final_order`, when
 // given, is the requested label order of the result; `into`, when given, receives
 // the result (its shape must match).
-static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_order, nsg_tensor* into) {
+static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_order, nsg_tensor* into,
+                        bool widen = true) {
   NSG_CHECK(A.t->dtype == B.t->dtype, NSG_ERR_INVALID, "contract: dtype mismatch");
+  auto dim_of = [&](int l) -> int64_t {
+    int p = pos_of(A.lab, l);
+    if (p >= 0) return A.t->dims[p];
+    return B.t->dims[pos_of(B.lab, l)];
+  };
+  const PairPlan<int> plan = plan_pair<int>(A.lab, double(A.t->size), B.lab, double(B.t->size), dim_of, widen);
+  if (plan.widened) {
+    // the wide product needs its operand's copy, and may need slices: where the budget has no
+    // room for them the thin one stays, in the operand order whose result is in place
+    for (int form = 0; form < 2; ++form) {
+      try {
+        return form == 0 ? contract_planned(c, A, B, plan, final_order, into)
+                         : contract_pair(c, A, B, final_order, into, false);
+      } catch (const Error& e) {
+        if (e.code != NSG_ERR_OOM) throw;
+      }
+    }
+    return contract_pair(c, B, A, final_order, into, false);
+  }
+  return contract_planned(c, A, B, plan, final_order, into);
+}
+
+static LT contract_planned(nsg_ctx* c, LT A, LT B, const PairPlan<int>& plan, const std::vector<int>* final_order,
+                           nsg_tensor* into) {
   const int dtype = A.t->dtype;
   auto dim_of = [&](int l) -> int64_t {
     int p = pos_of(A.lab, l);
     if (p >= 0) return A.t->dims[p];
     return B.t->dims[pos_of(B.lab, l)];
   };
-  const PairPlan<int> plan = plan_pair<int>(A.lab, double(A.t->size), B.lab, double(B.t->size), dim_of);
   const Labs<int>& K = plan.K;
   const Layout<int> &la = plan.la, &lb = plan.lb;
   for (int l : K)
     NSG_CHECK(A.t->dims[pos_of(A.lab, l)] == B.t->dims[pos_of(B.lab, l)], NSG_ERR_INVALID,
               "contract: dimension mismatch on a shared label");
   const int nk = K.n;
-  std::vector<LT> temps;
-  auto bring = [&](LT& x, const std::vector<int>& order) {
-    LT P = permute_to(c, x, order);
-    temps.push_back(P);
-    x = P;
+  ScopedLT tempA{c}, tempB{c}, result{c};
+  auto bring = [&](LT& x, ScopedLT& temp, const std::vector<int>& order) {
+    temp.x = permute_to(c, x, order);
+    x = temp.x;
     x.owned = false;
   };
-  if (plan.perm_a) bring(A, plan.a.list());
-  if (plan.perm_b) bring(B, plan.b.list());
+  if (plan.perm_a) bring(A, tempA, plan.a.list());
+  if (plan.perm_b) bring(B, tempB, plan.b.list());
   NSG_CHECK(la.contiguous && lb.contiguous && la.korder == lb.korder, NSG_ERR_INVALID,
             "contract: internal layout error");
   const int ra = int(A.lab.size()), rb = int(B.lab.size());
@@ -223,7 +268,7 @@ static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_or
   NSG_CHECK(outlab.size() <= NSG_MAX_RANK, NSG_ERR_UNSUPPORTED, "contract: result rank above 16");
   for (size_t k = 0; k < outlab.size(); ++k) odims[k] = dim_of(outlab[k]);
   bool need_final_perm = final_order && *final_order != outlab;
-  LT R;
+  LT& R = result.x;
   R.lab = outlab;
   if (into && !need_final_perm) {
     NSG_CHECK(into->size == [&] { int64_t p = 1; for (size_t k = 0; k < outlab.size(); ++k) p *= odims[k]; return p; }(),
@@ -237,13 +282,10 @@ static LT contract_pair(nsg_ctx* c, LT A, LT B, const std::vector<int>* final_or
   g.C = R.t->data;
   gemm(c, g);
   c->contractions += 1;
-  for (auto& t : temps) release(c, t);
-  if (need_final_perm) {
-    LT P = permute_to(c, R, *final_order, into);
-    release(c, R);
-    return P;
-  }
-  return R;
+  release(c, tempA.x);
+  release(c, tempB.x);
+  if (need_final_perm) return permute_to(c, R, *final_order, into);
+  return result.take();
 }
 
 }  // namespace nsg
@@ -411,9 +453,13 @@ int nsg_linmap_create(nsg_ctx* c, int n_fixed, nsg_tensor* const* fixed, const i
     const PairPlan<int> plan = plan_pair(l.order, l.size, rt.order, rt.size, [&](int x) { return dims.at(x); });
     const bool is_left = up->left == int(ni);
     if (is_left ? plan.perm_a : plan.perm_b) {
-      LT q = permute_to(c, r, (is_left ? plan.a : plan.b).list());
-      release(c, r);
-      r = q;
+      try {
+        LT q = permute_to(c, r, (is_left ? plan.a : plan.b).list());
+        release(c, r);
+        r = q;
+      } catch (const Error& e) {  // (no room: every application permutes it)
+        if (e.code != NSG_ERR_OOM) throw;
+      }
     }
     m->cached[int(ni)] = r;
   }

@@ -80,6 +80,7 @@ struct PairPlan {
   Labs<V> K, a, b, out;
   Layout<V> la, lb;
   bool perm_a = false, perm_b = false;
+  bool widened = false;  // a permutation that only makes a batched product wide
   bool batched_a() const { return la.contiguous && la.s > 0 && la.s + K.n < a.n; }
   bool batched_b() const { return lb.contiguous && lb.s > 0 && lb.s + K.n < b.n; }
   // rows and columns of the product, of each batch entry
@@ -97,7 +98,7 @@ struct PairPlan {
 };
 
 template <typename V, typename Dim>  // dim(label): its extent
-PairPlan<V> plan_pair(const Labs<V>& labA, double sizeA, const Labs<V>& labB, double sizeB, Dim dim) {
+PairPlan<V> plan_pair(const Labs<V>& labA, double sizeA, const Labs<V>& labB, double sizeB, Dim dim, bool widen = true) {
   PairPlan<V> p;
   p.a = labA;
   p.b = labB;
@@ -145,8 +146,14 @@ PairPlan<V> plan_pair(const Labs<V>& labA, double sizeA, const Labs<V>& labB, do
     const double inner = extent(x, 0, L.s), batch = extent(x, L.s + p.K.n, x.n);
     return inner < 32 && inner * batch >= 64 && extent(p.K, 0, p.K.n) >= 64;
   };
-  if (p.batched_a() && thin(p.a, p.la)) canon_A(p.lb.korder);
-  if (p.batched_b() && thin(p.b, p.lb)) canon_B(p.la.korder);
+  if (widen && p.batched_a() && thin(p.a, p.la)) {
+    canon_A(p.lb.korder);
+    p.widened = true;
+  }
+  if (widen && p.batched_b() && thin(p.b, p.lb)) {
+    canon_B(p.la.korder);
+    p.widened = true;
+  }
   if (p.batched_a() && p.batched_b()) {
     if (sizeA <= sizeB)
       canon_A(p.lb.korder);

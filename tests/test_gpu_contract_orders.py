@@ -122,3 +122,29 @@ def test_thin_batched_products(nsg_ctx, precision, tol, d, k, b):
     bound = tol * np.abs(x).max() * np.abs(y).max() * k
     assert np.max(np.abs(got - ref)) < bound
     assert np.max(np.abs(swapped - ref.transpose(1, 2, 0))) < bound
+
+
+@pytest.mark.parametrize("precision", ["fp64", "ozaki"])
+def test_thin_batches_without_room_for_a_copy(nsg_ctx, precision):
+    """A product batched over thin slices whose operand's permuted copy (and slices) the budget
+    does not hold runs as it is, with the same result, and nothing is left behind."""
+    rng = np.random.default_rng(11)
+    s, k, b, n = 2, 512, 640, 256
+    x, y = rng.standard_normal((s, k, b)), rng.standard_normal((k, n))
+    i, j, l, q = Index(s), Index(n), Index(k), Index(b)
+    out_bytes = 8 * s * n * b
+    try:
+        ctx = _native.Context(0, hbm_budget=x.nbytes + y.nbytes + out_bytes + (1 << 16), precision=precision)
+        _native.set_default_context(ctx)
+        A, B = DTensor.from_numpy(x, [i, l, q]), DTensor.from_numpy(y, [l, j])
+        before = ctx.memory()[0]
+        ref = np.einsum("slb,ln->snb", x, y)
+        for out, axes in (([i, j, q], (0, 1, 2)), ([j, i, q], (1, 0, 2))):
+            C = contract([A, B], out=out)
+            got = C.to_numpy().transpose(axes)
+            assert np.linalg.norm(got - ref) <= 1e-13 * np.linalg.norm(ref)
+            del C
+            assert ctx.memory()[0] == before
+        del A, B
+    finally:
+        _native.set_default_context(nsg_ctx)
