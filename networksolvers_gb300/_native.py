@@ -163,9 +163,10 @@ class Context:
     def set_tuning(self, param, value):
         """Launch-choice override (0 restores the compiled-in tuning table): param
         "splitk" (64 x 64-tile FP64 products, 1..64 K slices), "tridiag" (-1 all SMs, 2..16 cluster)
-        "dc_leaf" (divide and conquer leaf order, 4..32) or "lanczos_polls" (of the waits in
-        the Krylov solvers' launches; -1 gives up without one)."""
-        code = {"splitk": 0, "tridiag": 1, "dc_leaf": 2, "lanczos_polls": 3}[param]
+        "dc_leaf" (divide and conquer leaf order, 4..32), "lanczos_polls" (of the waits in the
+        Krylov solvers' launches; -1 gives up without one) or "dc_cluster" (largest cluster of
+        the divide and conquer, 4, 8 or 16; 1 none)."""
+        code = {"splitk": 0, "tridiag": 1, "dc_leaf": 2, "lanczos_polls": 3, "dc_cluster": 4}[param]
         self.check(self.L.nsg_ctx_set_tuning(self.h, code, int(value)))
 
     def profile(self, enable):

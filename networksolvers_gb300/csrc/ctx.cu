@@ -171,6 +171,10 @@ int nsg_ctx_set_tuning(nsg_ctx* c, int param, int value) {
   } else if (param == NSG_TUNE_LANCZOS_POLLS) {
     NSG_CHECK(value >= -1 && value <= (1 << 24), NSG_ERR_INVALID, "tuning: Lanczos polls -1..2^24");
     c->tune_lanczos_polls = value;
+  } else if (param == NSG_TUNE_DC_CLUSTER) {
+    NSG_CHECK(value == 0 || value == 1 || value == 4 || value == 8 || value == 16, NSG_ERR_INVALID,
+              "tuning: divide-and-conquer cluster 0, 1, 4, 8 or 16");
+    c->tune_dc_cluster = value;
   } else {
     NSG_CHECK(false, NSG_ERR_INVALID, "tuning: unknown parameter");
   }

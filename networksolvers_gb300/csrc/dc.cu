@@ -1109,6 +1109,47 @@ constexpr int kFusedMax = 128;
 // (batched) merge levels.  The context's override (4..32) trades that for fewer levels.
 static int dc_leaf_size(const nsg_ctx* c) { return c->tune_dc_leaf > 0 ? c->tune_dc_leaf : 8; }
 
+static int prep_smem(int nb) { return nb <= kSmemMerge ? nb * kPrepBytes : 0; }
+
+static cudaLaunchConfig_t dc_cluster_config(nsg_ctx* c, int C, int smem, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(kNT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = C;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// CTAs of the cluster for order n: 4, 8 or 16 by the work there is, and no more than the
+// device places together (a partition of it may hold fewer SMs side by side) or the context's
+// override says; 0, a launch per step, where not even 4 are.
+static int dc_cluster_size(nsg_ctx* c, int n) {
+  if (c->dc_cluster == 0) {
+    const auto fn = (const void*)dc_cluster_kernel;
+    ensure_smem_limit(fn, prep_smem(kFusedMax));
+    c->dc_cluster = 1;
+    for (int C = 16; C >= 4 && c->dc_cluster == 1; C /= 2) {
+      cudaLaunchAttribute attr[1];
+      const cudaLaunchConfig_t cfg = dc_cluster_config(c, C, prep_smem(kFusedMax), attr);
+      int fit = 0;
+      const bool ok = (C <= 8 || cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                      cudaOccupancyMaxActiveClusters(&fit, fn, &cfg) == cudaSuccess;
+      if (ok && fit > 0) c->dc_cluster = C;
+      if (!ok) cudaGetLastError();
+    }
+  }
+  int C = n <= 32 ? 4 : n <= 64 ? 8 : 16;
+  C = std::min(C, c->dc_cluster);
+  if (c->tune_dc_cluster > 0) C = std::min(C, c->tune_dc_cluster);
+  return C >= 4 ? C : 0;
+}
+
 double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* Q0, double* Q1, double* w, int* err) {
   DcWork W;
   W.n = n;
@@ -1163,25 +1204,10 @@ double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* 
   W.low = takei(2);
   W.rot_pq = takei(2 * N);
   W.counts = takei(MC);
-  auto prep_smem = [](int nb) { return nb <= kSmemMerge ? nb * kPrepBytes : 0; };
-  if (n <= kFusedMax && levels > 0) {
+  if (const int C = n <= kFusedMax && levels > 0 ? dc_cluster_size(c, n) : 0) {
     ProfScope ps(c, NSG_PROF_DC, 0.0);
-    cudaLaunchConfig_t cfg = {};
-    const int C = n <= 32 ? 4 : n <= 64 ? 8 : 16;
-    cfg.gridDim = dim3(C);
-    cfg.blockDim = dim3(kNT);
-    cfg.dynamicSmemBytes = prep_smem(n);
-    cfg.stream = c->stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (C > 8)
-      NSG_CUDA(cudaFuncSetAttribute((const void*)dc_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    ensure_smem_limit((const void*)dc_cluster_kernel, prep_smem(n));
+    const cudaLaunchConfig_t cfg = dc_cluster_config(c, C, prep_smem(n), attr);
     NSG_CUDA(cudaLaunchKernelEx(&cfg, dc_cluster_kernel, W, levels, Q0, Q1));
     count_launch(c);
     check_launch("dc cluster");

@@ -61,6 +61,8 @@ struct nsg_ctx {
   int tune_splitk = 0;  // FP64 GEMM K slices of the 64 x 64 tiles (> 0 forces both)
   int tune_tri = 0;     // tridiagonalisation: -1 grid kernel, 2..16 cluster size
   int tune_dc_leaf = 0; // divide and conquer leaf order (4..32; 0 the default)
+  int tune_dc_cluster = 0;     // largest cluster of the divide and conquer (1: none; 0 the default 16)
+  int dc_cluster = 0;          // the largest that fits the device, found at the first use
   int tune_lanczos_polls = 0;  // polls of a Lanczos launch's waits (-1 none; 0 the default)
   // pinned host staging for scalar readback
   double* host_scalars = nullptr;

@@ -70,3 +70,28 @@ def test_splitk_counts_agree(nsg_ctx):
             assert np.linalg.norm(c - ref) < 1e-13 * np.linalg.norm(ref), sp
     finally:
         nsg_ctx.set_tuning("splitk", 0)
+
+
+@pytest.mark.parametrize("n", [9, 24, 40, 64, 65, 128])
+def test_dc_clusters_agree(nsg_ctx, n):
+    """The divide and conquer of one cluster's orders on smaller clusters, and by a launch per
+    step (the path where the device places no cluster)."""
+    rng = np.random.default_rng(n + 2)
+    M = rng.standard_normal((n, n))
+    ref = np.linalg.svd(M, compute_uv=False) ** 2
+    l, r = Index(n), Index(n)
+    T = DTensor.from_numpy(M, [l, r])
+    assert nsg_ctx.L.nsg_ctx_set_tuning(nsg_ctx.h, 4, 2) == _native.ERR_INVALID
+    launches = []
+    try:
+        for cluster in (16, 8, 4, 1, 0):
+            nsg_ctx.set_tuning("dc_cluster", cluster)
+            before = nsg_ctx.counters()["launches"]
+            U, C, info = factorize(T, [l], cutoff=0.0, maxdim=n, spectrum=True)
+            launches.append(nsg_ctx.counters()["launches"] - before)
+            assert np.max(np.abs(info["spectrum"][:n] - ref)) < 1e-12 * ref[0], cluster
+            u, c = U.to_numpy(), C.to_numpy()
+            assert np.linalg.norm(u @ c - M) < 1e-11 * np.linalg.norm(M), cluster
+    finally:
+        nsg_ctx.set_tuning("dc_cluster", 0)
+    assert launches[0] == launches[1] == launches[2] == launches[4] < launches[3]
