@@ -20,6 +20,7 @@
 // pole, comparisons are integer ones where they can be, and the merge products skip the
 // rows and columns that the two halves' block structure makes zero.
 #include "nsg_internal.h"
+#include "secular.h"
 
 #include <cooperative_groups.h>
 
@@ -34,7 +35,6 @@ constexpr int kLeafMax = 32;
 constexpr int kNT = 256, kNW = kNT / 32;
 constexpr int kSmemMerge = 4096;  // rows of a block whose merge preparation runs in shared memory
 constexpr int kPrepBytes = 40;    // shared memory per row of that preparation
-constexpr double kEps = 2.220446049250313e-16;
 
 // Workspace: arrays of length n, a merge of the rows [lo, hi) using the slice [lo, hi):
 //   Ds, zs     sorted (sign-flipped) poles and normalised weights z
@@ -73,18 +73,6 @@ __host__ __device__ inline Span node_at(int n, int depth, int idx) {
   return s;
 }
 
-// Order-preserving integer key of a double (x < y exactly when key(x) < key(y); -0 and +0
-// equal), so the merges compare with integer instructions rather than the FP64 pipe,
-// and the exact negation -x by its sign bit.
-__device__ __forceinline__ long long order_key(double x) {
-  const long long b = __double_as_longlong(x);
-  if ((b & 0x7fffffffffffffffLL) == 0) return 0;
-  return b < 0 ? (b ^ 0x7fffffffffffffffLL) : b;
-}
-__device__ __forceinline__ double neg_exact(double x) {
-  return __longlong_as_double(__double_as_longlong(x) ^ (long long)(1ULL << 63));
-}
-
 // FP32 seeds of 1 / d and 1 / sqrt(d) (d > 0) to 2^-21, for normal d away from the ends of
 // the exponent range: the function of the leading 24 significand bits in FP32, its exponent
 // rebuilt by integer arithmetic.
@@ -119,17 +107,6 @@ __device__ __forceinline__ double recip(double d) {
   const double y = recip_seed(d), r = fma(-d, y, 1.0);
   return fma(y, fma(r, r, r), y);
 }
-// x 2^-e as a float (0 below its range), and x 2^e of a float as a double
-__device__ __forceinline__ float scaled_float(double x, int e) {
-  const int hi = __double2hiint(x), ex = ((hi >> 20) & 0x7ff) - e;
-  return ex <= 0 || ex >= 0x7ff ? 0.f : (float)__hiloint2double(hi - (e << 20), __double2loint(x));
-}
-__device__ __forceinline__ double scaled_double(float x, int e) {
-  const double d = (double)x;
-  const int ex = ((__double2hiint(d) >> 20) & 0x7ff) + e;
-  return x == 0.f || ex <= 0 || ex >= 0x7ff ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
-}
-
 __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
@@ -549,19 +526,9 @@ __device__ void prep_merge(const DcWork& W, const double* Q, int lo, int hi, int
   __syncthreads();
 }
 
-// One secular root by a group of G lanes (the 32 / G groups of a warp work on as many
-// roots, so the scalar part of a step, most of it at small k, serves them all).  Root i of
-// 1 + sum_j w_j / (D_j - lambda), w_j = rho z_j^2, lies in (D_i, D_{i+1}) (the last one in
-// (D_{k-1}, D_{k-1} + rho)); it is represented as origin + tau with the origin at the nearer
-// pole, so D_j - lambda = (D_j - origin) - tau is exact enough for the recomputed weights.
-// The first evaluation, at the interval's middle, chooses the origin and also feeds the
-// first step.  Steps: the two-pole rational model with the origin's weight kept (R.-C. Li,
-// LAPACK Working Note 89, 1994), solved in FP32, and bisection of the bracket (of its
-// exponent where it spans binades) when that leaves it or |f| grew: 4.7 evaluations on
-// average and 8 at most over random and graded problems (the last root of a graded one 11),
-// against 5.2 and 17 of the form that matches value and slope on both sides (J. R. Bunch,
-// C. P. Nielsen and D. C. Sorensen, Numer. Math. 31, 1978).  Groups without a root (i >= k) and finished ones keep
-// their warp company.
+// One secular root (secular.h) by a group of G lanes (the 32 / G groups of a warp work on as
+// many roots, so the scalar part of a step, most of it at small k, serves them all).  Groups
+// without a root (i >= k) and finished ones keep their warp company.
 template <int G>
 __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, int lane, double* Delta) {
   const double* Dk = W.Dk + lo;
@@ -577,13 +544,13 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
     dj[t] = j < k ? Dk[j] : 0.0;
     wr[t] = j < k ? wk[j] : 0.0;
   }
-  const bool inner = i < k - 1;
-  const double Di = k > 0 ? Dk[i] : 0.0, gap = inner ? Dk[i + 1] - Di : 0.0;
-  double dorg = Di;
+  const double Di = k > 0 ? Dk[i] : 0.0, gap = i < k - 1 ? Dk[i + 1] - Di : 0.0;
+  SecularRoot root;
+  root.start(i, k, Di, gap, rho);
   auto recenter = [&]() {
 #pragma unroll
     for (int t = 0; t < RC; ++t)
-      if (G * t < k) dd[t] = dj[t] - dorg;
+      if (G * t < k) dd[t] = dj[t] - root.dorg;
   };
   recenter();
   double f, dr;  // the secular function and its slope at tau without pole `skip`'s part
@@ -605,7 +572,7 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
       const int j = gl + G * t;
       if (j < k) term(j, dd[t] - tau, wr[t]);
     }
-    for (int j = gl + G * RC; j < k; j += G) term(j, (Dk[j] - dorg) - tau, wk[j]);
+    for (int j = gl + G * RC; j < k; j += G) term(j, (Dk[j] - root.dorg) - tau, wk[j]);
     // the four sums over the group with log2(G) + 1 additions: the first two steps fold the
     // lanes of one value into half the lanes of another
     const bool h1 = lane & (G / 2), h2 = lane & (G / 4);
@@ -622,102 +589,20 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
     dr = __shfl_sync(0xffffffffu, sum, G / 4, G);
     fa = __shfl_sync(0xffffffffu, fabsf((float)v - (float)o2), 0, G);
   };
-  double blo = 0.0, bhi = inner ? gap : rho, tau = 0.5 * bhi;
-  double ddi = 0.0, ddi1 = gap;
-  eval(tau, -1);
-  if (inner) {
-    const double mid = tau;
-    if (f >= 0) {
-      bhi = mid;
-    } else {
-      dorg = Dk[i + 1];
-      recenter();
-      tau = -mid;
-      blo = -mid;
-      bhi = 0.0;
-      ddi = -gap;
-      ddi1 = 0.0;
-    }
-  }
-  const float ftol = float(4.0 * kEps) * float(k + 1);
-  // the model's two poles relative to the origin (the last root's: the two last poles), and
-  // the origin's weight: the origin's pole enters with its own weight, the other one with
-  // the rest of the slope
-  const bool left = dorg == Di;  // the origin is the lower of the two (inner roots)
-  const double q1 = inner ? ddi : (k > 1 ? Dk[k - 2] - dorg : 0.0), q2 = inner ? ddi1 : 0.0;
-  const int jorg = inner && !left ? i + 1 : i;
-  const double worg = k > 0 ? wk[jorg] : 0.0;
-  float fprev = INFINITY;
+  eval(root.tau, -1);
+  if (root.inner && root.choose_origin(f, Dk[i + 1])) recenter();
+  root.set_model(i, Di, gap, k > 1 ? Dk[k - 2] : 0.0, k > 0 ? wk : nullptr);
+  auto reciprocal = [](double d) { return recip(d); };
+  auto quotient = [](float a, float b) { return __fdividef(a, b); };
   bool done = !real;
   for (int it = 0; it < 100; ++it) {
-    if (it > 0) eval(tau, jorg);
-    double tn = tau;
-    if (!done) {
-      if (__double2hiint(f) >= 0)
-        bhi = tau;
-      else
-        blo = tau;
-      const float ff = (float)f;
-      done = fabsf(ff) <= fmaf(ftol, fa, ftol);
-      if (it >= 5 && !done)
-        done = bhi - blo <= 2.0 * kEps * fmax(fabs(blo), fabs(bhi)) || bhi - blo < 1e-300;
-      if (!done) {
-        // |f| grew (or, for the last root under many poles, has halved slowly three times)
-        const bool slow = inner ? it >= 2 && fabsf(ff) > fprev : it >= 3 && fabsf(ff) > 0.5f * fprev;
-        fprev = fabsf(ff);
-        // the increment in FP32, lengths scaled by the farther pole's distance: it needs a
-        // few digits only, the next evaluation is in FP64 again
-        const double p1 = q1 - tau, p2 = q2 - tau;
-        const int e = max((__double2hiint(p1) >> 20) & 0x7ff, (__double2hiint(p2) >> 20) & 0x7ff) - 1023;
-        const float t = scaled_float(tau, e), u1 = scaled_float(p1, e), u2 = scaled_float(p2, e);
-        const float r = __fdividef(1.f, t), w1 = scaled_float(worg, e) * r * r;
-        const float s1 = scaled_float(dr, -e) - (it == 0 ? w1 : 0.f);  // the other poles' slope
-        // x: the increment, the root of c x^2 - a x + b = 0; y: the new distance from the
-        // origin directly, the root of c y^2 - h y + w q = 0 (for steps that take tau nearly
-        // to the origin, where the increment would cancel)
-        float x, y;
-        if (inner || k > 1) {
-          const float uo = inner && left ? u2 : u1;  // the other pole
-          const float pr = u1 * u2, a = fmaf(-pr, s1 + w1, (u1 + u2) * ff), b = pr * ff;
-          float c = fmaf(-uo, s1, fmaf(t, w1, ff));
-          if (!inner) c = fabsf(c);
-          const float v = a + copysignf(sqrtf(fmaxf(fmaf(a, a, -4.f * b * c), 0.f)), a);
-          x = (a < 0.f) == inner ? 0.5f * v / c : 2.f * b / v;
-          const float q = uo + t, w = w1 * t * t, h = fmaf(c, q, fmaf(s1 * uo, uo, w));
-          const float z = h + copysignf(sqrtf(fmaxf(fmaf(h, h, -4.f * c * w * q), 0.f)), h);
-          y = (h >= 0.f) == inner ? 2.f * w * q / z : 0.5f * z / c;
-        } else {  // one pole
-          x = -t * ff / fmaf(t, w1, ff);
-          y = t + x;
-        }
-        // (not a step downhill, not a number, or lost to FP32's range: Newton's step)
-        if (x * ff < 0.f && fabsf(x) < 1e30f)
-          tn = fabsf(x) > 0.5f * fabsf(t) && y * t > 0.f ? scaled_double(y, e) : tau + scaled_double(x, e);
-        else
-          tn = tau - f * recip(dr + (it == 0 ? 0.0 : scaled_double(w1, -e)));
-        const long long kt = order_key(tn);
-        if (!(tn == tn) || kt <= order_key(blo) || kt >= order_key(bhi) || slow) {
-          // out of the bracket, or slow: bisect, in the exponent where the bracket spans
-          // several binades
-          const long long ml = __double_as_longlong(blo) & 0x7fffffffffffffffLL;
-          const long long mh = __double_as_longlong(bhi) & 0x7fffffffffffffffLL;
-          const int em = int(min(ml, mh) >> 52), eM = int(max(ml, mh) >> 52);
-          tn = 0.5 * (blo + bhi);
-          if (em == 0 && it >= 2 && eM > 40)
-            tn = __hiloint2double((eM - 10) << 20, 0);
-          else if (em > 0 && eM - em > 6)
-            tn = __hiloint2double(((em + eM) / 2) << 20, 0);
-          if (__double2hiint(blo) < 0 && tn > 0.0) tn = neg_exact(tn);
-        }
-        done = tn == tau;
-      }
-    }
-    tau = tn;
+    if (it > 0) eval(root.tau, root.jorg);
+    if (!done) done = root.step(it, f, dr, fa, reciprocal, quotient);
     if (__all_sync(0xffffffffu, done)) break;
   }
   if (!real) return;
-  if (gl == 0) W.lam[lo + i] = dorg + tau;
-  for (int j = gl; j < k; j += G) Delta[(size_t)i * k + j] = (Dk[j] - dorg) - tau;
+  if (gl == 0) W.lam[lo + i] = root.dorg + root.tau;
+  for (int j = gl; j < k; j += G) Delta[(size_t)i * k + j] = (Dk[j] - root.dorg) - root.tau;
 }
 
 // Lanes per root: the fewest (8 at least) with which the roots' warps still do not exceed
