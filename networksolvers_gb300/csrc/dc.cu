@@ -595,13 +595,14 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
   auto reciprocal = [](double d) { return recip(d); };
   auto quotient = [](float a, float b) { return __fdividef(a, b); };
   bool done = !real;
-  for (int it = 0; it < 100; ++it) {
+  for (int it = 0; it < kSecularSteps; ++it) {
     if (it > 0) eval(root.tau, root.jorg);
     if (!done) done = root.step(it, f, dr, fa, reciprocal, quotient);
     if (__all_sync(0xffffffffu, done)) break;
   }
   if (!real) return;
   if (gl == 0) W.lam[lo + i] = root.dorg + root.tau;
+  if (gl == 0 && !done) atomicExch(W.err, 1);
   for (int j = gl; j < k; j += G) Delta[(size_t)i * k + j] = (Dk[j] - root.dorg) - root.tau;
 }
 

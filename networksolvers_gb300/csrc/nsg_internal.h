@@ -244,8 +244,8 @@ void scale(nsg_ctx* c, int dtype, int64_t n, double ar, double ai, void* x);
 
 // Eigen-decomposition of the real symmetric tridiagonal (d, e) on the device (dc.cu):
 // eigenvalues ascending into w, eigenvectors into the returned one of the n x n buffers Q0
-// and Q1 (column-major; both are scratch).  A leaf that does not converge sets *err (which
-// the caller zeroes before and reads after).
+// and Q1 (column-major; both are scratch).  A leaf or a secular root that does not converge
+// sets *err (which the caller zeroes before and reads after).
 double* tridiag_dc(nsg_ctx* c, int n, const double* d, const double* e, double* Q0, double* Q1, double* w, int* err);
 
 // Hermitian eigensolver (tridiagonalisation + divide and conquer + back-transformation).

@@ -1333,7 +1333,7 @@ static void syevd_dc_impl(nsg_ctx* c, int dtype, int n, T* A, std::vector<double
   Status hs;
   std::memcpy(&hs, host + n, sizeof(Status));
   NSG_CHECK(hs.bar.err == 0, NSG_ERR_TIMEOUT, "tridiagonalisation: grid barrier timed out");
-  NSG_CHECK(hs.leaf_err == 0, NSG_ERR_NONFINITE, "eigensolver: a tridiagonal leaf did not converge");
+  NSG_CHECK(hs.leaf_err == 0, NSG_ERR_NONFINITE, "eigensolver: a tridiagonal leaf or a secular root did not converge");
   w_host.assign(host, host + n);
   for (double x : w_host) NSG_CHECK(std::isfinite(x), NSG_ERR_NONFINITE, "eigensolver: non-finite eigenvalue");
   void* Zv = nullptr;
