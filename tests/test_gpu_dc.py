@@ -6,7 +6,7 @@ the bounds are 20 n eps (measured errors sit well below n eps)."""
 import numpy as np
 import pytest
 
-from networksolvers_gb300.itensors import DTensor, Index, eigen_hermitian
+from networksolvers_gb300.itensors import DTensor, Index, eigen_hermitian, factorize
 
 pytestmark = pytest.mark.gpu
 EPS = 2.3e-16
@@ -100,3 +100,18 @@ def test_tensor_core_merges(nsg_ctx, n, precision):
         check(nsg_ctx, A + A.T)
     finally:
         nsg_ctx.set_precision("fp64")
+
+
+def test_equal_eigenvalues_up_to_rounding(nsg_ctx):
+    """Gram matrices of orthogonal matrices and projectors: leaves of equal diagonal entries and
+    off-diagonal ones at the rounding level."""
+    rng = np.random.default_rng(0)
+    for rep in range(60):
+        n = (24, 64, 100, 200)[rep % 4]
+        Q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+        for A in (Q, Q[:, : n // 2] @ Q[:, : n // 2].T, np.eye(n) + 1e-16 * rng.standard_normal((n, n))):
+            i, j = Index(n), Index(n)
+            U, C, _ = factorize(DTensor.from_numpy(A, [i, j]), [i], cutoff=0.0, maxdim=n)
+            U, C = U.to_numpy(), C.to_numpy()
+            assert np.linalg.norm(U @ C - A, 2) < 20 * n * 2.3e-16
+            assert np.linalg.norm(U.T @ U - np.eye(n), 2) < 20 * n * 2.3e-16
