@@ -534,9 +534,9 @@ void gemm_f64_simt(nsg_ctx* c, const GemmArgs& g) {
   check_launch("gemm_f64_simt");
 }
 
-// FP64-level products: the eight-slice Ozaki tensor-core form (2^-55 of the row and
-// column scales) when the split precision is selected, otherwise the FP64 CUDA cores
-// (never TF32x3).
+// FP64-level products: the eight-slice Ozaki tensor-core form (within 4 K 2^-48 of the row and
+// column scales' product, the bound of its FP32 accumulator pair) when the split precision is
+// selected, otherwise the FP64 CUDA cores (never TF32x3).
 void gemm_accurate(nsg_ctx* c, const GemmArgs& g_in) {
   GemmArgs g = g_in;
   if (g.dtype == NSG_F64) {

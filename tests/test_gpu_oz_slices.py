@@ -141,3 +141,28 @@ def test_depth_beyond_a_grid(nsg_ctx):
         nsg_ctx.set_precision("fp64")
     bound = 4 * p * q * 2.0 ** -42 * np.abs(a).max(1)[:, None] * np.abs(b).max(0)[None]
     assert np.all(np.abs(got - q * (a @ b)) <= bound)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_eight_slices_batched_and_at_the_ends_of_the_range(nsg_ctx, cplx):
+    """The batched slicing and rows of extreme scale to the eight-slice bound: one slice less would
+    be 2^6 above it."""
+    rng = np.random.default_rng(6)
+    m, n, k, q = 128, 64, 129, 5
+    a, b = rnd(rng, (m, k, q), cplx), rnd(rng, (k, n), cplx)
+    a[0] = 0.0
+    a[1] *= 1e-300
+    a[2] *= 1e290
+    a[3, 5:] = 0.0
+    a[4, ::2] = 0.5
+    i, j, l, x = Index(m), Index(n), Index(k), Index(q)
+    nsg_ctx.set_precision("ozaki8")
+    try:
+        got = contract([DTensor.from_numpy(a, [i, l, x]), DTensor.from_numpy(b, [l, j])], out=[i, j, x]).to_numpy()
+    finally:
+        nsg_ctx.set_precision("fp64")
+    ref = np.einsum("ilx,lj->ijx", a, b)
+    scales = np.abs(a).max(1)[:, None, :] * np.abs(b).max(0)[None, :, None]
+    bound = (8 if cplx else 4) * k * 2.0 ** -48 * scales
+    assert np.all(np.abs(got - ref) <= bound + 1e-14 * np.abs(ref))
+    assert np.all(got[0] == 0.0)
