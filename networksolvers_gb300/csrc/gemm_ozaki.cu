@@ -280,8 +280,9 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_shallow_kernel(const _
   slice_slab<S>(op, b, r0, k0, len, P.K_p, tile, rowexp);
 }
 
-// blockIdx.x = 32-row tile (over the batch), blockIdx.y = first of the slabs of kMaxSlab it
-// takes (one, but for depths that exceed a grid's 65535)
+// blockIdx.x = 32-row tile (over the batch), blockIdx.y = its slab of kMaxSlab (MANY: the first
+// of those it takes)
+template <bool MANY>
 __global__ void __launch_bounds__(kSliceThreads)
     oz_row_max_kernel(const __grid_constant__ OzSource op, int64_t K, int slabs) {
   __shared__ unsigned rowmax[kSliceRows];
@@ -312,11 +313,12 @@ __global__ void __launch_bounds__(kSliceThreads)
     __syncthreads();
     // (a thread clears what it has stored)
     if (tid < kSliceRows) op.part[(int64_t)slab * op.rows_p * op.batch + blockIdx.x * kSliceRows + tid] = rowmax[tid];
+    if constexpr (!MANY) break;
   }
 }
 
-// blockIdx.x = 32-row tile, blockIdx.y = first of the slabs of kSliceK it takes
-template <int S>
+// blockIdx.x = 32-row tile, blockIdx.y = its slab of kSliceK (MANY: the first of those it takes)
+template <int S, bool MANY>
 __global__ void __launch_bounds__(kSliceThreads)
     oz_slice_deep_kernel(const __grid_constant__ OzSource op, int64_t K, int64_t K_p, int slabs) {
   __shared__ double tile[kTileBytes / 8];
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(kSliceThreads)
     load_slab(op, op.src + b * op.bs, r0, k0, len, K, tile, rowmax);
     __syncthreads();
     slice_slab<S>(op, b, r0, k0, len, K_p, tile, rowexp);
+    if constexpr (!MANY) break;
   }
 }
 
@@ -753,15 +756,22 @@ struct OzSlicer {
       count_launch(c);
     } else {
       const int slabs = int((P.K_p + kMaxSlab - 1) / kMaxSlab);
-      // (a CTA that slices reads the maxima of all slabs: beyond 512 CTAs a row tile they take
-      // several slabs each, so that the reading stays below the slicing)
-      const unsigned ymax = unsigned(std::min(slabs, 65535)),
-                     yslice = unsigned(std::min<int64_t>((P.K_p + kSliceK - 1) / kSliceK, 512));
       NSG_CHECK(tiles < (1ll << 31), NSG_ERR_UNSUPPORTED, "ozaki slices: grid too large");
+      // beyond 512 CTAs a row tile they take several slabs each: a CTA that slices reads the
+      // maxima of all slabs, and a grid has 65535 rows (the loop costs the others 2 to 4 % of an
+      // eigensolve at bond dimension 1024 and of an environment update)
+      const int64_t yslice = (P.K_p + kSliceK - 1) / kSliceK;
+      const bool many = yslice > 512;
       for (int o = 0; o < P.n; ++o) {
         const unsigned mine = unsigned(P.op[o].rows_p / kSliceRows * P.op[o].batch);
-        oz_row_max_kernel<<<dim3(mine, ymax), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, slabs);
-        oz_slice_deep_kernel<S><<<dim3(mine, yslice), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, P.K_p, slabs);
+        if (many) {
+          oz_row_max_kernel<true><<<dim3(mine, 512), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, slabs);
+          oz_slice_deep_kernel<S, true><<<dim3(mine, 512), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, P.K_p, slabs);
+        } else {
+          oz_row_max_kernel<false><<<dim3(mine, slabs), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, slabs);
+          oz_slice_deep_kernel<S, false><<<dim3(mine, unsigned(yslice)), kSliceThreads, 0, c->stream>>>(P.op[o], P.K, P.K_p,
+                                                                                                     slabs);
+        }
       }
       count_launch(c, 2 * P.n);
     }

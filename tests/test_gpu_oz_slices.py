@@ -125,11 +125,12 @@ def test_partial_products_of_one_term_at_a_time(nsg_ctx):
     assert np.max(np.abs(got[0] - a @ b)) < 8 * k * 2.0 ** -42 * np.abs(a).max() * np.abs(b).max()
 
 
-def test_depth_beyond_a_grid(nsg_ctx):
-    """Slices of more slabs of the depth than a grid has rows (65535 of 128), of operands that
-    repeat after 4096."""
+@pytest.mark.parametrize("p,q", [(4096, 16), (4097, 16), (4096, 2049)])
+def test_depth_beyond_a_grid(nsg_ctx, p, q):
+    """Slices of 512 slabs of the depth and one more, and of more than a grid has rows (65535 of
+    128), of operands that repeat."""
     rng = np.random.default_rng(8)
-    m, n, p, q = 64, 32, 4096, 2049
+    m, n = 64, 32
     a, b = rng.standard_normal((m, p)), rng.standard_normal((p, n))
     i, j, l = Index(m), Index(n), Index(p * q)
     nsg_ctx.set_precision("ozaki")
