@@ -138,7 +138,8 @@ int nsg_ctx_wait_probe(nsg_ctx* ctx, int64_t polls);
  * larger leaves mean fewer merge levels, so fewer launches per eigensolve above order 128, at
  * a longer leaf solve); NSG_TUNE_LANCZOS_POLLS: polls after which a wait inside the Krylov
  * solvers' launches gives up (1..2^24; 0 the default 2^22; -1 without a poll, for checks of the
- * giving-up: the solver then repeats its cycle with kernels that wait for nothing); NSG_TUNE_DC_CLUSTER: the
+ * giving-up: the solver then repeats its cycle with kernels that wait for nothing; -2 in
+ * eigsolve's final normalisation alone, which then leaves x as it is); NSG_TUNE_DC_CLUSTER: the
  * largest thread-block cluster that solves a tridiagonal of order up to 128 (4, 8 or 16; 1 by a
  * launch per step instead, as where no cluster fits; 0 the default 16). */
 #define NSG_TUNE_SPLITK 0

@@ -169,7 +169,7 @@ int nsg_ctx_set_tuning(nsg_ctx* c, int param, int value) {
     NSG_CHECK(value == 0 || (value >= 4 && value <= 32), NSG_ERR_INVALID, "tuning: leaf order 0 or 4..32");
     c->tune_dc_leaf = value;
   } else if (param == NSG_TUNE_LANCZOS_POLLS) {
-    NSG_CHECK(value >= -1 && value <= (1 << 24), NSG_ERR_INVALID, "tuning: Lanczos polls -1..2^24");
+    NSG_CHECK(value >= -2 && value <= (1 << 24), NSG_ERR_INVALID, "tuning: Lanczos polls -2..2^24");
     c->tune_lanczos_polls = value;
   } else if (param == NSG_TUNE_DC_CLUSTER) {
     NSG_CHECK(value == 0 || value == 1 || value == 4 || value == 8 || value == 16, NSG_ERR_INVALID,

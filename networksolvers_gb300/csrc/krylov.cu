@@ -162,8 +162,9 @@ void lanczos_step(nsg_ctx* c, nsg_linmap* m, std::vector<nsg_tensor*>& V, int j,
 // The Lanczos steps of one cycle with every scalar kept on the device: the two CGS
 // passes' coefficients and the sum of squares of w stay in `scal` (one block of
 // 4 (j + 1) + 2 doubles per step j, at step_offset(j)) and the next basis vector is
-// normalised by a kernel that reads that sum of squares, so the cycle issues no host
-// synchronisation; the host reads every scalar back once.  A step's vector work is one launch
+// normalised by a kernel that reads that sum of squares, so no step waits for a scalar on
+// the host; the host reads every scalar back once.  (An application of the map in a split
+// precision still ends with a read of the context's error flag.)  A step's vector work is one launch
 // (lanczos.cu), in the operations of lanczos_step; beyond the vectors that launch takes, the
 // kernels of lanczos_step.  All K steps run; steps after a breakdown are discarded by the
 // caller, and all of them when a wait of those launches gave up (the status word behind the
@@ -266,10 +267,9 @@ int nsg_eigsolve(nsg_ctx* c, nsg_linmap* m, nsg_tensor* x, int krylovdim, int ma
       for (int j = 0; j < k; ++j) ptrs[j] = V[j]->data;
       NSG_CUDA(cudaMemsetAsync(x->data, 0, x->bytes, c->stream));
       multi_axpy(c, dt, n, k, ptrs.data(), coef.data(), x->data);
-      // (by kernels that wait for nothing: the host does not read anything after them)
-      const void* xq[1] = {x->data};
-      multi_dot_dev(c, dt, n, 1, xq, x->data, sx);
-      axpby_devscalar(c, dt, n, sx, 0, x->data, x->data);
+      // x is of norm 1 to the rounding of its sum, and stays as it is where a wait in this
+      // launch gives up (which the host does not learn)
+      lv.step(0, nullptr, x->data, nullptr, nullptr, nullptr, sx, x->data);
       *eigval = lam;
       if (numops) *numops = ops;
       check_device_flag(c);
@@ -349,7 +349,7 @@ int nsg_exponentiate(nsg_ctx* c, nsg_linmap* m, double t_re, double t_im, nsg_te
       col.assign(E2.begin(), E2.begin() + kk);
     };
     // Speculative device-resident cycle: the number of steps the previous cycle needed
-    // (plus one) runs without host synchronisation, then the host replays the stopping
+    // (plus one) runs without scalars on the host, then the host replays the stopping
     // rule on the read-back scalars.  The vectors are those of the step-by-step form up to
     // the rounding of its sums (which other kernels add in another order); a rule that has
     // not stopped continues step by step from there, and a sum of squares outside the range

@@ -258,8 +258,9 @@ __global__ void __launch_bounds__(kT, 2) lanczos_step_kernel(const __grid_consta
       }
     }
   }
-  if (s.next) {
-    __syncthreads();
+  __syncthreads();
+  // (normalised in place: a CTA whose wait gave up leaves its part as it is)
+  if (s.next && (s.next != s.w || isfinite(res[0]))) {
     const double a = res[1];
     T* next = (T*)s.next;
     sweep(false, [](int64_t) {}, [&](int, int64_t i, T x) {
@@ -319,7 +320,8 @@ bool LanczosVectors::step(int nv, const void* const* v, void* w, const double* p
   s.msg = (ulonglong2*)msg;
   s.tag = tag;
   tag += 4;
-  s.polls = c->tune_lanczos_polls != 0 ? c->tune_lanczos_polls : 1 << 22;
+  const int polls = c->tune_lanczos_polls;
+  s.polls = polls == -2 ? (next == w ? -1 : 1 << 22) : polls != 0 ? polls : 1 << 22;
   s.gave_up = gave_up;
   const void* fn = dtype == NSG_C128 ? step_kernel<double2>(nv) : step_kernel<double>(nv);
   void* args[] = {&s};

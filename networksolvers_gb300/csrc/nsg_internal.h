@@ -63,7 +63,7 @@ struct nsg_ctx {
   int tune_dc_leaf = 0; // divide and conquer leaf order (4..32; 0 the default)
   int tune_dc_cluster = 0;     // largest cluster of the divide and conquer (1: none; 0 the default 16)
   int dc_cluster = 0;          // the largest that fits the device, found at the first use
-  int tune_lanczos_polls = 0;  // polls of a Lanczos launch's waits (-1 none; 0 the default)
+  int tune_lanczos_polls = 0;  // polls of a Lanczos launch's waits (-1, -2 none; 0 the default)
   // pinned host staging for scalar readback
   double* host_scalars = nullptr;
   size_t host_scalars_cap = 0;
@@ -223,7 +223,8 @@ double norm2(nsg_ctx* c, int dtype, int64_t n, const void* x);
 // (2 doubles each) go to co1 and co2, ss = {|w|^2, |w|}, next = w / |w| (unless null).  nv = 0:
 // w is only read.  Returns false, with nothing launched, for more vectors than it takes.
 // A wait that gives up sets *gave_up (which the caller zeroes before and reads with the
-// scalars); the vectors and scalars are then not to be used.
+// scalars); the vectors and scalars are then not to be used, but for w normalised in place (next
+// = w), of which the parts whose CTA gave up are left as they are.
 struct LanczosVectors {
   nsg_ctx* c;
   int dtype;

@@ -97,6 +97,11 @@ def test_waits_that_give_up(nsg_ctx, precision):
         assert abs(lam_g - lam) <= 1e-10 * abs(lam)
         assert np.linalg.norm(x_g - x) < 1e-8 and np.linalg.norm(y_g - y) < 1e-8 * np.linalg.norm(y)
         assert abs(np.linalg.norm(x_g) - 1) < 1e-13
+        nsg_ctx.set_tuning("lanczos_polls", -2)
+        lam_g, x_g, _, launches_g = solve()
+        nsg_ctx.set_tuning("lanczos_polls", 0)
+        assert lam_g == lam and launches_g == launches
+        assert np.linalg.norm(x_g - x) < 1e-14 and abs(np.linalg.norm(x_g) - 1) < 1e-13
         assert solve()[3] == launches
     finally:
         nsg_ctx.set_tuning("lanczos_polls", 0)
