@@ -171,10 +171,9 @@ __device__ __forceinline__ double above(double x, int low) {
 // a leaf of equal ones (of an orthogonal matrix's Gram matrix) may go on exchanging it: from the
 // tenth sweep on, which few other leaves reach, the bound doubles every other sweep (at most 16
 // sweeps, four eps, over three million random leaves, a ninth of them equal entries and noise).
-// (An implicit-QL chase is a serial chain of square roots and
-// divisions, 148 us for a leaf of 8 rows; Jacobi with FP64 angles 94, this 48.)  Writes the sorted
-// pairs into the leaf's diagonal block of Q0 and Q1 and into w; a leaf that still rotates
-// after 30 sweeps raises *err.
+// Measured: 48 us for leaves of 8 rows (an implicit-QL chase, a serial chain of square roots and
+// divisions, 148).  Writes the sorted pairs into the leaf's diagonal block of Q0 and Q1 and into
+// w; a leaf that still rotates after 30 sweeps raises *err.
 __device__ void solve_leaf(const DcWork& W, int lo, int hi, double* Q0, double* Q1) {
   __shared__ double A[kLeafMax][kLeafMax + 1], V[kLeafMax][kLeafMax + 1], cs[kLeafMax / 2], sn[kLeafMax / 2];
   __shared__ int pos[kLeafMax], moved, expo, top;
@@ -233,8 +232,8 @@ __device__ void solve_leaf(const DcWork& W, int lo, int hi, double* Q0, double* 
     ib[x] = t < vbase ? (t >> 1) / np : (t - vbase) % s;
   }
   __syncthreads();
+  float tiny = 1.2e-16f;
   for (int sweep = 0; s > 1; ++sweep) {
-    const float tiny = sweep < 10 ? 1.2e-16f : ldexpf(1.2e-16f, (sweep - 8) / 2);
     for (int r = 0; r < ne - 1; ++r) {
       if (tid < np) {
         const int p = pairs[r][tid][0], q = pairs[r][tid][1];
@@ -305,6 +304,7 @@ __device__ void solve_leaf(const DcWork& W, int lo, int hi, double* Q0, double* 
       if (tid == 0) atomicExch(W.err, 1);
       break;
     }
+    if (sweep >= 9 && (sweep & 1)) tiny *= 2.f;
   }
   if (tid < s) {
     const long long k = order_key(A[tid][tid]);
@@ -550,12 +550,11 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
     wr[t] = j < k ? wk[j] : 0.0;
   }
   const double Di = k > 0 ? Dk[i] : 0.0, gap = i < k - 1 ? Dk[i + 1] - Di : 0.0;
-  SecularRoot root;
-  root.start(i, k, Di, gap, rho);
+  double dorg = Di;
   auto recenter = [&]() {
 #pragma unroll
     for (int t = 0; t < RC; ++t)
-      if (G * t < k) dd[t] = dj[t] - root.dorg;
+      if (G * t < k) dd[t] = dj[t] - dorg;
   };
   recenter();
   double f, dr;  // the secular function and its slope at tau without pole `skip`'s part
@@ -577,7 +576,7 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
       const int j = gl + G * t;
       if (j < k) term(j, dd[t] - tau, wr[t]);
     }
-    for (int j = gl + G * RC; j < k; j += G) term(j, (Dk[j] - root.dorg) - tau, wk[j]);
+    for (int j = gl + G * RC; j < k; j += G) term(j, (Dk[j] - dorg) - tau, wk[j]);
     // the four sums over the group with log2(G) + 1 additions: the first two steps fold the
     // lanes of one value into half the lanes of another
     const bool h1 = lane & (G / 2), h2 = lane & (G / 4);
@@ -594,9 +593,37 @@ __device__ void secular_root(const DcWork& W, int lo, int k, int i, double rho, 
     dr = __shfl_sync(0xffffffffu, sum, G / 4, G);
     fa = __shfl_sync(0xffffffffu, fabsf((float)v - (float)o2), 0, G);
   };
-  eval(root.tau, -1);
-  if (root.inner && root.choose_origin(f, Dk[i + 1])) recenter();
-  root.set_model(i, Di, gap, k > 1 ? Dk[k - 2] : 0.0, k > 0 ? wk : nullptr);
+  const bool inner = i < k - 1;
+  double blo = 0.0, bhi = inner ? gap : rho, tau = 0.5 * bhi, ddi = 0.0, ddi1 = gap;
+  eval(tau, -1);
+  if (inner) {
+    const double mid = tau;
+    if (f >= 0) {
+      bhi = mid;
+    } else {
+      dorg = Dk[i + 1];
+      recenter();
+      tau = -mid;
+      blo = -mid;
+      bhi = 0.0;
+      ddi = -gap;
+      ddi1 = 0.0;
+    }
+  }
+  SecularRoot root;
+  root.dorg = dorg;
+  root.tau = tau;
+  root.blo = blo;
+  root.bhi = bhi;
+  root.ftol = float(4.0 * kEps) * float(k + 1);
+  root.fprev = INFINITY;
+  root.inner = inner;
+  root.single = k <= 1;
+  root.left = dorg == Di;
+  root.q1 = inner ? ddi : (k > 1 ? Dk[k - 2] - dorg : 0.0);
+  root.q2 = inner ? ddi1 : 0.0;
+  root.jorg = inner && !root.left ? i + 1 : i;
+  root.worg = k > 0 ? wk[root.jorg] : 0.0;
   auto reciprocal = [](double d) { return recip(d); };
   auto quotient = [](float a, float b) { return __fdividef(a, b); };
   bool done = !real;

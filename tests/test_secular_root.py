@@ -24,7 +24,7 @@ static void check(const Vec& D, const Vec& w, double rho, int i) {
   const int k = int(D.size());
   const double gap = i < k - 1 ? D[i + 1] - D[i] : 0.0;
   SecularRoot r;
-  r.start(i, k, D[i], gap, rho);
+  r.dorg = D[i];
   double f, dr;
   float fa;
   auto eval = [&](double tau, int skip) {
@@ -38,9 +38,29 @@ static void check(const Vec& D, const Vec& w, double rho, int i) {
     dr = dpsi + dphi;
     fa = fabsf((float)psi - (float)phi);
   };
+  // the start as the device makes it
+  r.inner = i < k - 1;
+  r.single = k <= 1;
+  r.blo = 0.0;
+  r.bhi = r.inner ? gap : rho;
+  r.tau = 0.5 * r.bhi;
   eval(r.tau, -1);
-  if (r.inner) r.choose_origin(f, D[i + 1]);
-  r.set_model(i, D[i], gap, k > 1 ? D[k - 2] : 0.0, w.data());
+  r.left = true;
+  if (r.inner && f >= 0) {
+    r.bhi = r.tau;
+  } else if (r.inner) {
+    r.left = false;
+    r.dorg = D[i + 1];
+    r.tau = -r.tau;
+    r.blo = r.tau;
+    r.bhi = 0.0;
+  }
+  r.ftol = float(4.0 * kEps) * float(k + 1);
+  r.fprev = INFINITY;
+  r.q1 = r.inner ? (r.left ? 0.0 : -gap) : (r.single ? 0.0 : D[k - 2] - r.dorg);
+  r.q2 = r.inner && r.left ? gap : 0.0;
+  r.jorg = r.inner && !r.left ? i + 1 : i;
+  r.worg = w[r.jorg];
   bool done = false;
   int it = 0;
   for (; it < kSecularSteps && !done; ++it) {
