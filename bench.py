@@ -375,11 +375,12 @@ def run_nsg(args):
                 "frac": achieved / fp64_peak, "traffic": None, "kernel": dom,
                 "peak_note": FP64_PEAK_NOTE}
         if dom == "tridiag":
-            # DRAM bytes of one launch from the ncu capture at n = 950 (7.28 MB read + 1.87 MB
-            # written: the L2-resident matrix once, the reflectors back), scaled by n^2 to the
-            # launches' mean order, which the algorithmic flops per launch (4/3 n^3) give
+            # DRAM bytes of one launch from the ncu capture of the resident kernel at n = 950
+            # (7.32 MB read, the matrix once, and 0.06 MB written: the reflectors stay in L2),
+            # scaled by n^2 to the launches' mean order, which the algorithmic flops per launch
+            # (4/3 n^3) give
             n_eff = (0.75 * c["flops"] / c["launches"]) ** (1.0 / 3.0)
-            roof["traffic"] = 9.15e6 * (n_eff / 950.0) ** 2
+            roof["traffic"] = 7.38e6 * (n_eff / 950.0) ** 2
             roof["traffic_note"] = (f"bytes per launch at the launches' mean order n = {n_eff:.0f} (from 4/3 n^3 "
                                     f"flops per launch), scaled by n^2 from ncu at n=950")
     if roof is not None:

@@ -54,11 +54,12 @@ function check(c::Ctx, rc)
 end
 const PRECISION = Dict(:fp64 => 0, :tf32x3 => 1, :ozaki => 2, :ozaki8 => 3)
 set_precision!(c::Ctx, p::Symbol) = check(c, @ccall lib.nsg_ctx_set_precision(c.h::Ptr{Cvoid}, PRECISION[p]::Cint)::Cint)
-# pin one launch choice of the compiled-in tuning table for this context (measurement):
-# :splitk => 1..64 K slices of small FP64 products, :tridiag => -1 (grid kernel) or a
-# cluster size 2/4/8/16, :dc_leaf => divide-and-conquer leaf order 4..32; 0 returns to
-# the table
-const TUNING = Dict(:splitk => 0, :tridiag => 1, :dc_leaf => 2)
+# pin one launch choice for this context (measurement): :splitk => FP64 products by the
+# 64 x 64-tile kernel with 1..64 K slices, :tridiag => -1 (all SMs) or a cluster size
+# 2/4/8/16, :dc_leaf => divide-and-conquer leaf order 4..32, :lanczos_polls => polls of the
+# Krylov launches' waits (-1 none), :dc_cluster => largest divide-and-conquer cluster 4/8/16
+# (1 none); 0 returns to the library's own choice
+const TUNING = Dict(:splitk => 0, :tridiag => 1, :dc_leaf => 2, :lanczos_polls => 3, :dc_cluster => 4)
 set_tuning!(c::Ctx, p::Symbol, v::Integer) =
   check(c, @ccall lib.nsg_ctx_set_tuning(c.h::Ptr{Cvoid}, TUNING[p]::Cint, Cint(v)::Cint)::Cint)
 # per-phase device timers of the region step: the overrides below bracket their phases,

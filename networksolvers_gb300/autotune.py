@@ -9,14 +9,14 @@ events around the kernels of the class (nsg_ctx_profile):
   8..576: the kernel over all SMs against one thread-block cluster of 2, 4, 8 and 16 CTAs
   (where the matrix fits the cluster's shared memory; a cluster within 15 % of the kernel
   over all SMs is preferred, since it leaves the other SMs to other streams);
-* the FP64 CUDA-core GEMM of small outputs (the eigensolver's products at small bond
-  dimension), for output sizes 32..256 and depths 64..4096: split K into 1..64 slices.
+* the 64 x 64-tile FP64 GEMM on small outputs, for output sizes 32..256 and depths
+  64..4096: split K into 1..64 slices (a record: the library gives such products to its
+  16 x 16-tile kernel, and splits K of the 64 x 64 tiles only where a context asks for it).
 
 For each case the fastest choice (median of --reps) goes into DIR/tuning.json and
 DIR/tuning_table.h (the header the library compiles in: copy it to
 networksolvers_gb300/csrc/ and rebuild).  Orders whose best path is the grid kernel end
-the cluster table; split-K buckets whose best count equals the built-in rule's are kept
-too (the table then pins what was measured).
+the cluster table.
 """
 from __future__ import annotations
 
@@ -156,9 +156,10 @@ def header(tri, split, device_name):
         "    " + " ".join(f"{{{a}, {b}}}," for a, b in (tri or [(0, 0)])),
         "};",
         "",
-        "// FP64 CUDA-core GEMM: number of K slices (split K) for products whose output has",
-        "// `tiles` 64 x 64 tiles (times the batch) and depth K, by buckets (tiles <= max_tiles",
-        "// and K <= max_k, first match); 0 keeps the built-in rule (about two slices per SM).",
+        "// The 64 x 64-tile FP64 GEMM: the fastest number of K slices (split K) for products whose",
+        "// output has `tiles` such tiles (times the batch) and depth K, by buckets (tiles <= max_tiles",
+        "// and K <= max_k, first match).  A record of the measurements: no dispatch reads it, products",
+        "// of few tiles take the 16 x 16-tile kernel unless a context asks for slices.",
         "struct SplitEntry {",
         "  int max_tiles;",
         "  int max_k;",

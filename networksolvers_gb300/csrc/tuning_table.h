@@ -19,9 +19,10 @@ constexpr TriEntry kTri[] = {
     {16, 8}, {64, 16},
 };
 
-// FP64 CUDA-core GEMM: number of K slices (split K) for products whose output has
-// `tiles` 64 x 64 tiles (times the batch) and depth K, by buckets (tiles <= max_tiles
-// and K <= max_k, first match); 0 keeps the built-in rule (about two slices per SM).
+// The 64 x 64-tile FP64 GEMM: the fastest number of K slices (split K) for products whose
+// output has `tiles` such tiles (times the batch) and depth K, by buckets (tiles <= max_tiles
+// and K <= max_k, first match).  A record of the measurements: no dispatch reads it, products
+// of few tiles take the 16 x 16-tile kernel unless a context asks for slices.
 struct SplitEntry {
   int max_tiles;
   int max_k;
